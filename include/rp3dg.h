@@ -334,7 +334,7 @@ int rp3dg_axis_mlp_grads(rp3dg_ctx* ctx, const float* features, const uint8_t* l
  * start-up and forbids later cudaMalloc calls (an allocation can stall the
  * whole device and can fail once the budget is spent), whereas
  * rp3dg_axis_mlp_grads grows its scratch with cudaMalloc for larger batches.
- * The scratch here is a fixed array inside the library (4.4 MB, held by every
+ * The scratch here is a fixed array inside the library (3.5 MB, held by every
  * GPU that loads the library until exit): n is limited to 4096 samples
  * (RP3DG_ECAPACITY beyond).  All calls share the array and it keeps the last
  * call's contents; calls that overlap on the GPU race.  The first call on a

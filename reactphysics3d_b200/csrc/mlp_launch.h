@@ -22,8 +22,15 @@ constexpr int MLP_OFF_W3 = MLP_OFF_B2 + MLP_H;
 constexpr int MLP_OFF_B3 = MLP_OFF_W3 + MLP_H * MLP_OUT;
 constexpr int MLP_NPARAMS = MLP_OFF_B3 + MLP_OUT;  // 6800
 
-// floats per sample of training scratch: h1[64] h2[64] dh1[64] dh2[64] dz[16]
-constexpr int MLP_SCRATCH_ROW = 272;
+// Training scratch: one row of partial gradients (and the partial loss) per
+// CTA of the gradient kernel, which takes MLP_TILE samples at a time; a batch
+// has a CTA per tile up to MLP_GRAD_CTAS.
+constexpr int MLP_TILE = 32;
+constexpr uint32_t MLP_GRAD_CTAS = 296;
+constexpr int MLP_PARTIAL_ROW = MLP_NPARAMS + 16;
+constexpr uint32_t mlp_partial_rows(uint32_t n) {
+    return n / MLP_TILE + (n % MLP_TILE != 0) < MLP_GRAD_CTAS ? n / MLP_TILE + (n % MLP_TILE != 0) : MLP_GRAD_CTAS;
+}
 
 struct MlpPairArgs {
     uint32_t n;

@@ -1613,7 +1613,7 @@ int mlp_pair_args(rp3dg_ctx* ctx, const rp3dg_pair_batch* p, rp3dg::MlpPairArgs&
 }
 
 int mlp_grads_into(rp3dg_ctx* ctx, const float* x, const uint8_t* y, uint32_t n, float* grads, float* loss) {
-    const size_t need = size_t(n) * rp3dg::MLP_SCRATCH_ROW * sizeof(float);
+    const size_t need = size_t(rp3dg::mlp_partial_rows(n)) * rp3dg::MLP_PARTIAL_ROW * sizeof(float);
     if (need > ctx->cap_mlp_scratch) {
         cudaFree(ctx->d_mlp_scratch);
         ctx->d_mlp_scratch = nullptr;
@@ -1621,8 +1621,7 @@ int mlp_grads_into(rp3dg_ctx* ctx, const float* x, const uint8_t* y, uint32_t n,
         if (e != cudaSuccess) { ctx->cap_mlp_scratch = 0; return cuda_fail(ctx, e, "cudaMalloc(mlp scratch)"); }
         ctx->cap_mlp_scratch = need;
     }
-    cudaError_t e = cudaMemsetAsync(mlp_loss(ctx), 0, sizeof(float), ctx->stream);
-    if (e == cudaSuccess) e = rp3dg::launch_mlp_grads(mlp_params(ctx), x, y, n, ctx->d_mlp_scratch, grads, mlp_loss(ctx), ctx->stream);
+    cudaError_t e = rp3dg::launch_mlp_grads(mlp_params(ctx), x, y, n, ctx->d_mlp_scratch, grads, mlp_loss(ctx), ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "mlp gradients");
     ctx->launches += 2;
     if (loss) {
