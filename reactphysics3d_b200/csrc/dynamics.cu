@@ -181,7 +181,10 @@ __global__ void __launch_bounds__(128) dyn_manifold_init(const DynArgs a) {
     const float fixed = float((is_fixed(a, b1) ? 1 : 0) | (is_fixed(a, b2) ? 2 : 0));
     q[DQ_MASS] = make_float4(im1, im2, friction, fixed);
     q[DQ_LF1] = a.llock[b1]; q[DQ_LF2] = a.llock[b2];
-    q[DQ_AF1] = a.alock[b1]; q[DQ_AF2] = a.alock[b2];
+    const float4 al1 = a.alock[b1], al2 = a.alock[b2];
+    q[DQ_AF1] = al1; q[DQ_AF2] = al2;
+    const v3 af1 = L3(al1), af2 = L3(al2);
+    const float beta = a.split ? BETA_SPLIT_IMPULSE : BETA;
     const v3 v1 = L3(a.lin_vel[b1]), w1 = L3(a.ang_vel[b1]);
     const v3 v2 = L3(a.lin_vel[b2]), w2 = L3(a.ang_vel[b2]);
     const float4 o1 = a.c_wori[id.z], o2 = a.c_wori[id.w];
@@ -209,11 +212,18 @@ __global__ void __launch_bounds__(128) dyn_manifold_init(const DynArgs a) {
         float bias = 0.0f;
         const float dvn = dv.x * n.x + dv.y * n.y + dv.z * n.z;
         if (dvn < -a.restitution_threshold) bias = restitution * dvn;
-        r.q[DP_R1] = F4w(r1, nd.w);
+        // the penetration bias and the products i * angular lock factor are the
+        // same in every pass (solve, :479-759, forms them anew): kept here
+        float bias_pen = 0.0f;
+        if (nd.w > SLOP) {
+            const float excess = nd.w - SLOP;
+            bias_pen = -(beta / a.dt) * ((0.0f < excess) ? excess : 0.0f);
+        }
+        r.q[DP_R1] = F4w(r1, 0.0f);
         r.q[DP_R2] = F4w(r2, inv_mass);
-        r.q[DP_N] = F4w(n, bias);
-        r.q[DP_I1] = F4w(i1, 0.0f);
-        r.q[DP_I2] = F4w(i2, 0.0f);
+        r.q[DP_N] = F4w(n, a.split ? bias : bias_pen + bias);
+        r.q[DP_I1] = F4w(vcmul(i1, af1), bias_pen);
+        r.q[DP_I2] = F4w(vcmul(i2, af2), 0.0f);
         r.mut = make_float4(a.p_impulse[p], 0.0f, resting ? 1.0f : 0.0f, 0.0f);
         nsum = V(nsum.x + n.x, nsum.y + n.y, nsum.z + n.z);
     }
@@ -296,17 +306,18 @@ RD void load_man_q(const float4* __restrict__ q, Man& c) {
 RD void load_man(const DynManifoldRec* __restrict__ rec, Man& c) { load_man_q<true>(rec->q, c); }
 
 struct Pt {
-    v3 r1, r2, n, i1, i2;
-    float depth, inv_mass, bias;
+    v3 r1, r2, n, i1, i2;          // i1, i2: times the angular lock factors
+    float inv_mass, bias, bias_pen;  // bias: of the constrained velocities
 };
 
 template <bool LDG = true>
 RD void load_pt_q(const float4* __restrict__ q, Pt& p) {
     const float4 a = ldq<LDG>(q + DP_R1), b = ldq<LDG>(q + DP_R2), c = ldq<LDG>(q + DP_N);
-    p.r1 = L3(a); p.depth = a.w;
+    p.r1 = L3(a);
     p.r2 = L3(b); p.inv_mass = b.w;
     p.n = L3(c); p.bias = c.w;
-    p.i1 = L3(ldq<LDG>(q + DP_I1));
+    const float4 d = ldq<LDG>(q + DP_I1);
+    p.i1 = L3(d); p.bias_pen = d.w;
     p.i2 = L3(ldq<LDG>(q + DP_I2));
 }
 
@@ -317,13 +328,10 @@ RD v3 lin_sub(v3 v, float im, v3 imp, v3 lf) {
 RD v3 lin_add(v3 v, float im, v3 imp, v3 lf) {
     return V(v.x + im * imp.x * lf.x, v.y + im * imp.y * lf.y, v.z + im * imp.z * lf.z);
 }
-// w -= i * af * s  /  w += i * af * s, per component (the point updates)
-RD v3 ang_sub(v3 w, v3 i, v3 af, float s) {
-    return V(w.x - i.x * af.x * s, w.y - i.y * af.y * s, w.z - i.z * af.z * s);
-}
-RD v3 ang_add(v3 w, v3 i, v3 af, float s) {
-    return V(w.x + i.x * af.x * s, w.y + i.y * af.y * s, w.z + i.z * af.z * s);
-}
+// w -= i * af * s  /  w += i * af * s, per component (the point updates; the
+// point rows hold i * af)
+RD v3 ang_sub(v3 w, v3 iaf, float s) { return V(w.x - iaf.x * s, w.y - iaf.y * s, w.z - iaf.z * s); }
+RD v3 ang_add(v3 w, v3 iaf, float s) { return V(w.x + iaf.x * s, w.y + iaf.y * s, w.z + iaf.z * s); }
 
 // Where the solver reads and writes the velocities (constrained and split)
 // of a manifold's two bodies: the global scratch arrays, or a warp's shared
@@ -341,16 +349,17 @@ struct RecSrc {
     const float4* pq;
     float4* pmut;
     int pq_stride, pmut_stride;
+    float2* pm2 = nullptr;   // PRE cores: the impulses (penetration, split), when kept apart from the resting flags in pmut
 };
-constexpr int PREC_F4 = int(sizeof(DynPointRec) / sizeof(float4));
+constexpr int PREC_ROWS = int(sizeof(DynPointRec) / sizeof(float4));
 RD RecSrc rec_global(const DynArgs& a, uint32_t mi, int32_t pstart) {
     RecSrc r;
     r.mq = a.mrec[mi].q;
     r.mmut = &a.mrec[mi].mut;
     r.pq = a.prec[pstart].q;
     r.pmut = &a.prec[pstart].mut;
-    r.pq_stride = PREC_F4;
-    r.pmut_stride = PREC_F4;
+    r.pq_stride = PREC_ROWS;
+    r.pmut_stride = PREC_ROWS;
     return r;
 }
 
@@ -368,13 +377,31 @@ RD BodyVel vel_global(const DynArgs& a, int32_t b1, int32_t b2) {
 // together before the points are solved and stored after, so that copies in
 // global memory cost one round trip; points beyond four (none after the
 // manifold step) are read and written in place.
+RD float4 pm2_load(const RecSrc& r, int k) {
+    const float2 v = r.pm2[k];
+    return make_float4(v.x, v.y, r.pmut[k * r.pmut_stride].z, 0.0f);
+}
 RD void pmv_load(const RecSrc& r, int nb, float4& p0, float4& p1, float4& p2, float4& p3) {
+    if (r.pm2) {
+        if (nb > 0) p0 = pm2_load(r, 0);
+        if (nb > 1) p1 = pm2_load(r, 1);
+        if (nb > 2) p2 = pm2_load(r, 2);
+        if (nb > 3) p3 = pm2_load(r, 3);
+        return;
+    }
     if (nb > 0) p0 = r.pmut[0];
     if (nb > 1) p1 = r.pmut[r.pmut_stride];
     if (nb > 2) p2 = r.pmut[2 * r.pmut_stride];
     if (nb > 3) p3 = r.pmut[3 * r.pmut_stride];
 }
 RD void pmv_store(const RecSrc& r, int nb, const float4& p0, const float4& p1, const float4& p2, const float4& p3) {
+    if (r.pm2) {
+        if (nb > 0) r.pm2[0] = make_float2(p0.x, p0.y);
+        if (nb > 1) r.pm2[1] = make_float2(p1.x, p1.y);
+        if (nb > 2) r.pm2[2] = make_float2(p2.x, p2.y);
+        if (nb > 3) r.pm2[3] = make_float2(p3.x, p3.y);
+        return;
+    }
     if (nb > 0) r.pmut[0] = p0;
     if (nb > 1) r.pmut[r.pmut_stride] = p1;
     if (nb > 2) r.pmut[2 * r.pmut_stride] = p2;
@@ -414,9 +441,9 @@ RD void warm_core(const DynArgs& a, const RecSrc& r, const BodyVel& bv, int32_t 
             const float pi = pm.x;
             const v3 ip = V(p.n.x * pi, p.n.y * pi, p.n.z * pi);
             v1 = lin_sub(v1, c.im1, ip, c.lf1);
-            w1 = ang_sub(w1, p.i1, c.af1, pi);
+            w1 = ang_sub(w1, p.i1, pi);
             v2 = lin_add(v2, c.im2, ip, c.lf2);
-            w2 = ang_add(w2, p.i2, c.af2, pi);
+            w2 = ang_add(w2, p.i2, pi);
         } else {
             pm.x = 0.0f;
             pm_set<PRE>(r, k, pm, pv0, pv1, pv2, pv3);
@@ -465,7 +492,7 @@ RD void warm_manifold(const DynArgs& a, uint32_t mi, const BodyVel& bv, int32_t 
 
 // One solve pass (:479-759) over one manifold.
 template <bool LDG, bool PRE = false>
-RD void solve_core(const DynArgs& a, const RecSrc& r, float beta, const BodyVel& bv, int32_t nb) {
+RD void solve_core(const DynArgs& a, const RecSrc& r, const BodyVel& bv, int32_t nb) {
     if (nb == 0) return;
     Man c;
     load_man_q<LDG>(r.mq, c);
@@ -482,36 +509,30 @@ RD void solve_core(const DynArgs& a, const RecSrc& r, float beta, const BodyVel&
         const v3 n = p.n;
         const v3 dv = rel_velocity(v1, w1, v2, w2, p.r1, p.r2);
         const float Jv = dv.x * n.x + dv.y * n.y + dv.z * n.z;
-        float bias_pen = 0.0f;
-        if (p.depth > SLOP) {
-            const float excess = p.depth - SLOP;
-            bias_pen = -(beta / a.dt) * ((0.0f < excess) ? excess : 0.0f);
-        }
-        const float b = bias_pen + p.bias;
-        float dl = a.split ? -(Jv + p.bias) * p.inv_mass : -(Jv + b) * p.inv_mass;
+        float dl = -(Jv + p.bias) * p.inv_mass;
         const float lt = pm.x;
         const float sum = pm.x + dl;
         pm.x = (sum < 0.0f) ? 0.0f : sum;
         dl = pm.x - lt;
         const v3 li = V(n.x * dl, n.y * dl, n.z * dl);
         v1 = lin_sub(v1, c.im1, li, c.lf1);
-        w1 = ang_sub(w1, p.i1, c.af1, dl);
+        w1 = ang_sub(w1, p.i1, dl);
         v2 = lin_add(v2, c.im2, li, c.lf2);
-        w2 = ang_add(w2, p.i2, c.af2, dl);
+        w2 = ang_add(w2, p.i2, dl);
         sum_pen += pm.x;
         if (a.split) {
             const v3 dvs = rel_velocity(s1, t1, s2, t2, p.r1, p.r2);
             const float Jvs = dvs.x * n.x + dvs.y * n.y + dvs.z * n.z;
-            float dls = -(Jvs + bias_pen) * p.inv_mass;
+            float dls = -(Jvs + p.bias_pen) * p.inv_mass;
             const float lts = pm.y;
             const float ss = pm.y + dls;
             pm.y = (ss < 0.0f) ? 0.0f : ss;
             dls = pm.y - lts;
             const v3 lis = V(n.x * dls, n.y * dls, n.z * dls);
             s1 = lin_sub(s1, c.im1, lis, c.lf1);
-            t1 = ang_sub(t1, p.i1, c.af1, dls);
+            t1 = ang_sub(t1, p.i1, dls);
             s2 = lin_add(s2, c.im2, lis, c.lf2);
-            t2 = ang_add(t2, p.i2, c.af2, dls);
+            t2 = ang_add(t2, p.i2, dls);
         }
         pm_set<PRE>(r, k, pm, pv0, pv1, pv2, pv3);
     }
@@ -568,8 +589,8 @@ RD void solve_core(const DynArgs& a, const RecSrc& r, float beta, const BodyVel&
     if (!(c.fixed & 1)) { *bv.v1 = F4(v1); *bv.w1 = F4(w1); *bv.s1 = F4(s1); *bv.t1 = F4(t1); }
     if (!(c.fixed & 2)) { *bv.v2 = F4(v2); *bv.w2 = F4(w2); *bv.s2 = F4(s2); *bv.t2 = F4(t2); }
 }
-RD void solve_manifold(const DynArgs& a, uint32_t mi, float beta, const BodyVel& bv, int32_t nb, int32_t pstart) {
-    solve_core<true>(a, rec_global(a, mi, pstart), beta, bv, nb);
+RD void solve_manifold(const DynArgs& a, uint32_t mi, const BodyVel& bv, int32_t nb, int32_t pstart) {
+    solve_core<true>(a, rec_global(a, mi, pstart), bv, nb);
 }
 
 // storeImpulses (:763-785) of one manifold.
@@ -611,6 +632,7 @@ RD void store_manifold(const DynArgs& a, uint32_t mi) {
 // it go to kernel 3c, one CTA per island, the island staged in up to the
 // whole opt-in shared memory of a CTA; both come from DynTuning)
 constexpr uint32_t BIG_ISLAND = 64;   // queued first: the longest islands start first
+constexpr uint32_t ISLAND_DONE = 0xffffffffu;   // entry of giant_list solved by kernel 3b
 
 RD int4 man_ids(const DynArgs& a, uint32_t mi) {
     const float4 q = __ldg(a.mrec[mi].q + DQ_IDS);
@@ -640,132 +662,557 @@ __global__ void __launch_bounds__(128) dyn_islands_small(const DynArgs a) {
         const int4 id = man_ids(a, mi);
         warm_manifold(a, mi, vel_global(a, id.x, id.y), id.z, id.w);
     }
-    const float beta = a.split ? BETA_SPLIT_IMPULSE : BETA;
     for (int it = 0; it < a.iterations; it++)
         for (uint32_t mi = m0; mi < m1; mi++) {
             const int4 id = man_ids(a, mi);
-            solve_manifold(a, mi, beta, vel_global(a, id.x, id.y), id.z, id.w);
+            solve_manifold(a, mi, vel_global(a, id.x, id.y), id.z, id.w);
         }
     for (uint32_t mi = m0; mi < m1; mi++) store_manifold(a, mi);
 }
 
+// ---- a manifold on eight lanes --------------------------------------------
+//
+// An island's manifolds form a chain of levels of two or three manifolds
+// each, so a warp that gives every manifold one lane issues the ~1,400
+// instructions of a four-point manifold for two or three active lanes and is
+// bound by its own issue rate.  Here eight lanes share a manifold.  Lanes 0-3
+// solve its constrained velocities and lanes 4-7 its split-impulse velocities
+// (two independent chains until the bodies are stored); in each half lane
+// c < 3 keeps component c of the linear velocities and components c + 1, c + 2
+// of the angular ones (lane 3 repeats lane 0 and stores nothing).  Component c
+// of v + w x r needs exactly those, so the only exchange is the three products
+// of a dot product, read with shuffles and added in the reference's order by
+// every lane: each value goes through the same operations in the same order
+// as in warm_core / solve_core, bit for bit.  Measured on a chain of one
+// manifold a level, cycles a level with 1 / 4 points: one CTA an island
+// 1,562 / 2,392 with a lane a manifold, 1,299 / 1,856 here; one warp an island
+// 2,277 / 4,319 and 1,981 / 2,478.  4,096 captured worlds: 5.28 -> 1.85 ms.
+constexpr uint32_t LANES_PER_MANIFOLD = 8, WARP_MANIFOLDS = 32 / LANES_PER_MANIFOLD;
+// A manifold's rows staged in shared memory: its record's constant rows, then
+// its points' records (the impulse rows among them are the values at staging
+// time; only their resting flags are read).
+struct __align__(16) LaneSlot {
+    float4 mq[DQ_ROWS];
+    float4 pq[4 * PREC_ROWS];
+};
+
+RD void cp_async16(void* smem, const void* gmem) {
+    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+RD void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+RD void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+struct LaneId {
+    uint32_t group;     // manifold of the warp's four
+    uint32_t role;      // 0 constrained, 1 split velocities
+    uint32_t c, c1, c2; // component and the two after it
+    bool writer;
+};
+RD LaneId lane_id(uint32_t lane) {
+    LaneId id;
+    id.group = lane >> 3;
+    id.role = (lane >> 2) & 1u;
+    const uint32_t c = lane & 3u;
+    id.writer = c < 3;
+    id.c = c < 3 ? c : 0u;
+    id.c1 = id.c == 2 ? 0u : id.c + 1;
+    id.c2 = id.c == 0 ? 2u : id.c - 1;
+    return id;
+}
+// (x + y) + z of the three components' products, the same in every lane
+RD float lanes_sum(float p) {
+    const float x = __shfl_sync(0xffffffffu, p, 0, 4), y = __shfl_sync(0xffffffffu, p, 1, 4);
+    const float z = __shfl_sync(0xffffffffu, p, 2, 4);
+    return x + y + z;
+}
+// the same where lane c holds the product of component c + 1
+RD float lanes_sum_next(float p) {
+    const float x = __shfl_sync(0xffffffffu, p, 2, 4), y = __shfl_sync(0xffffffffu, p, 0, 4);
+    const float z = __shfl_sync(0xffffffffu, p, 1, 4);
+    return x + y + z;
+}
+// row of Matrix3x3 * Vector3
+RD float row_dot(const float4& m, v3 v) { return m.x * v.x + m.y * v.y + m.z * v.z; }
+
+// This lane's share of the two bodies' velocities.
+struct LaneVel { float v1, w1a, w1b, v2, w2a, w2b; };
+// b1 / b2: the bodies' rows of the lane's role, the angular row `wofs` floats
+// behind the linear one.
+RD LaneVel lane_vel_load(const float* b1, const float* b2, uint32_t wofs, const LaneId& id) {
+    return LaneVel{b1[id.c], b1[wofs + id.c1], b1[wofs + id.c2], b2[id.c], b2[wofs + id.c1], b2[wofs + id.c2]};
+}
+// every component is stored by one lane (its angular share by c + 1)
+RD void lane_vel_store(float* b1, float* b2, uint32_t wofs, const LaneId& id, uint32_t fixed, const LaneVel& u) {
+    if (!(fixed & 1u)) { b1[id.c] = u.v1; b1[wofs + id.c1] = u.w1a; }
+    if (!(fixed & 2u)) { b2[id.c] = u.v2; b2[wofs + id.c1] = u.w2a; }
+}
+
+// warm_core on eight lanes; the whole warp calls it, `nbw` is the largest
+// point count of the warp's manifolds.  imp[k] is point k's penetration
+// impulse, f the friction impulses (all lanes of the half agree).
+RD void lanes_warm(const float* mq, const float* pq, uint32_t nb, uint32_t nbw, bool active, const LaneId& id,
+                   float* b1, float* b2, uint32_t wofs, float (&imp)[4], float (&f)[3]) {
+    const float4* q = reinterpret_cast<const float4*>(mq);
+    const float4 ms = q[DQ_MASS];
+    const uint32_t fixed = uint32_t(ms.w);
+    const float lf1 = mq[4 * DQ_LF1 + id.c], lf2 = mq[4 * DQ_LF2 + id.c];
+    const float af1a = mq[4 * DQ_AF1 + id.c1], af1b = mq[4 * DQ_AF1 + id.c2];
+    const float af2a = mq[4 * DQ_AF2 + id.c1], af2b = mq[4 * DQ_AF2 + id.c2];
+    LaneVel u = lane_vel_load(b1, b2, wofs, id);
+    bool resting_any = false;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) {
+        if (k >= nbw) break;
+        const float* p = pq + k * 4 * PREC_ROWS;
+        if (k < nb) {
+            if (p[4 * DP_ROWS + 2] != 0.0f) {   // mut.z: resting
+                resting_any = true;
+                const float pi = imp[k];
+                const float ip = p[4 * DP_N + id.c] * pi;
+                u.v1 = u.v1 - ms.x * ip * lf1;
+                u.w1a = u.w1a - p[4 * DP_I1 + id.c1] * pi;
+                u.w1b = u.w1b - p[4 * DP_I1 + id.c2] * pi;
+                u.v2 = u.v2 + ms.y * ip * lf2;
+                u.w2a = u.w2a + p[4 * DP_I2 + id.c1] * pi;
+                u.w2b = u.w2b + p[4 * DP_I2 + id.c2] * pi;
+            } else {
+                imp[k] = 0.0f;
+            }
+        }
+    }
+    if (resting_any) {
+        const v3 o1 = L3(q[DQ_OFV1]), o2 = L3(q[DQ_OFV2]);
+        const v3 fv1 = L3(q[DQ_FV1]), fv2 = L3(q[DQ_FV2]), n = L3(q[DQ_N]);
+        const v3 r1ct1 = L3(q[DQ_R1CT1]), r1ct2 = L3(q[DQ_R1CT2]), r2ct1 = L3(q[DQ_R2CT1]), r2ct2 = L3(q[DQ_R2CT2]);
+        const float4 I1a = q[DQ_I1 + id.c1], I1b = q[DQ_I1 + id.c2], I2a = q[DQ_I2 + id.c1], I2b = q[DQ_I2 + id.c2];
+        const v3 ofi = V(f[0] * o1.x + f[1] * o2.x, f[0] * o1.y + f[1] * o2.y, f[0] * o1.z + f[1] * o2.z);
+        f[0] = vdot(ofi, fv1);
+        f[1] = vdot(ofi, fv2);
+        const float f1 = f[0], f2 = f[1], ftw = f[2];
+        // first friction constraint
+        v3 ai1 = V(-r1ct1.x * f1, -r1ct1.y * f1, -r1ct1.z * f1);
+        float li2 = mq[4 * DQ_FV1 + id.c] * f1;
+        v3 ai2 = V(r2ct1.x * f1, r2ct1.y * f1, r2ct1.z * f1);
+        u.v1 = u.v1 - ms.x * li2 * lf1;
+        u.w1a = u.w1a + af1a * row_dot(I1a, ai1); u.w1b = u.w1b + af1b * row_dot(I1b, ai1);
+        u.v2 = u.v2 + ms.y * li2 * lf2;
+        u.w2a = u.w2a + af2a * row_dot(I2a, ai2); u.w2b = u.w2b + af2b * row_dot(I2b, ai2);
+        // second friction constraint
+        ai1 = V(-r1ct2.x * f2, -r1ct2.y * f2, -r1ct2.z * f2);
+        li2 = mq[4 * DQ_FV2 + id.c] * f2;
+        ai2 = V(r2ct2.x * f2, r2ct2.y * f2, r2ct2.z * f2);
+        u.v1 = u.v1 - ms.x * li2 * lf1;
+        u.w1a = u.w1a + af1a * row_dot(I1a, ai1); u.w1b = u.w1b + af1b * row_dot(I1b, ai1);
+        u.v2 = u.v2 + ms.y * li2 * lf2;
+        u.w2a = u.w2a + af2a * row_dot(I2a, ai2); u.w2b = u.w2b + af2b * row_dot(I2b, ai2);
+        // twist friction constraint (both bodies a second time, as warm_core)
+        ai1 = V(-n.x * ftw, -n.y * ftw, -n.z * ftw);
+        ai2 = V(n.x * ftw, n.y * ftw, n.z * ftw);
+        u.w1a = u.w1a + af1a * row_dot(I1a, ai1); u.w1b = u.w1b + af1b * row_dot(I1b, ai1);
+        u.w2a = u.w2a + af2a * row_dot(I2a, ai2); u.w2b = u.w2b + af2b * row_dot(I2b, ai2);
+        u.w1a = u.w1a - af1a * row_dot(I1a, ai2); u.w1b = u.w1b - af1b * row_dot(I1b, ai2);
+        u.w2a = u.w2a + af2a * row_dot(I2a, ai2); u.w2b = u.w2b + af2b * row_dot(I2b, ai2);
+    } else {
+        f[0] = f[1] = f[2] = 0.0f;
+    }
+    __syncwarp();   // every lane has read its share (lanes_solve: its shuffles)
+    if (active && id.writer && id.role == 0) lane_vel_store(b1, b2, wofs, id, fixed, u);
+}
+
+// A point's rows as one lane needs them.
+struct LanePt { float n, r1a, r1b, r2a, r2b, i1a, i1b, i2a, i2b, inv_mass, bias; };
+RD LanePt lane_pt(const float* p, const LaneId& id) {
+    LanePt t;
+    t.r1a = p[4 * DP_R1 + id.c1]; t.r1b = p[4 * DP_R1 + id.c2];
+    t.r2a = p[4 * DP_R2 + id.c1]; t.r2b = p[4 * DP_R2 + id.c2];
+    t.n = p[4 * DP_N + id.c];
+    t.bias = p[id.role ? 4 * DP_I1 + 3 : 4 * DP_N + 3];
+    t.inv_mass = p[4 * DP_R2 + 3];
+    t.i1a = p[4 * DP_I1 + id.c1]; t.i1b = p[4 * DP_I1 + id.c2];
+    t.i2a = p[4 * DP_I2 + id.c1]; t.i2b = p[4 * DP_I2 + id.c2];
+    return t;
+}
+
+// solve_core on eight lanes (split: the stage's split-impulse switch); imp[k]
+// is the lane's role's impulse of point k.  A point's rows are read while the
+// one before it is solved (a LaneSlot has rows for four points: those of
+// points the manifold does not have are read and discarded).
+RD void lanes_solve(bool split, const float* mq, const float* pq, uint32_t nb, uint32_t nbw, bool active,
+                    const LaneId& id, float* b1, float* b2, uint32_t wofs, float (&imp)[4], float (&f)[3]) {
+    const float4* q = reinterpret_cast<const float4*>(mq);
+    LaneVel u = lane_vel_load(b1, b2, wofs, id);
+    LanePt next = lane_pt(pq, id);
+    const float4 ms = q[DQ_MASS];
+    const uint32_t fixed = uint32_t(ms.w);
+    const float lf1 = mq[4 * DQ_LF1 + id.c], lf2 = mq[4 * DQ_LF2 + id.c];
+    float sum_pen = 0.0f;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) {
+        if (k >= nbw) break;
+        const LanePt p = next;
+        if (k < 3) next = lane_pt(pq + (k + 1) * 4 * PREC_ROWS, id);
+        const float dv = u.v2 + u.w2a * p.r2b - u.w2b * p.r2a - u.v1 - u.w1a * p.r1b + u.w1b * p.r1a;
+        const float Jv = lanes_sum(dv * p.n);
+        float dl = -(Jv + p.bias) * p.inv_mass;
+        const float sum = imp[k] + dl;
+        const float now = (sum < 0.0f) ? 0.0f : sum;
+        dl = now - imp[k];
+        const float li = p.n * dl;
+        LaneVel t;
+        t.v1 = u.v1 - ms.x * li * lf1;
+        t.w1a = u.w1a - p.i1a * dl; t.w1b = u.w1b - p.i1b * dl;
+        t.v2 = u.v2 + ms.y * li * lf2;
+        t.w2a = u.w2a + p.i2a * dl; t.w2b = u.w2b + p.i2b * dl;
+        if (k < nb) {
+            u = t;
+            imp[k] = now;
+            sum_pen += now;
+        }
+    }
+    const float af1a = mq[4 * DQ_AF1 + id.c1], af1b = mq[4 * DQ_AF1 + id.c2];
+    const float af2a = mq[4 * DQ_AF2 + id.c1], af2b = mq[4 * DQ_AF2 + id.c2];
+    const float t1 = mq[4 * DQ_FV1 + id.c], t2 = mq[4 * DQ_FV2 + id.c], nt = mq[4 * DQ_N + id.c1];
+    const v3 r1ct1 = L3(q[DQ_R1CT1]), r1ct2 = L3(q[DQ_R1CT2]), r2ct1 = L3(q[DQ_R2CT1]), r2ct2 = L3(q[DQ_R2CT2]);
+    const float4 I1a = q[DQ_I1 + id.c1], I1b = q[DQ_I1 + id.c2], I2a = q[DQ_I2 + id.c1], I2b = q[DQ_I2 + id.c2];
+    const float f1a = mq[4 * DQ_R1F + id.c1], f1b = mq[4 * DQ_R1F + id.c2], inv_f1 = mq[4 * DQ_R1F + 3];
+    const float f2a = mq[4 * DQ_R2F + id.c1], f2b = mq[4 * DQ_R2F + id.c2], inv_f2 = mq[4 * DQ_R2F + 3];
+    const float4 nq = q[DQ_N];
+    // the split half ends here: what it computes below is discarded
+    const LaneVel us = u;
+    const float limit = ms.z * sum_pen;
+    // first friction constraint
+    {
+        const float dv = u.v2 + u.w2a * f2b - u.w2b * f2a - u.v1 - u.w1a * f1b + u.w1b * f1a;
+        float dl = -lanes_sum(dv * t1) * inv_f1;
+        const float lt = f[0];
+        f[0] = smax(-limit, smin(lt + dl, limit));
+        dl = f[0] - lt;
+        const v3 ai1 = V(-r1ct1.x * dl, -r1ct1.y * dl, -r1ct1.z * dl), ai2 = V(r2ct1.x * dl, r2ct1.y * dl, r2ct1.z * dl);
+        const float li2 = t1 * dl;
+        u.v1 = u.v1 - ms.x * li2 * lf1;
+        u.w1a = u.w1a + af1a * row_dot(I1a, ai1); u.w1b = u.w1b + af1b * row_dot(I1b, ai1);
+        u.v2 = u.v2 + ms.y * li2 * lf2;
+        u.w2a = u.w2a + af2a * row_dot(I2a, ai2); u.w2b = u.w2b + af2b * row_dot(I2b, ai2);
+    }
+    // second friction constraint
+    {
+        const float dv = u.v2 + u.w2a * f2b - u.w2b * f2a - u.v1 - u.w1a * f1b + u.w1b * f1a;
+        float dl = -lanes_sum(dv * t2) * inv_f2;
+        const float lt = f[1];
+        f[1] = smax(-limit, smin(lt + dl, limit));
+        dl = f[1] - lt;
+        const v3 ai1 = V(-r1ct2.x * dl, -r1ct2.y * dl, -r1ct2.z * dl), ai2 = V(r2ct2.x * dl, r2ct2.y * dl, r2ct2.z * dl);
+        const float li2 = t2 * dl;
+        u.v1 = u.v1 - ms.x * li2 * lf1;
+        u.w1a = u.w1a + af1a * row_dot(I1a, ai1); u.w1b = u.w1b + af1b * row_dot(I1b, ai1);
+        u.v2 = u.v2 + ms.y * li2 * lf2;
+        u.w2a = u.w2a + af2a * row_dot(I2a, ai2); u.w2b = u.w2b + af2b * row_dot(I2b, ai2);
+    }
+    // twist friction constraint
+    {
+        const float Jv = lanes_sum_next((u.w2a - u.w1a) * nt);
+        float dl = -Jv * nq.w;
+        const float lt = f[2];
+        f[2] = smax(-limit, smin(lt + dl, limit));
+        dl = f[2] - lt;
+        const v3 ai2 = V(nq.x * dl, nq.y * dl, nq.z * dl);
+        u.w1a = u.w1a - af1a * row_dot(I1a, ai2); u.w1b = u.w1b - af1b * row_dot(I1b, ai2);
+        u.w2a = u.w2a + af2a * row_dot(I2a, ai2); u.w2b = u.w2b + af2b * row_dot(I2b, ai2);
+    }
+    if (id.role) u = us;
+    if (active && id.writer && (id.role == 0 || split)) lane_vel_store(b1, b2, wofs, id, fixed, u);
+}
+
+// ---- level schedule of one island (one warp) --------------------------------
+//
+// A manifold's level is one more than the latest level of its movable bodies;
+// every body of the island gets a slot for its velocities (fixed bodies too:
+// their slots are read, never written back).  32 manifolds at a time: the
+// lanes look their bodies up in a shared hash (compare-and-swap insertion; a
+// slot's number follows the races, which decides where a velocity is staged
+// and nothing else), then a 32-step shuffle scan settles the levels in
+// manifold order, then a stable counting sort by level.  (One lane doing this
+// serially took ~250 cycles a manifold.)
+struct IslandSched {
+    int32_t* hkey;        // H entries: body (-1 empty)
+    uint32_t* hval;       // slot << 16 | last level
+    int32_t* slot_body;   // nbmax: body of each slot, -1 - body when fixed
+    short2* slot;         // per manifold: slot of body 1 / body 2
+    uint16_t *klev, *order, *lev;   // level, level order, start of each level (lev[depth] = cnt)
+    uint32_t H, nbmax;
+    uint32_t* nslots;     // shared counter
+};
+
+RD uint32_t sched_find(const IslandSched& S, int32_t b, bool fixed, bool& ok) {
+    uint32_t h = (uint32_t(b) * 2654435761u >> 12) & (S.H - 1);
+    for (uint32_t probe = 0; probe < S.H; probe++, h = (h + 1) & (S.H - 1)) {
+        const int32_t k = atomicCAS(S.hkey + h, -1, b);
+        if (k == b) return h;
+        if (k < 0) {
+            const uint32_t s = atomicAdd(S.nslots, 1u);
+            if (s >= S.nbmax) { ok = false; return h; }
+            S.hval[h] = s << 16;
+            S.slot_body[s] = fixed ? -1 - b : b;
+            return h;
+        }
+    }
+    ok = false;
+    return 0;
+}
+
+// False (nothing written to global memory) when the island has more bodies
+// than slots.
+RD bool island_schedule(const DynArgs& a, uint32_t m0, uint32_t cnt, const IslandSched& S, uint32_t lane, uint32_t& depth) {
+    for (uint32_t h = lane; h < S.H; h += 32) S.hkey[h] = -1;
+    if (lane == 0) *S.nslots = 0;
+    __syncwarp();
+    depth = 0;
+    bool ok = true;
+    for (uint32_t base = 0; base < cnt; base += 32) {
+        const uint32_t k = base + lane;
+        int32_t b1 = -1, b2 = -1;   // movable bodies (the scan's keys)
+        uint32_t h1 = 0, h2 = 0;
+        bool used = false;
+        if (k < cnt) {
+            const int4 id = man_ids(a, m0 + k);
+            if (id.z != 0) {
+                const uint32_t fixed = man_fixed(a, m0 + k);
+                used = true;
+                h1 = sched_find(S, id.x, (fixed & 1u) != 0, ok);
+                h2 = sched_find(S, id.y, (fixed & 2u) != 0, ok);
+                b1 = (fixed & 1u) ? -1 : id.x;
+                b2 = (fixed & 2u) ? -1 : id.y;
+            }
+        }
+        if (__any_sync(0xffffffffu, !ok)) return false;
+        __syncwarp();
+        const uint32_t e1 = used ? S.hval[h1] : 0u, e2 = used ? S.hval[h2] : 0u;
+        uint32_t l1 = b1 >= 0 ? e1 & 0xffffu : 0u, l2 = b2 >= 0 ? e2 & 0xffffu : 0u, L = 1;
+        bool last1 = true, last2 = true;
+        const uint32_t steps = cnt - base < 32 ? cnt - base : 32u;
+        for (uint32_t j = 0; j < steps; j++) {
+            if (lane == j) L = 1 + (l1 > l2 ? l1 : l2);
+            const uint32_t Lj = __shfl_sync(0xffffffffu, L, int(j));
+            const int32_t c1 = __shfl_sync(0xffffffffu, b1, int(j)), c2 = __shfl_sync(0xffffffffu, b2, int(j));
+            const bool m1 = b1 >= 0 && (b1 == c1 || b1 == c2), m2 = b2 >= 0 && (b2 == c1 || b2 == c2);
+            if (lane > j) {
+                if (m1) l1 = Lj;
+                if (m2) l2 = Lj;
+            } else if (lane < j) {
+                if (m1) last1 = false;
+                if (m2) last2 = false;
+            }
+        }
+        if (k < cnt) {
+            if (b1 >= 0 && last1) S.hval[h1] = (e1 & 0xffff0000u) | L;
+            if (b2 >= 0 && last2) S.hval[h2] = (e2 & 0xffff0000u) | L;
+            S.slot[k] = used ? make_short2(short(e1 >> 16), short(e2 >> 16)) : make_short2(0, 0);
+            S.klev[k] = uint16_t(L);
+            depth = L > depth ? L : depth;
+        }
+        __syncwarp();
+    }
+    depth = __reduce_max_sync(0xffffffffu, depth);
+    for (uint32_t L = lane; L <= depth; L += 32) S.lev[L] = 0;
+    __syncwarp();
+    const uint32_t lt = (1u << lane) - 1u;
+    // manifolds per level (the lowest lane of a level's peers adds them), scan, scatter
+    for (uint32_t base = 0; base < cnt; base += 32) {
+        const uint32_t k = base + lane;
+        const uint32_t L = k < cnt ? S.klev[k] : 0u;
+        const uint32_t peers = __match_any_sync(0xffffffffu, L);
+        if (k < cnt && (peers & lt) == 0) S.lev[L - 1] = uint16_t(S.lev[L - 1] + __popc(peers));
+        __syncwarp();
+    }
+    uint32_t run = 0;
+    for (uint32_t base = 0; base < depth; base += 32) {
+        const uint32_t L = base + lane;
+        const uint32_t v = L < depth ? S.lev[L] : 0u;
+        uint32_t inc = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= uint32_t(o)) inc += t;
+        }
+        if (L < depth) S.lev[L] = uint16_t(run + inc - v);
+        run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    __syncwarp();
+    for (uint32_t base = 0; base < cnt; base += 32) {
+        const uint32_t k = base + lane;
+        const uint32_t L = k < cnt ? S.klev[k] : 0u;
+        const uint32_t peers = __match_any_sync(0xffffffffu, L);
+        const uint32_t at = k < cnt ? S.lev[L - 1] : 0u;
+        __syncwarp();
+        if (k < cnt) {
+            S.order[at + __popc(peers & lt)] = uint16_t(k);
+            if ((peers & lt) == 0) S.lev[L - 1] = uint16_t(at + __popc(peers));
+        }
+        __syncwarp();
+    }
+    // lev[L] is now the end of level L: shift to the starts
+    for (uint32_t top = depth; top > 0;) {
+        const uint32_t n = top < 32 ? top : 32u;   // positions top - n + 1 .. top take their predecessors' ends
+        const uint32_t p = top - n + 1 + lane;
+        const uint16_t v = lane < n ? S.lev[p - 1] : uint16_t(0);
+        __syncwarp();
+        if (lane < n) S.lev[p] = v;
+        __syncwarp();
+        top -= n;
+    }
+    if (lane == 0) S.lev[0] = 0;
+    __syncwarp();
+    return true;
+}
+
 // Shared memory of one warp of kernel 3b.
-constexpr uint32_t STAGE_HASH = 2 * STAGE_BODIES;   // open addressing, load <= 1/2
-struct WarpStage {
-    float4 vel[4][STAGE_BODIES];        // constrained v, w and split v, w of the staged bodies
-    int4 man[STAGE_MANIFOLDS];          // body 1, body 2, points, first point
-    short2 slot[STAGE_MANIFOLDS];       // slot of body 1 / body 2 (-1: fixed body)
+constexpr uint32_t STAGE_HASH = 512;   // open addressing over at most STAGE_BODIES bodies
+struct __align__(16) WarpStage {
+    float4 vel[4][STAGE_BODIES];        // constrained v, w and split v, w of the island's bodies
+    union {
+        struct {
+            int32_t hkey[STAGE_HASH];
+            uint32_t hval[STAGE_HASH];
+            uint16_t klev[STAGE_MANIFOLDS];
+            short2 slot[STAGE_MANIFOLDS];
+        } s;                                 // while the schedule is built
+        LaneSlot ring[2][WARP_MANIFOLDS];    // while it is solved
+    };
+    int4 desc[STAGE_MANIFOLDS];         // by level: slot 1 | slot 2 << 16, points, manifold (island index), first point
     uint16_t order[STAGE_MANIFOLDS];    // island manifolds sorted by level
-    uint16_t lev[STAGE_MANIFOLDS];      // start of each level
-    uint16_t klev[STAGE_MANIFOLDS];     // level of each manifold
-    int32_t hkey[STAGE_HASH];           // body id (-1 empty)
-    uint32_t hval[STAGE_HASH];          // slot << 16 | last level
-    int32_t slot_body[STAGE_BODIES];    // body of each slot
+    uint16_t lev[STAGE_MANIFOLDS + 8];  // start of each level
+    int32_t slot_body[STAGE_BODIES];    // body of each slot (-1 - body: fixed)
+    uint32_t nslots;
 };
 static_assert(sizeof(WarpStage) <= LARGE_WARP_SMEM, "warp stage");
 
-// Slot and last level of a movable body (inserted on first use); false when
-// the island has more movable bodies than the stage holds.
-RD bool stage_body(WarpStage* st, int32_t b, uint32_t& nslots, uint32_t& idx) {
-    uint32_t h = (uint32_t(b) * 2654435761u) >> 23;   // 9 bits: STAGE_HASH = 512
-    for (uint32_t probe = 0; probe < STAGE_HASH; probe++, h = (h + 1) & (STAGE_HASH - 1)) {
-        const int32_t k = st->hkey[h];
-        if (k == b) { idx = h; return true; }
-        if (k < 0) {
-            if (nslots >= STAGE_BODIES) return false;
-            st->hkey[h] = b;
-            st->hval[h] = nslots << 16;
-            st->slot_body[nslots] = b;
-            nslots++;
-            idx = h;
-            return true;
-        }
+// A level's manifolds are taken four at a time (a chunk: order[pos .. end)).
+struct LaneChunk { uint32_t pos, end, L; };
+RD LaneChunk chunk_next(const WarpStage* st, LaneChunk c, uint32_t depth, bool& wrapped) {
+    wrapped = false;
+    c.pos += WARP_MANIFOLDS;
+    if (c.pos >= c.end) {
+        if (++c.L == depth) { c.L = 0; wrapped = true; }
+        c.pos = st->lev[c.L];
+        c.end = st->lev[c.L + 1];
     }
-    return false;
+    return c;
+}
+// A lane group's manifold of a chunk (desc row; no points: none) with its
+// impulses, read one chunk ahead (only the manifold itself writes them).
+struct LaneJob {
+    int4 d;
+    float imp[4], f[3];
+};
+RD int4 chunk_desc(const WarpStage* st, const LaneChunk& c, const LaneId& id) {
+    const uint32_t at = c.pos + id.group;
+    return at < c.end ? st->desc[at] : make_int4(0, 0, 0, 0);
+}
+RD void job_load(const DynArgs& a, uint32_t m0, const int4& d, const LaneId& id, LaneJob& j) {
+    j.d = d;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++)
+        j.imp[k] = k < uint32_t(d.y) ? reinterpret_cast<const float*>(&a.prec[d.w + k].mut)[id.role] : 0.0f;
+    const float4 mut = d.y ? a.mrec[m0 + uint32_t(d.z)].mut : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    j.f[0] = mut.x; j.f[1] = mut.y; j.f[2] = mut.z;
+}
+// Each lane group stages its own manifold's rows.
+RD void chunk_stage(const DynArgs& a, uint32_t m0, LaneSlot* slot, const int4& d, uint32_t lane) {
+    if (d.y) {
+        const uint32_t sub = lane & 7u;
+        const float4* mq = a.mrec[m0 + uint32_t(d.z)].q;
+#pragma unroll
+        for (uint32_t r = 0; r < DQ_ROWS; r += 8)
+            if (r + sub < DQ_ROWS) cp_async16(&slot->mq[r + sub], mq + r + sub);
+        const float4* pq = a.prec[d.w].q;
+        const uint32_t rows = uint32_t(d.y) * PREC_ROWS;
+#pragma unroll
+        for (uint32_t r = 0; r < 4 * PREC_ROWS; r += 8)
+            if (r + sub < rows) cp_async16(&slot->pq[r + sub], pq + r + sub);
+    }
+    cp_async_commit();
 }
 
-// Schedule of a staged island in shared memory; false if it does not fit.
-RD bool schedule_staged(const DynArgs& a, uint32_t m0, uint32_t cnt, WarpStage* st, uint32_t lane,
-                        uint32_t& depth, uint32_t& nslots) {
-    for (uint32_t h = lane; h < STAGE_HASH; h += 32) st->hkey[h] = -1;
-    for (uint32_t k = lane; k < cnt; k += 32) {
-        int4 id = man_ids(a, m0 + k);
-        const uint32_t fixed = man_fixed(a, m0 + k);
-        // fixed bodies are marked by a negative id in the table
-        if (fixed & 1) id.x = -1 - id.x;
-        if (fixed & 2) id.y = -1 - id.y;
-        st->man[k] = id;
-    }
-    __syncwarp();
-    bool ok = true;
-    if (lane == 0) {
-        depth = 0;
-        nslots = 0;
-        for (uint32_t k = 0; k < cnt && ok; k++) {
-            const int4 id = st->man[k];
-            uint32_t L = 1;
-            short2 sl = make_short2(-1, -1);
-            if (id.z != 0) {
-                uint32_t h1 = 0, h2 = 0, l1 = 0, l2 = 0;
-                if (id.x >= 0) { ok = stage_body(st, id.x, nslots, h1); if (ok) { l1 = st->hval[h1] & 0xffffu; sl.x = short(st->hval[h1] >> 16); } }
-                if (ok && id.y >= 0) { ok = stage_body(st, id.y, nslots, h2); if (ok) { l2 = st->hval[h2] & 0xffffu; sl.y = short(st->hval[h2] >> 16); } }
-                if (!ok) break;
-                L = 1 + (l1 > l2 ? l1 : l2);
-                if (id.x >= 0) st->hval[h1] = (st->hval[h1] & 0xffff0000u) | L;
-                if (id.y >= 0) st->hval[h2] = (st->hval[h2] & 0xffff0000u) | L;
-            }
-            st->slot[k] = sl;
-            st->klev[k] = uint16_t(L);
-            depth = L > depth ? L : depth;
-        }
-        if (ok) {
-            for (uint32_t L = 0; L < depth; L++) st->lev[L] = 0;
-            for (uint32_t k = 0; k < cnt; k++) st->lev[st->klev[k] - 1]++;
-            uint32_t run = 0;
-            for (uint32_t L = 0; L < depth; L++) { run += st->lev[L]; st->lev[L] = uint16_t(run); }
-            for (uint32_t k = cnt; k-- > 0;) st->order[--st->lev[st->klev[k] - 1]] = uint16_t(k);
-        }
-    }
-    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-    depth = __shfl_sync(0xffffffffu, depth, 0);
-    nslots = __shfl_sync(0xffffffffu, nslots, 0);
-    __syncwarp();
-    return ok;
-}
-
-RD void solve_staged(const DynArgs& a, uint32_t m0, uint32_t cnt, WarpStage* st, uint32_t lane, uint32_t depth,
-                     uint32_t nslots) {
+// Solves a scheduled island from the warp's stage: the rows of the next
+// chunk arrive by cp.async while a chunk is solved.
+RD void solve_staged(const DynArgs& a, uint32_t m0, uint32_t cnt, WarpStage* st, uint32_t lane, uint32_t depth) {
+    const uint32_t nslots = st->nslots;
     for (uint32_t s = lane; s < nslots; s += 32) {
-        const int32_t b = st->slot_body[s];
+        const int32_t e = st->slot_body[s], b = e < 0 ? -1 - e : e;
         st->vel[0][s] = a.cv[b]; st->vel[1][s] = a.cw[b];
         st->vel[2][s] = a.sv[b]; st->vel[3][s] = a.sw[b];
     }
+    for (uint32_t k = lane; k < cnt; k += 32) {
+        const uint32_t kk = st->order[k];
+        const int4 id = man_ids(a, m0 + kk);
+        const short2 sl = st->s.slot[kk];
+        st->desc[k] = make_int4(int(uint32_t(uint16_t(sl.x)) | (uint32_t(uint16_t(sl.y)) << 16)), id.z, int(kk), id.w);
+    }
+    __syncwarp();   // the schedule's part of the union is free now
+    const LaneId id = lane_id(lane);
+    float* vel = reinterpret_cast<float*>(st->vel[2 * id.role]);
+    constexpr uint32_t wofs = 4 * STAGE_BODIES;
+    LaneChunk c{0, st->lev[1], 0};
+    // a pass of one chunk reads its impulses after they are stored
+    const bool single = depth == 1 && cnt <= WARP_MANIFOLDS;
+    int pass = 0;
+    uint32_t buf = 0;
+    LaneJob job, nxt;
+    job_load(a, m0, chunk_desc(st, c, id), id, job);
+    chunk_stage(a, m0, &st->ring[0][id.group], job.d, lane);
+    cp_async_wait<0>();
     __syncwarp();
-    const float beta = a.split ? BETA_SPLIT_IMPULSE : BETA;
-    for (int pass = 0; pass <= a.iterations; pass++) {
-        for (uint32_t L = 0; L < depth; L++) {
-            const uint32_t b = st->lev[L];
-            const uint32_t e = (L + 1 < depth) ? st->lev[L + 1] : cnt;
-            for (uint32_t k = b + lane; k < e; k += 32) {
-                const uint32_t kk = st->order[k];
-                const int4 id = st->man[kk];
-                const short2 sl = st->slot[kk];
-                BodyVel bv;
-                if (sl.x >= 0) { bv.v1 = &st->vel[0][sl.x]; bv.w1 = &st->vel[1][sl.x]; bv.s1 = &st->vel[2][sl.x]; bv.t1 = &st->vel[3][sl.x]; }
-                else { const int32_t b1 = -1 - id.x; bv.v1 = a.cv + b1; bv.w1 = a.cw + b1; bv.s1 = a.sv + b1; bv.t1 = a.sw + b1; }
-                if (sl.y >= 0) { bv.v2 = &st->vel[0][sl.y]; bv.w2 = &st->vel[1][sl.y]; bv.s2 = &st->vel[2][sl.y]; bv.t2 = &st->vel[3][sl.y]; }
-                else { const int32_t b2 = -1 - id.y; bv.v2 = a.cv + b2; bv.w2 = a.cw + b2; bv.s2 = a.sv + b2; bv.t2 = a.sw + b2; }
-                if (pass == 0) warm_manifold(a, m0 + kk, bv, id.z, id.w);
-                else solve_manifold(a, m0 + kk, beta, bv, id.z, id.w);
+    for (;;) {
+        bool wrapped;
+        const LaneChunk cn = chunk_next(st, c, depth, wrapped);
+        const int pass_n = pass + (wrapped ? 1 : 0);
+        const bool more = pass_n <= a.iterations;
+        const int4 dn = chunk_desc(st, cn, id);
+        if (more) chunk_stage(a, m0, &st->ring[buf ^ 1][id.group], dn, lane);
+        if (more && !single) job_load(a, m0, dn, id, nxt);
+        const LaneSlot* sl = &st->ring[buf][id.group];
+        const float *mq = reinterpret_cast<const float*>(sl->mq), *pq = reinterpret_cast<const float*>(sl->pq);
+        const uint32_t nb = uint32_t(job.d.y);
+        const bool active = nb != 0;
+        float *b1 = vel + 4 * (job.d.x & 0xffff), *b2 = vel + 4 * int(uint32_t(job.d.x) >> 16);
+        const uint32_t nbw = __reduce_max_sync(0xffffffffu, nb);
+        if (pass == 0) lanes_warm(mq, pq, nb, nbw, active, id, b1, b2, wofs, job.imp, job.f);
+        else lanes_solve(a.split != 0, mq, pq, nb, nbw, active, id, b1, b2, wofs, job.imp, job.f);
+        if (active && (lane & 3u) == 0 && (id.role == 0 || (pass != 0 && a.split))) {
+            DynPointRec* pr = a.prec + job.d.w;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; k++)
+                if (k < nb) reinterpret_cast<float*>(&pr[k].mut)[id.role] = job.imp[k];
+            if (id.role == 0) {
+                float* mut = reinterpret_cast<float*>(&a.mrec[m0 + uint32_t(job.d.z)].mut);
+                mut[0] = job.f[0]; mut[1] = job.f[1]; mut[2] = job.f[2];
             }
-            __syncwarp();
         }
+        cp_async_wait<0>();
+        __syncwarp();
+        if (!more) break;
+        if (single) job_load(a, m0, dn, id, nxt);
+        c = cn;
+        pass = pass_n;
+        buf ^= 1;
+        job = nxt;
     }
     for (uint32_t s = lane; s < nslots; s += 32) {
         const int32_t b = st->slot_body[s];
+        if (b < 0) continue;
         a.cv[b] = st->vel[0][s]; a.cw[b] = st->vel[1][s];
         a.sv[b] = st->vel[2][s]; a.sw[b] = st->vel[3][s];
     }
+}
+
+RD bool schedule_staged(const DynArgs& a, uint32_t m0, uint32_t cnt, WarpStage* st, uint32_t lane, uint32_t& depth) {
+    IslandSched S;
+    S.hkey = st->s.hkey; S.hval = st->s.hval; S.H = STAGE_HASH;
+    S.slot_body = st->slot_body; S.nbmax = STAGE_BODIES;
+    S.slot = st->s.slot; S.klev = st->s.klev; S.order = st->order; S.lev = st->lev;
+    S.nslots = &st->nslots;
+    return island_schedule(a, m0, cnt, S, lane, depth);
 }
 
 // Islands too large for the stage: the same schedule in global scratch.
@@ -810,7 +1257,6 @@ RD void solve_global(const DynArgs& a, uint32_t m0, uint32_t cnt, uint32_t lane)
     }
     depth = __shfl_sync(0xffffffffu, depth, 0);
     __syncwarp();
-    const float beta = a.split ? BETA_SPLIT_IMPULSE : BETA;
     for (int pass = 0; pass <= a.iterations; pass++) {
         for (uint32_t L = 0; L < depth; L++) {
             const uint32_t b = lev[L];
@@ -819,7 +1265,7 @@ RD void solve_global(const DynArgs& a, uint32_t m0, uint32_t cnt, uint32_t lane)
                 const uint32_t mi = m0 + ord[k];
                 const int4 id = man_ids(a, mi);
                 if (pass == 0) warm_manifold(a, mi, vel_global(a, id.x, id.y), id.z, id.w);
-                else solve_manifold(a, mi, beta, vel_global(a, id.x, id.y), id.z, id.w);
+                else solve_manifold(a, mi, vel_global(a, id.x, id.y), id.z, id.w);
             }
             __syncwarp();
         }
@@ -830,6 +1276,29 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32, 2) dyn_islands_large(const D
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WarpStage* st = reinterpret_cast<WarpStage*>(smem_raw + size_t(wid) * LARGE_WARP_SMEM);
+    // Giant islands that fit a warp's stage are taken here, the longest work
+    // first, when there are more of them than CTAs of kernel 3c (one each):
+    // 300 chains of 300 manifolds took 6.4 ms as CTAs (three rounds of 148),
+    // 2.7 ms as warps; 148 or fewer are faster as CTAs.
+    const uint32_t n_giant = a.counters[3];
+    if (n_giant > a.giant_ctas) {
+        for (;;) {
+            uint32_t k = 0;
+            if (lane == 0) k = atomicAdd(a.counters + 7, 1u);
+            k = __shfl_sync(0xffffffffu, k, 0);
+            if (k >= n_giant) break;
+            const uint32_t is = a.giant_list[k];
+            const uint32_t m0 = a.i_start[is], cnt = a.i_count[is];
+            uint32_t depth = 0;
+            if (cnt <= STAGE_MANIFOLDS && schedule_staged(a, m0, cnt, st, lane, depth)) {
+                solve_staged(a, m0, cnt, st, lane, depth);
+                __syncwarp();
+                for (uint32_t j = lane; j < cnt; j += 32) store_manifold(a, m0 + j);
+                if (lane == 0) a.giant_list[k] = ISLAND_DONE;
+            }
+            __syncwarp();
+        }
+    }
     const uint32_t n_big = a.counters[0], n_mid = a.counters[2];
     for (;;) {
         uint32_t k = 0;
@@ -838,11 +1307,10 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32, 2) dyn_islands_large(const D
         if (k >= n_big + n_mid) break;
         const uint32_t is = k < n_big ? a.large_list[k] : a.large_list[a.ni - 1 - (k - n_big)];
         const uint32_t m0 = a.i_start[is], cnt = a.i_count[is];
-        uint32_t depth = 0, nslots = 0;
-        if (cnt <= STAGE_MANIFOLDS && schedule_staged(a, m0, cnt, st, lane, depth, nslots))
-            solve_staged(a, m0, cnt, st, lane, depth, nslots);
-        else
-            solve_global(a, m0, cnt, lane);
+        uint32_t depth = 0;
+        if (cnt <= STAGE_MANIFOLDS && schedule_staged(a, m0, cnt, st, lane, depth)) solve_staged(a, m0, cnt, st, lane, depth);
+        else solve_global(a, m0, cnt, lane);
+        __syncwarp();
         for (uint32_t j = lane; j < cnt; j += 32) store_manifold(a, m0 + j);
         __syncwarp();
     }
@@ -882,12 +1350,11 @@ __global__ void __launch_bounds__(64) dyn_islands_joint(const DynArgs a) {
         warm_manifold(a, mi, vel_global(a, id.x, id.y), id.z, id.w);
     }
     for (uint32_t j = j0; j < j0 + jn; j++) joint_warm(a, a.j_list[j]);
-    const float beta = a.split ? BETA_SPLIT_IMPULSE : BETA;
     for (int it = 0; it < a.iterations; it++) {
         for (uint32_t j = j0; j < j0 + jn; j++) joint_solve(a, a.j_list[j]);
         for (uint32_t mi = m0; mi < m0 + cnt; mi++) {
             const int4 id = man_ids(a, mi);
-            solve_manifold(a, mi, beta, vel_global(a, id.x, id.y), id.z, id.w);
+            solve_manifold(a, mi, vel_global(a, id.x, id.y), id.z, id.w);
         }
     }
     for (uint32_t mi = m0; mi < m0 + cnt; mi++) store_manifold(a, mi);
@@ -932,32 +1399,33 @@ __global__ void __launch_bounds__(64) dyn_joints_position(const DynArgs a) {
 // warm_core / solve_core, the same as the other paths: only where the rows and
 // impulses live changes.  An island that does not fit falls back to the
 // schedule in global scratch (solve_global), run by warp 0.
-constexpr uint32_t GIANT_RING = 8;     // manifolds of a level staged (the first 8)
+constexpr uint32_t GIANT_SOLVERS = 4;  // solver warps; the warp after them stages
+constexpr uint32_t GIANT_RING = GIANT_SOLVERS * WARP_MANIFOLDS;   // manifolds of a level staged (the first 16)
 constexpr uint32_t GIANT_LEVELS = 3;   // levels in the ring
-constexpr uint32_t GIANT_THREADS = 64;
+constexpr uint32_t GIANT_THREADS = (GIANT_SOLVERS + 1) * 32;
 struct __align__(16) GiantSlot {
-    int4 desc;                         // slot 1 | slot 2 << 16 (0xffff: fixed), points, manifold (island index), first point
-    float4 mq[DQ_ROWS];
-    float4 pq[4 * PREC_F4];
+    int4 desc;                         // slot 1 | slot 2 << 16, points, manifold (island index), first point
+    LaneSlot rows;
+};
+// named barrier 1 over the CTA's warps
+template <uint32_t THREADS>
+RD void cta_bar() { asm volatile("bar.sync 1, %0;\n" ::"n"(THREADS) : "memory"); }
+
+// A level of the ring: its first position in the level order and its width,
+// the largest point count of each solver warp's manifolds (0: nothing to do).
+struct __align__(16) GiantLevel {
+    uint32_t first, width, pad[2];
+    uint32_t nbw[GIANT_SOLVERS];
+    GiantSlot slot[GIANT_RING];
 };
 
-RD void cp_async16(void* smem, const void* gmem) {
-    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-RD void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-RD void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-// named barrier 1 over both warps of the CTA
-RD void giant_bar() { asm volatile("bar.sync 1, %0;\n" ::"n"(GIANT_THREADS) : "memory"); }
-
 struct GiantStage {
-    float4 *vel, *mmut, *pmut;
-    GiantSlot* ring;
+    float4 *vel, *mmut;
+    float2* pmut;          // penetration impulse, split impulse
+    GiantLevel* ring;
     int32_t *hkey, *slot_body;
     uint32_t* hval;
-    int2* man;             // body ids (fixed bodies as -1 - id)
-    short2* slot;          // staged slot of body 1 / body 2 (-1: fixed)
+    short2* slot;          // slots of body 1 / body 2
     uint16_t *order, *klev, *lev;
     uint32_t* pofs;        // first point of each manifold, relative to the island's first point
     uint8_t* npt;
@@ -974,12 +1442,11 @@ RD bool giant_layout(const DynArgs& a, uint32_t cnt, uint32_t np, unsigned char*
     auto take = [&](size_t bytes) { const size_t o = off; off = (off + bytes + 15) & ~size_t(15); return sm + o; };
     g.vel = reinterpret_cast<float4*>(take(size_t(4) * g.nbmax * 16));
     g.mmut = reinterpret_cast<float4*>(take(size_t(cnt) * 16));
-    g.pmut = reinterpret_cast<float4*>(take(size_t(np) * 16));
-    g.ring = reinterpret_cast<GiantSlot*>(take(size_t(GIANT_LEVELS) * GIANT_RING * sizeof(GiantSlot)));
+    g.pmut = reinterpret_cast<float2*>(take(size_t(np) * 8));
+    g.ring = reinterpret_cast<GiantLevel*>(take(size_t(GIANT_LEVELS) * sizeof(GiantLevel)));
     g.hkey = reinterpret_cast<int32_t*>(take(size_t(g.H) * 4));
     g.hval = reinterpret_cast<uint32_t*>(take(size_t(g.H) * 4));
     g.slot_body = reinterpret_cast<int32_t*>(take(size_t(g.nbmax) * 4));
-    g.man = reinterpret_cast<int2*>(take(size_t(cnt) * 8));
     g.slot = reinterpret_cast<short2*>(take(size_t(cnt) * 4));
     g.order = reinterpret_cast<uint16_t*>(take(size_t(cnt) * 2));
     g.klev = reinterpret_cast<uint16_t*>(take(size_t(cnt) * 2));
@@ -989,193 +1456,182 @@ RD bool giant_layout(const DynArgs& a, uint32_t cnt, uint32_t np, unsigned char*
     return off <= a.giant_smem;
 }
 
-RD bool giant_body(GiantStage& g, int32_t b, uint32_t& nslots, uint32_t& idx) {
-    uint32_t h = (uint32_t(b) * 2654435761u) & (g.H - 1);
-    for (uint32_t probe = 0; probe < g.H; probe++, h = (h + 1) & (g.H - 1)) {
-        const int32_t k = g.hkey[h];
-        if (k == b) { idx = h; return true; }
-        if (k < 0) {
-            if (nslots >= g.nbmax) return false;
-            g.hkey[h] = b;
-            g.hval[h] = nslots << 16;
-            g.slot_body[nslots] = b;
-            nslots++;
-            idx = h;
-            return true;
-        }
-    }
-    return false;
-}
-
-// Stage and schedule an island (warp 0); false (nothing written to global
-// memory) when it does not fit or its points are not one contiguous range.
+// Schedule an island (warp 0); false (nothing written to global memory) when
+// it does not fit or its points are not one contiguous range.
 RD bool giant_schedule(const DynArgs& a, uint32_t m0, uint32_t cnt, unsigned char* sm, GiantStage& g,
-                       uint32_t lane, uint32_t& depth, uint32_t& nslots, uint32_t& p0) {
+                       uint32_t lane, uint32_t& depth, uint32_t* nslots, uint32_t& p0) {
     const int4 f = man_ids(a, m0), l = man_ids(a, m0 + cnt - 1);
     p0 = uint32_t(f.w);
     const int64_t end = int64_t(l.w) + int64_t(l.z);
     if (f.w < 0 || end < int64_t(p0) || end > int64_t(a.np)) return false;
     const uint32_t np = uint32_t(end - int64_t(p0));
     if (!giant_layout(a, cnt, np, sm, g)) return false;
-    for (uint32_t h = lane; h < g.H; h += 32) g.hkey[h] = -1;
-    for (uint32_t k = lane; k < cnt; k += 32) {
-        const int4 id = man_ids(a, m0 + k);
-        const uint32_t fixed = man_fixed(a, m0 + k);
-        g.man[k] = make_int2((fixed & 1) ? -1 - id.x : id.x, (fixed & 2) ? -1 - id.y : id.y);
-        g.pofs[k] = uint32_t(id.w) - p0;
-        g.npt[k] = uint8_t(id.z < 0 ? 0 : (id.z > 255 ? 255 : id.z));
-    }
-    __syncwarp();
-    bool ok = true;
-    if (lane == 0) {
-        depth = 0;
-        nslots = 0;
-        uint32_t expect = 0;
-        for (uint32_t k = 0; k < cnt && ok; k++) {
-            const int2 id = g.man[k];
-            if (g.pofs[k] != expect || g.npt[k] > 4) { ok = false; break; }
-            expect += g.npt[k];
-            uint32_t L = 1;
-            short2 sl = make_short2(-1, -1);
-            if (g.npt[k] != 0) {
-                uint32_t h1 = 0, h2 = 0, l1 = 0, l2 = 0;
-                if (id.x >= 0) { ok = giant_body(g, id.x, nslots, h1); if (ok) { l1 = g.hval[h1] & 0xffffu; sl.x = short(g.hval[h1] >> 16); } }
-                if (ok && id.y >= 0) { ok = giant_body(g, id.y, nslots, h2); if (ok) { l2 = g.hval[h2] & 0xffffu; sl.y = short(g.hval[h2] >> 16); } }
-                if (!ok) break;
-                L = 1 + (l1 > l2 ? l1 : l2);
-                if (id.x >= 0) g.hval[h1] = (g.hval[h1] & 0xffff0000u) | L;
-                if (id.y >= 0) g.hval[h2] = (g.hval[h2] & 0xffff0000u) | L;
-            }
-            g.slot[k] = sl;
-            g.klev[k] = uint16_t(L);
-            depth = L > depth ? L : depth;
+    uint32_t expect = 0;
+    for (uint32_t base = 0; base < cnt; base += 32) {
+        const uint32_t k = base + lane;
+        uint32_t pofs = 0, npt = 0;
+        if (k < cnt) {
+            const int4 id = man_ids(a, m0 + k);
+            pofs = uint32_t(id.w) - p0;
+            npt = uint32_t(id.z < 0 ? 0 : (id.z > 255 ? 255 : id.z));
+            g.pofs[k] = pofs;
+            g.npt[k] = uint8_t(npt);
         }
-        if (ok && expect != np) ok = false;
-        if (ok) {
-            for (uint32_t L = 0; L <= depth; L++) g.lev[L] = 0;
-            for (uint32_t k = 0; k < cnt; k++) g.lev[g.klev[k] - 1]++;
-            uint32_t run = 0;
-            for (uint32_t L = 0; L < depth; L++) { run += g.lev[L]; g.lev[L] = uint16_t(run); }
-            g.lev[depth] = uint16_t(cnt);
-            for (uint32_t k = cnt; k-- > 0;) g.order[--g.lev[g.klev[k] - 1]] = uint16_t(k);
+        uint32_t inc = npt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= uint32_t(o)) inc += t;
         }
+        if (__any_sync(0xffffffffu, k < cnt && (npt > 4 || pofs != expect + inc - npt))) return false;
+        expect += __shfl_sync(0xffffffffu, inc, 31);
     }
-    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-    depth = __shfl_sync(0xffffffffu, depth, 0);
-    nslots = __shfl_sync(0xffffffffu, nslots, 0);
-    __syncwarp();
-    return ok;
+    if (expect != np) return false;
+    IslandSched S;
+    S.hkey = g.hkey; S.hval = g.hval; S.H = g.H;
+    S.slot_body = g.slot_body; S.nbmax = g.nbmax;
+    S.slot = g.slot; S.klev = g.klev; S.order = g.order; S.lev = g.lev;
+    S.nslots = nslots;
+    return island_schedule(a, m0, cnt, S, lane, depth);
 }
 
-// Warp 1: stage level t (of the linearised passes x levels) into ring level t % 3.
+// Staging warp: the next level of the linearised passes x levels (cursor S)
+// into its ring level.  Lane s < 16 looks its manifold up; then the whole warp
+// copies slot after slot, two rows a lane.
+struct GiantCursor { uint32_t t, L, ring; };
 RD void giant_stage_level(const DynArgs& a, const GiantStage& g, uint32_t m0, uint32_t p0, uint32_t depth,
-                          uint32_t total, uint32_t t, uint32_t lane) {
-    if (t < total) {
-        const uint32_t L = t % depth;
-        const uint32_t j = g.lev[L] + lane;
-        if (lane < GIANT_RING && j < g.lev[L + 1]) {
-            const uint32_t kk = g.order[j];
-            GiantSlot* sl = g.ring + (t % GIANT_LEVELS) * GIANT_RING + lane;
+                          uint32_t total, GiantCursor& S, uint32_t lane) {
+    if (S.t < total) {
+        const uint32_t first = g.lev[S.L], width = g.lev[S.L + 1] - first;
+        GiantLevel* R = g.ring + S.ring;
+        uint32_t kk = 0, np = 0, pofs = 0;
+        if (lane < GIANT_RING && lane < width) {
+            kk = g.order[first + lane];
             const short2 bs = g.slot[kk];
-            const uint32_t np = g.npt[kk];
-            sl->desc = make_int4(int(uint32_t(uint16_t(bs.x)) | (uint32_t(uint16_t(bs.y)) << 16)), int(np), int(kk),
-                                 int(g.pofs[kk]));
-            const float4* src = a.mrec[m0 + kk].q;
-            for (int r = 0; r < DQ_ROWS; r++) cp_async16(&sl->mq[r], src + r);
-            const float4* ps = a.prec[p0 + g.pofs[kk]].q;
-            for (uint32_t r = 0; r < np * PREC_F4; r++) cp_async16(&sl->pq[r], ps + r);
+            np = g.npt[kk];
+            pofs = g.pofs[kk];
+            R->slot[lane].desc = make_int4(int(uint32_t(uint16_t(bs.x)) | (uint32_t(uint16_t(bs.y)) << 16)), int(np),
+                                           int(kk), int(pofs));
         }
+        const uint32_t n = width < GIANT_RING ? width : GIANT_RING;
+        for (uint32_t s = 0; s < n; s++) {
+            const uint32_t ks = __shfl_sync(0xffffffffu, kk, int(s)), ns = __shfl_sync(0xffffffffu, np, int(s));
+            const uint32_t ps = __shfl_sync(0xffffffffu, pofs, int(s));
+            const float4* mq = a.mrec[m0 + ks].q;
+            const float4* pq = a.prec[ns ? p0 + ps : 0u].q;
+            float4* dst = R->slot[s].rows.mq;   // the point rows follow the manifold's
+            const uint32_t rows = DQ_ROWS + ns * PREC_ROWS;
+            if (lane < rows) cp_async16(dst + lane, lane < DQ_ROWS ? mq + lane : pq + (lane - DQ_ROWS));
+            if (lane + 32 < rows) cp_async16(dst + lane + 32, pq + (lane + 32 - DQ_ROWS));
+        }
+        uint32_t w = np;
+        for (int o = 1; o < int(WARP_MANIFOLDS); o <<= 1) {
+            const uint32_t v = __shfl_xor_sync(0xffffffffu, w, o);
+            w = v > w ? v : w;
+        }
+        if (lane < GIANT_RING && lane % WARP_MANIFOLDS == 0) R->nbw[lane / WARP_MANIFOLDS] = w;
+        if (lane == 0) { R->first = first; R->width = width; }
+        S.t++;
+        if (++S.L == depth) S.L = 0;
+        if (++S.ring == GIANT_LEVELS) S.ring = 0;
     }
     cp_async_commit();
 }
 
-RD BodyVel giant_vel(const DynArgs& a, const GiantStage& g, int32_t s1, int32_t s2, int2 id) {
-    BodyVel bv;
-    const uint32_t n = g.nbmax;
-    if (s1 >= 0) { bv.v1 = g.vel + s1; bv.w1 = g.vel + n + s1; bv.s1 = g.vel + 2 * n + s1; bv.t1 = g.vel + 3 * n + s1; }
-    else { const int32_t b1 = -1 - id.x; bv.v1 = a.cv + b1; bv.w1 = a.cw + b1; bv.s1 = a.sv + b1; bv.t1 = a.sw + b1; }
-    if (s2 >= 0) { bv.v2 = g.vel + s2; bv.w2 = g.vel + n + s2; bv.s2 = g.vel + 2 * n + s2; bv.t2 = g.vel + 3 * n + s2; }
-    else { const int32_t b2 = -1 - id.y; bv.v2 = a.cv + b2; bv.w2 = a.cw + b2; bv.s2 = a.sv + b2; bv.t2 = a.sw + b2; }
-    return bv;
+// A lane group's staged manifold of a level, its impulses in shared memory.
+RD void giant_manifold(const DynArgs& a, const GiantStage& g, const LaneId& id, bool warm, const GiantSlot* sl,
+                       bool active, uint32_t nbw, uint32_t lane) {
+    const int4 d = sl->desc;
+    const uint32_t nb = active ? uint32_t(d.y) : 0u;
+    active = nb != 0;
+    float* vel = reinterpret_cast<float*>(g.vel) + size_t(8) * g.nbmax * id.role;
+    float* b1 = vel + (active ? 4 * (d.x & 0xffff) : 0);
+    float* b2 = vel + (active ? 4 * int(uint32_t(d.x) >> 16) : 0);
+    const uint32_t wofs = 4 * g.nbmax;
+    float* pm = reinterpret_cast<float*>(g.pmut + (active ? d.w : 0)) + id.role;
+    float* mm = reinterpret_cast<float*>(g.mmut + (active ? d.z : 0));
+    const float *mq = reinterpret_cast<const float*>(sl->rows.mq), *pq = reinterpret_cast<const float*>(sl->rows.pq);
+    float imp[4], f[3];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) imp[k] = k < nb ? pm[2 * k] : 0.0f;
+    f[0] = mm[0]; f[1] = mm[1]; f[2] = mm[2];
+    if (warm) lanes_warm(mq, pq, nb, nbw, active, id, b1, b2, wofs, imp, f);
+    else lanes_solve(a.split != 0, mq, pq, nb, nbw, active, id, b1, b2, wofs, imp, f);
+    if (active && (lane & 3u) == 0 && (id.role == 0 || (!warm && a.split))) {
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++)
+            if (k < nb) pm[2 * k] = imp[k];
+        if (id.role == 0) { mm[0] = f[0]; mm[1] = f[1]; mm[2] = f[2]; }
+    }
 }
 
-// Both warps: stage, solve and write back one island.
+// All warps: stage, solve and write back one island.
 RD void giant_solve(const DynArgs& a, uint32_t m0, uint32_t cnt, const GiantStage& g, uint32_t warp,
                     uint32_t lane, uint32_t depth, uint32_t nslots, uint32_t p0) {
     const uint32_t np = g.pofs[cnt - 1] + g.npt[cnt - 1];
     const uint32_t tid = warp * 32 + lane;
     for (uint32_t s = tid; s < nslots; s += GIANT_THREADS) {
-        const int32_t b = g.slot_body[s];
+        const int32_t e = g.slot_body[s], b = e < 0 ? -1 - e : e;
         g.vel[s] = a.cv[b];
         g.vel[g.nbmax + s] = a.cw[b];
         g.vel[2 * g.nbmax + s] = a.sv[b];
         g.vel[3 * g.nbmax + s] = a.sw[b];
     }
     for (uint32_t k = tid; k < cnt; k += GIANT_THREADS) g.mmut[k] = a.mrec[m0 + k].mut;
-    for (uint32_t p = tid; p < np; p += GIANT_THREADS) g.pmut[p] = a.prec[p0 + p].mut;
+    for (uint32_t p = tid; p < np; p += GIANT_THREADS) g.pmut[p] = *reinterpret_cast<const float2*>(&a.prec[p0 + p].mut);
     const uint32_t total = uint32_t(a.iterations + 1) * depth;
-    if (warp == 1) {
-        giant_stage_level(a, g, m0, p0, depth, total, 0, lane);
-        giant_stage_level(a, g, m0, p0, depth, total, 1, lane);
+    if (warp == GIANT_SOLVERS) {
+        GiantCursor S{0, 0, 0};
+        giant_stage_level(a, g, m0, p0, depth, total, S, lane);
+        giant_stage_level(a, g, m0, p0, depth, total, S, lane);
         cp_async_wait<1>();
-        giant_bar();                       // level 0 staged, stage loads done
+        cta_bar<GIANT_THREADS>();          // level 0 staged, stage loads done
         for (uint32_t t = 0; t < total; t++) {
-            giant_stage_level(a, g, m0, p0, depth, total, t + 2, lane);
+            giant_stage_level(a, g, m0, p0, depth, total, S, lane);   // level t + 2
             cp_async_wait<1>();            // level t + 1 staged
-            giant_bar();                   // end of level t
+            cta_bar<GIANT_THREADS>();      // end of level t
         }
         cp_async_wait<0>();
     } else {
-        const float beta = a.split ? BETA_SPLIT_IMPULSE : BETA;
-        giant_bar();
+        const LaneId id = lane_id(lane);
+        cta_bar<GIANT_THREADS>();
+        uint32_t ring = 0;
         for (uint32_t t = 0; t < total; t++) {
-            const uint32_t L = t % depth;
             const bool warm = t < depth;
-            const uint32_t b = g.lev[L], e = g.lev[L + 1];
-            if (lane < GIANT_RING && b + lane < e) {
-                const GiantSlot* sl = g.ring + (t % GIANT_LEVELS) * GIANT_RING + lane;
-                const int4 d = sl->desc;
-                const int32_t s1 = int32_t(int16_t(d.x & 0xffff)), s2 = int32_t(int16_t(uint32_t(d.x) >> 16));
-                const BodyVel bv = giant_vel(a, g, s1, s2, g.man[d.z]);
-                RecSrc r;
-                r.mq = sl->mq;
-                r.pq = sl->pq;
-                r.pq_stride = PREC_F4;
-                r.mmut = g.mmut + d.z;
-                r.pmut = g.pmut + d.w;
-                r.pmut_stride = 1;
-                if (warm) warm_core<false>(a, r, bv, d.y);
-                else solve_core<false>(a, r, beta, bv, d.y);
-            }
-            // manifolds of a level beyond the staged ones read their rows from global memory
-            for (uint32_t j = b + GIANT_RING + lane; j < e; j += 32) {
+            const GiantLevel* R = g.ring + ring;
+            const uint32_t at = warp * WARP_MANIFOLDS + id.group;
+            const uint32_t nbw = R->nbw[warp], b = R->first, width = R->width, e = b + width;
+            if (nbw) giant_manifold(a, g, id, warm, &R->slot[at], at < width, nbw, lane);
+            // a level's manifolds beyond the staged ones: one a lane, their rows
+            // from global memory
+            for (uint32_t j = b + GIANT_RING + warp * 32 + lane; j < e; j += GIANT_SOLVERS * 32) {
                 const uint32_t kk = g.order[j];
-                const short2 sl = g.slot[kk];
-                const BodyVel bv = giant_vel(a, g, sl.x, sl.y, g.man[kk]);
-                RecSrc r;
-                r.mq = a.mrec[m0 + kk].q;
-                r.pq = a.prec[p0 + g.pofs[kk]].q;
-                r.pq_stride = PREC_F4;
+                const short2 bs = g.slot[kk];
+                BodyVel bv;
+                const uint32_t n = g.nbmax;
+                bv.v1 = g.vel + bs.x; bv.w1 = bv.v1 + n; bv.s1 = bv.w1 + n; bv.t1 = bv.s1 + n;
+                bv.v2 = g.vel + bs.y; bv.w2 = bv.v2 + n; bv.s2 = bv.w2 + n; bv.t2 = bv.s2 + n;
+                RecSrc r = rec_global(a, m0 + kk, int32_t(g.npt[kk] ? p0 + g.pofs[kk] : 0u));
                 r.mmut = g.mmut + kk;
-                r.pmut = g.pmut + g.pofs[kk];
-                r.pmut_stride = 1;
-                if (warm) warm_core<true>(a, r, bv, g.npt[kk]);
-                else solve_core<true>(a, r, beta, bv, g.npt[kk]);
+                r.pm2 = g.pmut + g.pofs[kk];
+                if (warm) warm_core<true, true>(a, r, bv, g.npt[kk]);
+                else solve_core<true, true>(a, r, bv, g.npt[kk]);
             }
             __syncwarp();
-            giant_bar();
+            cta_bar<GIANT_THREADS>();
+            if (++ring == GIANT_LEVELS) ring = 0;
         }
     }
     __syncthreads();
     for (uint32_t s = tid; s < nslots; s += GIANT_THREADS) {
         const int32_t b = g.slot_body[s];
+        if (b < 0) continue;
         a.cv[b] = g.vel[s];
         a.cw[b] = g.vel[g.nbmax + s];
         a.sv[b] = g.vel[2 * g.nbmax + s];
         a.sw[b] = g.vel[3 * g.nbmax + s];
     }
     for (uint32_t k = tid; k < cnt; k += GIANT_THREADS) a.mrec[m0 + k].mut = g.mmut[k];
-    for (uint32_t p = tid; p < np; p += GIANT_THREADS) a.prec[p0 + p].mut = g.pmut[p];
+    for (uint32_t p = tid; p < np; p += GIANT_THREADS) *reinterpret_cast<float2*>(&a.prec[p0 + p].mut) = g.pmut[p];
     __syncthreads();
 }
 
@@ -1193,6 +1649,8 @@ RD void giant_solve(const DynArgs& a, uint32_t m0, uint32_t cnt, const GiantStag
 // the ring with the velocities and impulses read from and written to global
 // memory; both warps meet at the named barrier once per level.
 constexpr uint32_t STREAM_RING = 32;
+constexpr uint32_t STREAM_THREADS = 64;
+using StreamSlot = GiantSlot;          // desc: unused, points, manifold (island index), first point
 
 // Warp 0: levels and the level-ordered manifolds of an island.  Writes
 // a.order[m0 + i] (island-relative manifold indices in level order) and
@@ -1309,7 +1767,7 @@ RD uint32_t stream_kk(const DynArgs& a, uint32_t m0, int2 bd, uint32_t lane) {
 
 // One pipeline step for level x (negative in the prologue: loads only); the
 // header of level x (its bounds) goes to hdr[x % 3] for warp 0.
-RD void stream_stage_step(const DynArgs& a, GiantSlot* ring, int2* hdr, StreamPipe& P, uint32_t m0, uint32_t depth,
+RD void stream_stage_step(const DynArgs& a, StreamSlot* ring, int2* hdr, StreamPipe& P, uint32_t m0, uint32_t depth,
                           int64_t total, int64_t x, uint32_t lane) {
     const int2 nb3 = stream_bounds(a, m0, depth, total, x + 3);
     const uint32_t nk2 = stream_kk(a, m0, P.b2, lane);
@@ -1319,12 +1777,12 @@ RD void stream_stage_step(const DynArgs& a, GiantSlot* ring, int2* hdr, StreamPi
         if (lane == 0) hdr[uint32_t(x) % GIANT_LEVELS] = P.b0;
         if (P.k0 != ~0u) {
             const uint32_t np = P.i0.z < 0 ? 0u : (P.i0.z > 4 ? 4u : uint32_t(P.i0.z));
-            GiantSlot* sl = ring + (uint32_t(x) % GIANT_LEVELS) * STREAM_RING + lane;
+            StreamSlot* sl = ring + (uint32_t(x) % GIANT_LEVELS) * STREAM_RING + lane;
             sl->desc = make_int4(0, int(np), int(P.k0), P.i0.w);
             const float4* src = a.mrec[m0 + P.k0].q;
-            for (int r = 0; r < DQ_ROWS; r++) cp_async16(&sl->mq[r], src + r);
+            for (int r = 0; r < DQ_ROWS; r++) cp_async16(&sl->rows.mq[r], src + r);
             const float4* ps = a.prec[P.i0.w].q;
-            for (uint32_t r = 0; r < np * PREC_F4; r++) cp_async16(&sl->pq[r], ps + r);
+            for (uint32_t r = 0; r < np * PREC_ROWS; r++) cp_async16(&sl->rows.pq[r], ps + r);
         }
     }
     if (x >= 0) cp_async_commit();
@@ -1337,7 +1795,7 @@ RD void stream_stage_step(const DynArgs& a, GiantSlot* ring, int2* hdr, StreamPi
 }
 
 // Both warps: warm start and velocity iterations of a scheduled island.
-RD void stream_solve(const DynArgs& a, uint32_t m0, GiantSlot* ring, uint32_t warp, uint32_t lane, uint32_t depth) {
+RD void stream_solve(const DynArgs& a, uint32_t m0, StreamSlot* ring, uint32_t warp, uint32_t lane, uint32_t depth) {
     const uint32_t total = uint32_t(a.iterations + 1) * depth;
     int2* hdr = reinterpret_cast<int2*>(ring + GIANT_LEVELS * STREAM_RING);
     if (warp == 1) {
@@ -1347,34 +1805,33 @@ RD void stream_solve(const DynArgs& a, uint32_t m0, GiantSlot* ring, uint32_t wa
         P.i0 = make_int4(0, 0, 0, 0);
         for (int64_t x = -3; x <= 1; x++) stream_stage_step(a, ring, hdr, P, m0, depth, total, x, lane);
         cp_async_wait<1>();
-        giant_bar();
+        cta_bar<STREAM_THREADS>();
         for (uint32_t t = 0; t < total; t++) {
             stream_stage_step(a, ring, hdr, P, m0, depth, total, int64_t(t) + 2, lane);
             cp_async_wait<1>();
-            giant_bar();
+            cta_bar<STREAM_THREADS>();
         }
         cp_async_wait<0>();
     } else {
-        const float beta = a.split ? BETA_SPLIT_IMPULSE : BETA;
-        giant_bar();
+        cta_bar<STREAM_THREADS>();
         for (uint32_t t = 0; t < total; t++) {
             const bool warm = t < depth;
             const int2 bd = hdr[t % GIANT_LEVELS];
             const uint32_t b = uint32_t(bd.x), e = uint32_t(bd.y);
             if (lane < STREAM_RING && b + lane < e) {
-                const GiantSlot* sl = ring + (t % GIANT_LEVELS) * STREAM_RING + lane;
+                const StreamSlot* sl = ring + (t % GIANT_LEVELS) * STREAM_RING + lane;
                 const int4 d = sl->desc;
-                const float4 ids = sl->mq[DQ_IDS];
+                const float4 ids = sl->rows.mq[DQ_IDS];
                 const BodyVel bv = vel_global(a, __float_as_int(ids.x), __float_as_int(ids.y));
                 RecSrc r;
-                r.mq = sl->mq;
-                r.pq = sl->pq;
-                r.pq_stride = PREC_F4;
+                r.mq = sl->rows.mq;
+                r.pq = sl->rows.pq;
+                r.pq_stride = PREC_ROWS;
                 r.mmut = &a.mrec[m0 + uint32_t(d.z)].mut;
                 r.pmut = &a.prec[d.w].mut;
-                r.pmut_stride = PREC_F4;
+                r.pmut_stride = PREC_ROWS;
                 if (warm) warm_core<false, true>(a, r, bv, d.y);
-                else solve_core<false, true>(a, r, beta, bv, d.y);
+                else solve_core<false, true>(a, r, bv, d.y);
             }
             // manifolds of a level beyond the ring read their rows from global memory
             for (uint32_t j = b + STREAM_RING + lane; j < e; j += 32) {
@@ -1382,10 +1839,10 @@ RD void stream_solve(const DynArgs& a, uint32_t m0, GiantSlot* ring, uint32_t wa
                 const int4 id = man_ids(a, mi);
                 const BodyVel bv = vel_global(a, id.x, id.y);
                 if (warm) warm_core<true, true>(a, rec_global(a, mi, id.w), bv, id.z);
-                else solve_core<true, true>(a, rec_global(a, mi, id.w), beta, bv, id.z);
+                else solve_core<true, true>(a, rec_global(a, mi, id.w), bv, id.z);
             }
             __syncwarp();
-            giant_bar();
+            cta_bar<STREAM_THREADS>();
         }
     }
     __syncthreads();
@@ -1394,6 +1851,7 @@ RD void stream_solve(const DynArgs& a, uint32_t m0, GiantSlot* ring, uint32_t wa
 __global__ void __launch_bounds__(GIANT_THREADS, 1) dyn_islands_giant(const DynArgs a) {
     extern __shared__ __align__(16) unsigned char gsm[];
     __shared__ uint32_t s_island, s_ok, s_depth, s_nslots, s_p0;
+    constexpr uint32_t SCHED_WARP = 0;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t n_giant = a.counters[3];
     for (;;) {
@@ -1402,22 +1860,26 @@ __global__ void __launch_bounds__(GIANT_THREADS, 1) dyn_islands_giant(const DynA
         const uint32_t k = s_island;
         if (k >= n_giant) break;
         const uint32_t is = a.giant_list[k];
+        if (is == ISLAND_DONE) {
+            __syncthreads();
+            continue;
+        }
         const uint32_t m0 = a.i_start[is], cnt = a.i_count[is];
         GiantStage g;
-        if (warp == 0) {
-            uint32_t depth = 0, nslots = 0, p0 = 0;
-            const bool ok = giant_schedule(a, m0, cnt, gsm, g, lane, depth, nslots, p0);
-            if (lane == 0) { s_ok = ok ? 1u : 0u; s_depth = depth; s_nslots = nslots; s_p0 = p0; }
+        if (warp == SCHED_WARP) {
+            uint32_t depth = 0, p0 = 0;
+            const bool ok = giant_schedule(a, m0, cnt, gsm, g, lane, depth, &s_nslots, p0);
+            if (lane == 0) { s_ok = ok ? 1u : 0u; s_depth = depth; s_p0 = p0; }
         }
         __syncthreads();
         if (s_ok) {
-            if (warp == 1) {
+            if (warp != SCHED_WARP) {
                 // the same layout (a pure function of the island's sizes)
                 const int4 l = man_ids(a, m0 + cnt - 1);
                 giant_layout(a, cnt, uint32_t(int64_t(l.w) + int64_t(l.z) - int64_t(s_p0)), gsm, g);
             }
             giant_solve(a, m0, cnt, g, warp, lane, s_depth, s_nslots, s_p0);
-        } else if (size_t(GIANT_LEVELS) * STREAM_RING * sizeof(GiantSlot) + GIANT_LEVELS * sizeof(int2) <= a.giant_smem) {
+        } else if (size_t(GIANT_LEVELS) * STREAM_RING * sizeof(StreamSlot) + GIANT_LEVELS * sizeof(int2) <= a.giant_smem) {
             // streamed by dyn_islands_stream (queued at the back of giant_list)
             if (threadIdx.x == 0) a.giant_list[a.ni - 1 - atomicAdd(a.counters + 5, 1u)] = is;
             __syncthreads();
@@ -1432,7 +1894,7 @@ __global__ void __launch_bounds__(GIANT_THREADS, 1) dyn_islands_giant(const DynA
 }
 
 // ---- kernel 3d: islands streamed through global memory -------------------
-__global__ void __launch_bounds__(GIANT_THREADS, 1) dyn_islands_stream(const DynArgs a) {
+__global__ void __launch_bounds__(STREAM_THREADS, 1) dyn_islands_stream(const DynArgs a) {
     extern __shared__ __align__(16) unsigned char ssm[];
     __shared__ uint32_t s_island, s_depth;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1449,8 +1911,8 @@ __global__ void __launch_bounds__(GIANT_THREADS, 1) dyn_islands_stream(const Dyn
             if (lane == 0) s_depth = depth;
         }
         __syncthreads();
-        stream_solve(a, m0, reinterpret_cast<GiantSlot*>(ssm), warp, lane, s_depth);
-        for (uint32_t j = threadIdx.x; j < cnt; j += GIANT_THREADS) store_manifold(a, m0 + j);
+        stream_solve(a, m0, reinterpret_cast<StreamSlot*>(ssm), warp, lane, s_depth);
+        for (uint32_t j = threadIdx.x; j < cnt; j += STREAM_THREADS) store_manifold(a, m0 + j);
         __syncthreads();
     }
 }
@@ -1619,13 +2081,13 @@ __global__ void __launch_bounds__(128) color_scatter(const DynArgs a, ColorScrat
 
 template <int PASS>   // 0 warm start, 1 velocity iteration
 __global__ void __launch_bounds__(128) colored_pass(const DynArgs a, const uint32_t* __restrict__ order, uint32_t off,
-                                                    uint32_t cnt, float beta) {
+                                                    uint32_t cnt) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= cnt) return;
     const uint32_t mi = order[off + k];
     const int4 id = man_ids(a, mi);
     if (PASS == 0) warm_manifold(a, mi, vel_global(a, id.x, id.y), id.z, id.w);
-    else solve_manifold(a, mi, beta, vel_global(a, id.x, id.y), id.z, id.w);
+    else solve_manifold(a, mi, vel_global(a, id.x, id.y), id.z, id.w);
 }
 
 __global__ void __launch_bounds__(128) colored_store(const DynArgs a) {
@@ -1739,12 +2201,11 @@ bool colored_islands(const DynArgs& a, cudaStream_t s, uint64_t* launches) {
     cudaMemcpyAsync(c.offset, off, sizeof(off), cudaMemcpyHostToDevice, s);
     color_scatter<<<blocks(nm), 128, 0, s>>>(a, c);
     *launches += 1;
-    const float beta = a.split ? BETA_SPLIT_IMPULSE : BETA;
     for (uint32_t k = 0; k < ncol; k++)
-        if (cnt[k]) { colored_pass<0><<<blocks(cnt[k]), 128, 0, s>>>(a, c.order, off[k], cnt[k], beta); (*launches)++; }
+        if (cnt[k]) { colored_pass<0><<<blocks(cnt[k]), 128, 0, s>>>(a, c.order, off[k], cnt[k]); (*launches)++; }
     for (int it = 0; it < a.iterations; it++)
         for (uint32_t k = 0; k < ncol; k++)
-            if (cnt[k]) { colored_pass<1><<<blocks(cnt[k]), 128, 0, s>>>(a, c.order, off[k], cnt[k], beta); (*launches)++; }
+            if (cnt[k]) { colored_pass<1><<<blocks(cnt[k]), 128, 0, s>>>(a, c.order, off[k], cnt[k]); (*launches)++; }
     colored_store<<<blocks(nm), 128, 0, s>>>(a);
     (*launches)++;
     if (a.stats) {
@@ -1769,7 +2230,7 @@ cudaError_t launch_dynamics(const DynArgs& a, cudaStream_t s, uint64_t* launches
     bool colored_done = false;
     if (a.colored && a.color && a.nj == 0 && a.nm) colored_done = colored_islands(a, s, launches);
     if (a.ni && !colored_done) {
-        cudaMemsetAsync(a.counters, 0, 7 * sizeof(uint32_t), s);
+        cudaMemsetAsync(a.counters, 0, 8 * sizeof(uint32_t), s);
         dyn_islands_small<<<blocks(a.ni), 128, 0, s>>>(a);
         (*launches)++;
         const size_t smem = size_t(LARGE_WARPS) * LARGE_WARP_SMEM;
@@ -1780,9 +2241,9 @@ cudaError_t launch_dynamics(const DynArgs& a, cudaStream_t s, uint64_t* launches
             cudaFuncSetAttribute(dyn_islands_giant, cudaFuncAttributeMaxDynamicSharedMemorySize, int(a.giant_smem));
             dyn_islands_giant<<<a.giant_ctas, GIANT_THREADS, a.giant_smem, s>>>(a);
             (*launches)++;
-            const size_t ring = size_t(GIANT_LEVELS) * STREAM_RING * sizeof(GiantSlot) + GIANT_LEVELS * sizeof(int2);
+            const size_t ring = size_t(GIANT_LEVELS) * STREAM_RING * sizeof(StreamSlot) + GIANT_LEVELS * sizeof(int2);
             cudaFuncSetAttribute(dyn_islands_stream, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ring));
-            dyn_islands_stream<<<a.giant_ctas, GIANT_THREADS, ring, s>>>(a);
+            dyn_islands_stream<<<a.giant_ctas, STREAM_THREADS, ring, s>>>(a);
             (*launches)++;
         }
         if (a.nji) { dyn_islands_joint<<<(a.nji + 63) / 64, 64, 0, s>>>(a); (*launches)++; }

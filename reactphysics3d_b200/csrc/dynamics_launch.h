@@ -30,7 +30,9 @@ struct __align__(16) DynManifoldRec {
     float4 mut;   // friction 1, friction 2, twist impulses; w: scheduling level
 };
 
-enum DynPointRow { DP_R1 = 0, DP_R2, DP_N, DP_I1, DP_I2, DP_ROWS };  // (r1, depth), (r2, inverse mass), (n, restitution bias)
+// (r1, -), (r2, inverse mass), (n, bias of the constrained velocities),
+// (I1 (r1 x n) * angular lock factor 1, bias of the split velocities), (I2 (r2 x n) * angular lock factor 2, -)
+enum DynPointRow { DP_R1 = 0, DP_R2, DP_N, DP_I1, DP_I2, DP_ROWS };
 struct __align__(16) DynPointRec {
     float4 q[DP_ROWS];
     float4 mut;   // penetration impulse, split impulse, resting (1 / 0)
@@ -101,10 +103,10 @@ struct __align__(16) JointRec {
 
 // Kernel 3b stages an island's schedule and its movable bodies' velocities
 // in the shared memory of the warp that solves it, when they fit.
-constexpr uint32_t STAGE_BODIES = 256;
+constexpr uint32_t STAGE_BODIES = 304;
 constexpr uint32_t STAGE_MANIFOLDS = 512;
 constexpr int LARGE_WARPS = 3;                 // warps per CTA of kernel 3b (2 CTAs per SM)
-constexpr size_t LARGE_WARP_SMEM = 34816;      // bytes of shared memory per warp
+constexpr size_t LARGE_WARP_SMEM = 38144;      // bytes of shared memory per warp
 
 struct DynArgs {
     // params
@@ -151,7 +153,8 @@ struct DynArgs {
     int32_t* body_slot;    // nb: shared-memory slot of each movable body (scratch)
     uint32_t* counters;    // [0] big islands queued (front of large_list), [1] islands taken, [2] others queued (back),
                            // [3] giant islands queued, [4] giant islands taken,
-                           // [5] streamed islands queued (back of giant_list), [6] streamed islands taken
+                           // [5] streamed islands queued (back of giant_list), [6] streamed islands taken,
+                           // [7] giant islands offered to kernel 3b
     uint32_t* large_list;  // ni: queued islands
     uint32_t* giant_list;  // ni: islands for kernel 3c
     uint32_t large_ctas;   // grid of kernel 3b (persistent)
