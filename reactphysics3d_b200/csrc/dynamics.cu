@@ -685,8 +685,10 @@ __global__ void __launch_bounds__(128) dyn_islands_small(const DynArgs a) {
 // every lane: each value goes through the same operations in the same order
 // as in warm_core / solve_core, bit for bit.  Measured on a chain of one
 // manifold a level, cycles a level with 1 / 4 points: one CTA an island
-// 1,562 / 2,392 with a lane a manifold, 1,299 / 1,856 here; one warp an island
-// 2,277 / 4,319 and 1,981 / 2,478.  4,096 captured worlds: 5.28 -> 1.85 ms.
+// 1,562 / 2,392 with a lane a manifold, 1,273 / 1,841 here; one warp an island
+// 2,277 / 4,319 and 1,697 / 2,141 (1,981 / 2,478 while its copies and loads of
+// the next chunk were conditional: a dozen divergent branches).  4,096
+// captured worlds: 5.28 -> 1.76 ms.
 constexpr uint32_t LANES_PER_MANIFOLD = 8, WARP_MANIFOLDS = 32 / LANES_PER_MANIFOLD;
 // A manifold's rows staged in shared memory: its record's constant rows, then
 // its points' records (the impulse rows among them are the values at staging
@@ -704,10 +706,21 @@ RD void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"
 template <int N>
 RD void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+// Predicated stores, written out, where a nest of C++ conditionals becomes a
+// chain of divergent branches.
+RD void st_shared_if(bool ok, float* p, float v) {
+    const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(p));
+    asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q st.shared.f32 [%0], %1;\n}\n" ::"r"(sa), "f"(v), "r"(int(ok)) : "memory");
+}
+RD void st_global_if(bool ok, float* p, float v) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q st.global.f32 [%0], %1;\n}\n" ::"l"(p), "f"(v), "r"(int(ok)) : "memory");
+}
+
 struct LaneId {
     uint32_t group;     // manifold of the warp's four
     uint32_t role;      // 0 constrained, 1 split velocities
     uint32_t c, c1, c2; // component and the two after it
+    uint32_t q;         // lane of the half
     bool writer;
 };
 RD LaneId lane_id(uint32_t lane) {
@@ -716,6 +729,7 @@ RD LaneId lane_id(uint32_t lane) {
     id.role = (lane >> 2) & 1u;
     const uint32_t c = lane & 3u;
     id.writer = c < 3;
+    id.q = c;
     id.c = c < 3 ? c : 0u;
     id.c1 = id.c == 2 ? 0u : id.c + 1;
     id.c2 = id.c == 0 ? 2u : id.c - 1;
@@ -743,10 +757,20 @@ struct LaneVel { float v1, w1a, w1b, v2, w2a, w2b; };
 RD LaneVel lane_vel_load(const float* b1, const float* b2, uint32_t wofs, const LaneId& id) {
     return LaneVel{b1[id.c], b1[wofs + id.c1], b1[wofs + id.c2], b2[id.c], b2[wofs + id.c1], b2[wofs + id.c2]};
 }
-// every component is stored by one lane (its angular share by c + 1)
-RD void lane_vel_store(float* b1, float* b2, uint32_t wofs, const LaneId& id, uint32_t fixed, const LaneVel& u) {
-    if (!(fixed & 1u)) { b1[id.c] = u.v1; b1[wofs + id.c1] = u.w1a; }
-    if (!(fixed & 2u)) { b2[id.c] = u.v2; b2[wofs + id.c1] = u.w2a; }
+// Every component is stored by one lane (its angular share by c + 1); the
+// rows are in shared memory.
+RD void lane_vel_store(float* b1, float* b2, uint32_t wofs, const LaneId& id, bool ok, uint32_t fixed, const LaneVel& u) {
+    const bool s1 = ok && !(fixed & 1u), s2 = ok && !(fixed & 2u);
+    st_shared_if(s1, b1 + id.c, u.v1);
+    st_shared_if(s1, b1 + wofs + id.c1, u.w1a);
+    st_shared_if(s2, b2 + id.c, u.v2);
+    st_shared_if(s2, b2 + wofs + id.c1, u.w2a);
+}
+// A half's four lanes hold the same impulses: each stores one point's and one
+// friction impulse.
+RD float lane_pick(uint32_t q, const float (&x)[4]) {
+    const float lo = q & 1u ? x[1] : x[0], hi = q & 1u ? x[3] : x[2];
+    return q & 2u ? hi : lo;
 }
 
 // warm_core on eight lanes; the whole warp calls it, `nbw` is the largest
@@ -766,23 +790,24 @@ RD void lanes_warm(const float* mq, const float* pq, uint32_t nb, uint32_t nbw, 
     for (uint32_t k = 0; k < 4; k++) {
         if (k >= nbw) break;
         const float* p = pq + k * 4 * PREC_ROWS;
-        if (k < nb) {
-            if (p[4 * DP_ROWS + 2] != 0.0f) {   // mut.z: resting
-                resting_any = true;
-                const float pi = imp[k];
-                const float ip = p[4 * DP_N + id.c] * pi;
-                u.v1 = u.v1 - ms.x * ip * lf1;
-                u.w1a = u.w1a - p[4 * DP_I1 + id.c1] * pi;
-                u.w1b = u.w1b - p[4 * DP_I1 + id.c2] * pi;
-                u.v2 = u.v2 + ms.y * ip * lf2;
-                u.w2a = u.w2a + p[4 * DP_I2 + id.c1] * pi;
-                u.w2b = u.w2b + p[4 * DP_I2 + id.c2] * pi;
-            } else {
-                imp[k] = 0.0f;
-            }
+        const bool resting = p[4 * DP_ROWS + 2] != 0.0f;   // mut.z
+        const float pi = imp[k];
+        const float ip = p[4 * DP_N + id.c] * pi;
+        LaneVel t;
+        t.v1 = u.v1 - ms.x * ip * lf1;
+        t.w1a = u.w1a - p[4 * DP_I1 + id.c1] * pi;
+        t.w1b = u.w1b - p[4 * DP_I1 + id.c2] * pi;
+        t.v2 = u.v2 + ms.y * ip * lf2;
+        t.w2a = u.w2a + p[4 * DP_I2 + id.c1] * pi;
+        t.w2b = u.w2b + p[4 * DP_I2 + id.c2] * pi;
+        if (k < nb && resting) {
+            u = t;
+            resting_any = true;
         }
+        if (k < nb && !resting) imp[k] = 0.0f;
     }
-    if (resting_any) {
+    if (__any_sync(0xffffffffu, resting_any)) {
+        const LaneVel u0 = u;
         const v3 o1 = L3(q[DQ_OFV1]), o2 = L3(q[DQ_OFV2]);
         const v3 fv1 = L3(q[DQ_FV1]), fv2 = L3(q[DQ_FV2]), n = L3(q[DQ_N]);
         const v3 r1ct1 = L3(q[DQ_R1CT1]), r1ct2 = L3(q[DQ_R1CT2]), r2ct1 = L3(q[DQ_R2CT1]), r2ct2 = L3(q[DQ_R2CT2]);
@@ -814,11 +839,11 @@ RD void lanes_warm(const float* mq, const float* pq, uint32_t nb, uint32_t nbw, 
         u.w2a = u.w2a + af2a * row_dot(I2a, ai2); u.w2b = u.w2b + af2b * row_dot(I2b, ai2);
         u.w1a = u.w1a - af1a * row_dot(I1a, ai2); u.w1b = u.w1b - af1b * row_dot(I1b, ai2);
         u.w2a = u.w2a + af2a * row_dot(I2a, ai2); u.w2b = u.w2b + af2b * row_dot(I2b, ai2);
-    } else {
-        f[0] = f[1] = f[2] = 0.0f;
+        if (!resting_any) u = u0;
     }
+    if (!resting_any) f[0] = f[1] = f[2] = 0.0f;
     __syncwarp();   // every lane has read its share (lanes_solve: its shuffles)
-    if (active && id.writer && id.role == 0) lane_vel_store(b1, b2, wofs, id, fixed, u);
+    lane_vel_store(b1, b2, wofs, id, active && id.writer && id.role == 0, fixed, u);
 }
 
 // A point's rows as one lane needs them.
@@ -852,9 +877,10 @@ RD void lanes_solve(bool split, const float* mq, const float* pq, uint32_t nb, u
     for (uint32_t k = 0; k < 4; k++) {
         if (k >= nbw) break;
         const LanePt p = next;
-        if (k < 3) next = lane_pt(pq + (k + 1) * 4 * PREC_ROWS, id);
         const float dv = u.v2 + u.w2a * p.r2b - u.w2b * p.r2a - u.v1 - u.w1a * p.r1b + u.w1b * p.r1a;
         const float Jv = lanes_sum(dv * p.n);
+        // (behind the shuffles, whose queue the reads share)
+        if (k < 3) next = lane_pt(pq + (k + 1) * 4 * PREC_ROWS, id);
         float dl = -(Jv + p.bias) * p.inv_mass;
         const float sum = imp[k] + dl;
         const float now = (sum < 0.0f) ? 0.0f : sum;
@@ -871,6 +897,7 @@ RD void lanes_solve(bool split, const float* mq, const float* pq, uint32_t nb, u
             sum_pen += now;
         }
     }
+    // the split half ends here: what it computes below is discarded
     const float af1a = mq[4 * DQ_AF1 + id.c1], af1b = mq[4 * DQ_AF1 + id.c2];
     const float af2a = mq[4 * DQ_AF2 + id.c1], af2b = mq[4 * DQ_AF2 + id.c2];
     const float t1 = mq[4 * DQ_FV1 + id.c], t2 = mq[4 * DQ_FV2 + id.c], nt = mq[4 * DQ_N + id.c1];
@@ -879,7 +906,6 @@ RD void lanes_solve(bool split, const float* mq, const float* pq, uint32_t nb, u
     const float f1a = mq[4 * DQ_R1F + id.c1], f1b = mq[4 * DQ_R1F + id.c2], inv_f1 = mq[4 * DQ_R1F + 3];
     const float f2a = mq[4 * DQ_R2F + id.c1], f2b = mq[4 * DQ_R2F + id.c2], inv_f2 = mq[4 * DQ_R2F + 3];
     const float4 nq = q[DQ_N];
-    // the split half ends here: what it computes below is discarded
     const LaneVel us = u;
     const float limit = ms.z * sum_pen;
     // first friction constraint
@@ -922,7 +948,7 @@ RD void lanes_solve(bool split, const float* mq, const float* pq, uint32_t nb, u
         u.w2a = u.w2a + af2a * row_dot(I2a, ai2); u.w2b = u.w2b + af2b * row_dot(I2b, ai2);
     }
     if (id.role) u = us;
-    if (active && id.writer && (id.role == 0 || split)) lane_vel_store(b1, b2, wofs, id, fixed, u);
+    lane_vel_store(b1, b2, wofs, id, active && id.writer && (id.role == 0 || split), fixed, u);
 }
 
 // ---- level schedule of one island (one warp) --------------------------------
@@ -1089,47 +1115,54 @@ static_assert(sizeof(WarpStage) <= LARGE_WARP_SMEM, "warp stage");
 
 // A level's manifolds are taken four at a time (a chunk: order[pos .. end)).
 struct LaneChunk { uint32_t pos, end, L; };
-RD LaneChunk chunk_next(const WarpStage* st, LaneChunk c, uint32_t depth, bool& wrapped) {
-    wrapped = false;
-    c.pos += WARP_MANIFOLDS;
-    if (c.pos >= c.end) {
-        if (++c.L == depth) { c.L = 0; wrapped = true; }
-        c.pos = st->lev[c.L];
-        c.end = st->lev[c.L + 1];
-    }
-    return c;
+RD LaneChunk chunk_next(const WarpStage* st, const LaneChunk& c, uint32_t depth, uint32_t& wrapped) {
+    const bool level = c.pos + WARP_MANIFOLDS >= c.end;
+    const uint32_t L = c.L + (level ? 1u : 0u);
+    wrapped = L == depth ? 1u : 0u;
+    LaneChunk n;
+    n.L = wrapped ? 0u : L;
+    const uint32_t first = st->lev[n.L];
+    n.pos = level ? first : c.pos + WARP_MANIFOLDS;
+    n.end = st->lev[n.L + 1];
+    return n;
 }
-// A lane group's manifold of a chunk (desc row; no points: none) with its
-// impulses, read one chunk ahead (only the manifold itself writes them).
+// A lane group's manifold of a chunk (desc row; no points: none) and its
+// impulses, read one chunk ahead (only the manifold itself writes them): lane
+// q of a half holds point q's and friction impulse q (q < 3).
 struct LaneJob {
     int4 d;
-    float imp[4], f[3];
+    float imp, f;
 };
+// A group without a manifold gets the chunk's first one with no points: its
+// loads and copies are valid and what they bring is discarded (no branches).
 RD int4 chunk_desc(const WarpStage* st, const LaneChunk& c, const LaneId& id) {
     const uint32_t at = c.pos + id.group;
-    return at < c.end ? st->desc[at] : make_int4(0, 0, 0, 0);
+    int4 d = st->desc[at < c.end ? at : c.pos];
+    d.y = at < c.end ? d.y : 0;
+    return d;
 }
 RD void job_load(const DynArgs& a, uint32_t m0, const int4& d, const LaneId& id, LaneJob& j) {
     j.d = d;
-#pragma unroll
-    for (uint32_t k = 0; k < 4; k++)
-        j.imp[k] = k < uint32_t(d.y) ? reinterpret_cast<const float*>(&a.prec[d.w + k].mut)[id.role] : 0.0f;
-    const float4 mut = d.y ? a.mrec[m0 + uint32_t(d.z)].mut : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    j.f[0] = mut.x; j.f[1] = mut.y; j.f[2] = mut.z;
+    const uint32_t k = id.q < uint32_t(d.y) ? id.q : 0u;
+    j.imp = reinterpret_cast<const float*>(&a.prec[uint32_t(d.w) + k].mut)[id.role];
+    j.f = reinterpret_cast<const float*>(&a.mrec[m0 + uint32_t(d.z)].mut)[id.c];
 }
-// Each lane group stages its own manifold's rows.
+// Each lane group stages its own manifold's rows (a lane past the last row
+// copies the last row again).
 RD void chunk_stage(const DynArgs& a, uint32_t m0, LaneSlot* slot, const int4& d, uint32_t lane) {
-    if (d.y) {
-        const uint32_t sub = lane & 7u;
-        const float4* mq = a.mrec[m0 + uint32_t(d.z)].q;
+    const uint32_t sub = lane & 7u;
+    const float4* mq = a.mrec[m0 + uint32_t(d.z)].q;
 #pragma unroll
-        for (uint32_t r = 0; r < DQ_ROWS; r += 8)
-            if (r + sub < DQ_ROWS) cp_async16(&slot->mq[r + sub], mq + r + sub);
-        const float4* pq = a.prec[d.w].q;
-        const uint32_t rows = uint32_t(d.y) * PREC_ROWS;
+    for (uint32_t r = 0; r < DQ_ROWS; r += 8) {
+        const uint32_t row = r + sub < DQ_ROWS ? r + sub : DQ_ROWS - 1;
+        cp_async16(&slot->mq[row], mq + row);
+    }
+    const float4* pq = a.prec[d.w].q;
+    const uint32_t last = (d.y ? uint32_t(d.y) : 1u) * PREC_ROWS - 1;
 #pragma unroll
-        for (uint32_t r = 0; r < 4 * PREC_ROWS; r += 8)
-            if (r + sub < rows) cp_async16(&slot->pq[r + sub], pq + r + sub);
+    for (uint32_t r = 0; r < 4 * PREC_ROWS; r += 8) {
+        const uint32_t row = r + sub < last ? r + sub : last;
+        cp_async16(&slot->pq[row], pq + row);
     }
     cp_async_commit();
 }
@@ -1161,40 +1194,44 @@ RD void solve_staged(const DynArgs& a, uint32_t m0, uint32_t cnt, WarpStage* st,
     LaneJob job, nxt;
     job_load(a, m0, chunk_desc(st, c, id), id, job);
     chunk_stage(a, m0, &st->ring[0][id.group], job.d, lane);
+    uint32_t wrapped;
+    c = chunk_next(st, c, depth, wrapped);
+    int pass_n = int(wrapped);             // pass of the next chunk
+    int4 dn = chunk_desc(st, c, id);       // its manifolds
     cp_async_wait<0>();
     __syncwarp();
     for (;;) {
-        bool wrapped;
-        const LaneChunk cn = chunk_next(st, c, depth, wrapped);
-        const int pass_n = pass + (wrapped ? 1 : 0);
         const bool more = pass_n <= a.iterations;
-        const int4 dn = chunk_desc(st, cn, id);
         if (more) chunk_stage(a, m0, &st->ring[buf ^ 1][id.group], dn, lane);
         if (more && !single) job_load(a, m0, dn, id, nxt);
+        // the chunk after it, looked up while this one is solved
+        c = chunk_next(st, c, depth, wrapped);
+        const int pass_nn = pass_n + int(wrapped);
+        const int4 dnn = chunk_desc(st, c, id);
         const LaneSlot* sl = &st->ring[buf][id.group];
         const float *mq = reinterpret_cast<const float*>(sl->mq), *pq = reinterpret_cast<const float*>(sl->pq);
         const uint32_t nb = uint32_t(job.d.y);
         const bool active = nb != 0;
         float *b1 = vel + 4 * (job.d.x & 0xffff), *b2 = vel + 4 * int(uint32_t(job.d.x) >> 16);
-        const uint32_t nbw = __reduce_max_sync(0xffffffffu, nb);
-        if (pass == 0) lanes_warm(mq, pq, nb, nbw, active, id, b1, b2, wofs, job.imp, job.f);
-        else lanes_solve(a.split != 0, mq, pq, nb, nbw, active, id, b1, b2, wofs, job.imp, job.f);
-        if (active && (lane & 3u) == 0 && (id.role == 0 || (pass != 0 && a.split))) {
-            DynPointRec* pr = a.prec + job.d.w;
+        float imp[4], f[3];
 #pragma unroll
-            for (uint32_t k = 0; k < 4; k++)
-                if (k < nb) reinterpret_cast<float*>(&pr[k].mut)[id.role] = job.imp[k];
-            if (id.role == 0) {
-                float* mut = reinterpret_cast<float*>(&a.mrec[m0 + uint32_t(job.d.z)].mut);
-                mut[0] = job.f[0]; mut[1] = job.f[1]; mut[2] = job.f[2];
-            }
-        }
+        for (int k = 0; k < 4; k++) imp[k] = __shfl_sync(0xffffffffu, job.imp, k, 4);
+#pragma unroll
+        for (int k = 0; k < 3; k++) f[k] = __shfl_sync(0xffffffffu, job.f, k, 4);
+        const uint32_t nbw = __reduce_max_sync(0xffffffffu, nb);
+        if (pass == 0) lanes_warm(mq, pq, nb, nbw, active, id, b1, b2, wofs, imp, f);
+        else lanes_solve(a.split != 0, mq, pq, nb, nbw, active, id, b1, b2, wofs, imp, f);
+        const bool keep = active && (id.role == 0 || (pass != 0 && a.split));
+        st_global_if(keep && id.q < nb, reinterpret_cast<float*>(&a.prec[uint32_t(job.d.w) + id.q].mut) + id.role, lane_pick(id.q, imp));
+        st_global_if(active && id.writer && id.role == 0, reinterpret_cast<float*>(&a.mrec[m0 + uint32_t(job.d.z)].mut) + id.c,
+                     id.c == 0 ? f[0] : (id.c == 1 ? f[1] : f[2]));
         cp_async_wait<0>();
         __syncwarp();
         if (!more) break;
         if (single) job_load(a, m0, dn, id, nxt);
-        c = cn;
         pass = pass_n;
+        pass_n = pass_nn;
+        dn = dnn;
         buf ^= 1;
         job = nxt;
     }
@@ -1272,6 +1309,12 @@ RD void solve_global(const DynArgs& a, uint32_t m0, uint32_t cnt, uint32_t lane)
     }
 }
 
+// Whether the islands of more than BIG_ISLAND manifolds go to kernel 3c with
+// the giant ones: when there is a CTA for each of them.  A CTA takes a level
+// of up to 16 manifolds in one round (a warp four a round) and a chain's level
+// in 1,273-1,841 cycles (a warp 1,697-2,141).
+RD bool big_on_ctas(const DynArgs& a) { return a.giant_smem && a.counters[3] + a.counters[0] <= a.giant_ctas; }
+
 __global__ void __launch_bounds__(LARGE_WARPS * 32, 2) dyn_islands_large(const DynArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1299,7 +1342,7 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32, 2) dyn_islands_large(const D
             __syncwarp();
         }
     }
-    const uint32_t n_big = a.counters[0], n_mid = a.counters[2];
+    const uint32_t n_big = big_on_ctas(a) ? 0u : a.counters[0], n_mid = a.counters[2];
     for (;;) {
         uint32_t k = 0;
         if (lane == 0) k = atomicAdd(a.counters + 1, 1u);
@@ -1399,12 +1442,14 @@ __global__ void __launch_bounds__(64) dyn_joints_position(const DynArgs a) {
 // warm_core / solve_core, the same as the other paths: only where the rows and
 // impulses live changes.  An island that does not fit falls back to the
 // schedule in global scratch (solve_global), run by warp 0.
-constexpr uint32_t GIANT_SOLVERS = 4;  // solver warps; the warp after them stages
+// Solver warps, after the staging warp 0: the first solver, which every level
+// needs, then does not share warp 0's scheduler (the fourth does).
+constexpr uint32_t GIANT_SOLVERS = 4;
 constexpr uint32_t GIANT_RING = GIANT_SOLVERS * WARP_MANIFOLDS;   // manifolds of a level staged (the first 16)
 constexpr uint32_t GIANT_LEVELS = 3;   // levels in the ring
 constexpr uint32_t GIANT_THREADS = (GIANT_SOLVERS + 1) * 32;
 struct __align__(16) GiantSlot {
-    int4 desc;                         // slot 1 | slot 2 << 16, points, manifold (island index), first point
+    int4 desc;                         // 16 * slot 1, 16 * slot 2, points | manifold (island index) << 8, first point
     LaneSlot rows;
 };
 // named barrier 1 over the CTA's warps
@@ -1419,53 +1464,61 @@ struct __align__(16) GiantLevel {
     GiantSlot slot[GIANT_RING];
 };
 
+// The CTA's dynamic shared memory at a byte offset.
+template <class T>
+RD T* gsh(uint32_t off) {
+    extern __shared__ __align__(16) unsigned char gsm[];
+    return reinterpret_cast<T*>(gsm + off);
+}
+// Byte offsets of an island's arrays in the CTA's shared memory (offsets, not
+// pointers: every access is then a shared-memory access to the compiler).
 struct GiantStage {
-    float4 *vel, *mmut;
-    float2* pmut;          // penetration impulse, split impulse
-    GiantLevel* ring;
-    int32_t *hkey, *slot_body;
-    uint32_t* hval;
-    short2* slot;          // slots of body 1 / body 2
-    uint16_t *order, *klev, *lev;
-    uint32_t* pofs;        // first point of each manifold, relative to the island's first point
-    uint8_t* npt;
+    uint32_t vel;          // float4 x 4 nbmax: constrained v, w, split v, w
+    uint32_t mmut;         // float4 a manifold: friction impulses
+    uint32_t pmut;         // float2 a point: penetration impulse, split impulse
+    uint32_t ring;         // GiantLevel x GIANT_LEVELS
+    uint32_t hkey, hval, slot_body;
+    uint32_t slot;         // short2: slots of body 1 / body 2
+    uint32_t order, klev, lev;   // uint16
+    uint32_t pofs;         // uint32: first point of each manifold, relative to the island's first point
+    uint32_t npt;          // uint8
     uint32_t H, nbmax;
 };
 
-RD bool giant_layout(const DynArgs& a, uint32_t cnt, uint32_t np, unsigned char* sm, GiantStage& g) {
+RD bool giant_layout(const DynArgs& a, uint32_t cnt, uint32_t np, GiantStage& g) {
     if (cnt > 65535u) return false;
     g.nbmax = 2 * cnt < a.nb ? 2 * cnt : a.nb;
     if (g.nbmax > 32767u) return false;
     g.H = 1;
     while (g.H < 2 * g.nbmax) g.H <<= 1;
     size_t off = 0;
-    auto take = [&](size_t bytes) { const size_t o = off; off = (off + bytes + 15) & ~size_t(15); return sm + o; };
-    g.vel = reinterpret_cast<float4*>(take(size_t(4) * g.nbmax * 16));
-    g.mmut = reinterpret_cast<float4*>(take(size_t(cnt) * 16));
-    g.pmut = reinterpret_cast<float2*>(take(size_t(np) * 8));
-    g.ring = reinterpret_cast<GiantLevel*>(take(size_t(GIANT_LEVELS) * sizeof(GiantLevel)));
-    g.hkey = reinterpret_cast<int32_t*>(take(size_t(g.H) * 4));
-    g.hval = reinterpret_cast<uint32_t*>(take(size_t(g.H) * 4));
-    g.slot_body = reinterpret_cast<int32_t*>(take(size_t(g.nbmax) * 4));
-    g.slot = reinterpret_cast<short2*>(take(size_t(cnt) * 4));
-    g.order = reinterpret_cast<uint16_t*>(take(size_t(cnt) * 2));
-    g.klev = reinterpret_cast<uint16_t*>(take(size_t(cnt) * 2));
-    g.lev = reinterpret_cast<uint16_t*>(take(size_t(cnt + 1) * 2));
-    g.pofs = reinterpret_cast<uint32_t*>(take(size_t(cnt) * 4));
+    auto take = [&](size_t bytes) { const size_t o = off; off = (off + bytes + 15) & ~size_t(15); return uint32_t(o); };
+    g.vel = take(size_t(4) * g.nbmax * 16);
+    g.mmut = take(size_t(cnt) * 16);
+    g.pmut = take(size_t(np) * 8);
+    g.ring = take(size_t(GIANT_LEVELS) * sizeof(GiantLevel));
+    g.hkey = take(size_t(g.H) * 4);
+    g.hval = take(size_t(g.H) * 4);
+    g.slot_body = take(size_t(g.nbmax) * 4);
+    g.slot = take(size_t(cnt) * 4);
+    g.order = take(size_t(cnt) * 2);
+    g.klev = take(size_t(cnt) * 2);
+    g.lev = take(size_t(cnt + 1) * 2);
+    g.pofs = take(size_t(cnt) * 4);
     g.npt = take(size_t(cnt));
     return off <= a.giant_smem;
 }
 
 // Schedule an island (warp 0); false (nothing written to global memory) when
 // it does not fit or its points are not one contiguous range.
-RD bool giant_schedule(const DynArgs& a, uint32_t m0, uint32_t cnt, unsigned char* sm, GiantStage& g,
+RD bool giant_schedule(const DynArgs& a, uint32_t m0, uint32_t cnt, GiantStage& g,
                        uint32_t lane, uint32_t& depth, uint32_t* nslots, uint32_t& p0) {
     const int4 f = man_ids(a, m0), l = man_ids(a, m0 + cnt - 1);
     p0 = uint32_t(f.w);
     const int64_t end = int64_t(l.w) + int64_t(l.z);
     if (f.w < 0 || end < int64_t(p0) || end > int64_t(a.np)) return false;
     const uint32_t np = uint32_t(end - int64_t(p0));
-    if (!giant_layout(a, cnt, np, sm, g)) return false;
+    if (!giant_layout(a, cnt, np, g)) return false;
     uint32_t expect = 0;
     for (uint32_t base = 0; base < cnt; base += 32) {
         const uint32_t k = base + lane;
@@ -1474,8 +1527,8 @@ RD bool giant_schedule(const DynArgs& a, uint32_t m0, uint32_t cnt, unsigned cha
             const int4 id = man_ids(a, m0 + k);
             pofs = uint32_t(id.w) - p0;
             npt = uint32_t(id.z < 0 ? 0 : (id.z > 255 ? 255 : id.z));
-            g.pofs[k] = pofs;
-            g.npt[k] = uint8_t(npt);
+            gsh<uint32_t>(g.pofs)[k] = pofs;
+            gsh<uint8_t>(g.npt)[k] = uint8_t(npt);
         }
         uint32_t inc = npt;
         for (int o = 1; o < 32; o <<= 1) {
@@ -1487,9 +1540,9 @@ RD bool giant_schedule(const DynArgs& a, uint32_t m0, uint32_t cnt, unsigned cha
     }
     if (expect != np) return false;
     IslandSched S;
-    S.hkey = g.hkey; S.hval = g.hval; S.H = g.H;
-    S.slot_body = g.slot_body; S.nbmax = g.nbmax;
-    S.slot = g.slot; S.klev = g.klev; S.order = g.order; S.lev = g.lev;
+    S.hkey = gsh<int32_t>(g.hkey); S.hval = gsh<uint32_t>(g.hval); S.H = g.H;
+    S.slot_body = gsh<int32_t>(g.slot_body); S.nbmax = g.nbmax;
+    S.slot = gsh<short2>(g.slot); S.klev = gsh<uint16_t>(g.klev); S.order = gsh<uint16_t>(g.order); S.lev = gsh<uint16_t>(g.lev);
     S.nslots = nslots;
     return island_schedule(a, m0, cnt, S, lane, depth);
 }
@@ -1501,16 +1554,16 @@ struct GiantCursor { uint32_t t, L, ring; };
 RD void giant_stage_level(const DynArgs& a, const GiantStage& g, uint32_t m0, uint32_t p0, uint32_t depth,
                           uint32_t total, GiantCursor& S, uint32_t lane) {
     if (S.t < total) {
-        const uint32_t first = g.lev[S.L], width = g.lev[S.L + 1] - first;
-        GiantLevel* R = g.ring + S.ring;
+        const uint16_t* lev = gsh<uint16_t>(g.lev);
+        const uint32_t first = lev[S.L], width = lev[S.L + 1] - first;
+        GiantLevel* R = gsh<GiantLevel>(g.ring) + S.ring;
         uint32_t kk = 0, np = 0, pofs = 0;
         if (lane < GIANT_RING && lane < width) {
-            kk = g.order[first + lane];
-            const short2 bs = g.slot[kk];
-            np = g.npt[kk];
-            pofs = g.pofs[kk];
-            R->slot[lane].desc = make_int4(int(uint32_t(uint16_t(bs.x)) | (uint32_t(uint16_t(bs.y)) << 16)), int(np),
-                                           int(kk), int(pofs));
+            kk = gsh<uint16_t>(g.order)[first + lane];
+            const short2 bs = gsh<short2>(g.slot)[kk];
+            np = gsh<uint8_t>(g.npt)[kk];
+            pofs = gsh<uint32_t>(g.pofs)[kk];
+            R->slot[lane].desc = make_int4(16 * int(bs.x), 16 * int(bs.y), int(np | kk << 8), int(pofs));
         }
         const uint32_t n = width < GIANT_RING ? width : GIANT_RING;
         for (uint32_t s = 0; s < n; s++) {
@@ -1520,8 +1573,10 @@ RD void giant_stage_level(const DynArgs& a, const GiantStage& g, uint32_t m0, ui
             const float4* pq = a.prec[ns ? p0 + ps : 0u].q;
             float4* dst = R->slot[s].rows.mq;   // the point rows follow the manifold's
             const uint32_t rows = DQ_ROWS + ns * PREC_ROWS;
-            if (lane < rows) cp_async16(dst + lane, lane < DQ_ROWS ? mq + lane : pq + (lane - DQ_ROWS));
-            if (lane + 32 < rows) cp_async16(dst + lane + 32, pq + (lane + 32 - DQ_ROWS));
+            // (a lane past the last row copies the last row again)
+            const uint32_t r0 = lane < rows ? lane : rows - 1, r1 = lane + 32 < rows ? lane + 32 : rows - 1;
+            cp_async16(dst + r0, r0 < DQ_ROWS ? mq + r0 : pq + (r0 - DQ_ROWS));
+            cp_async16(dst + r1, r1 < DQ_ROWS ? mq + r1 : pq + (r1 - DQ_ROWS));
         }
         uint32_t w = np;
         for (int o = 1; o < int(WARP_MANIFOLDS); o <<= 1) {
@@ -1539,47 +1594,50 @@ RD void giant_stage_level(const DynArgs& a, const GiantStage& g, uint32_t m0, ui
 
 // A lane group's staged manifold of a level, its impulses in shared memory.
 RD void giant_manifold(const DynArgs& a, const GiantStage& g, const LaneId& id, bool warm, const GiantSlot* sl,
-                       bool active, uint32_t nbw, uint32_t lane) {
-    const int4 d = sl->desc;
-    const uint32_t nb = active ? uint32_t(d.y) : 0u;
+                       int4 d, bool active, uint32_t nbw) {
+    d.x = active ? d.x : 0; d.y = active ? d.y : 0; d.z = active ? d.z : 0; d.w = active ? d.w : 0;
+    const uint32_t nb = uint32_t(d.z) & 255u;
     active = nb != 0;
-    float* vel = reinterpret_cast<float*>(g.vel) + size_t(8) * g.nbmax * id.role;
-    float* b1 = vel + (active ? 4 * (d.x & 0xffff) : 0);
-    float* b2 = vel + (active ? 4 * int(uint32_t(d.x) >> 16) : 0);
+    const uint32_t vel = g.vel + 32 * g.nbmax * id.role;
+    float *b1 = gsh<float>(vel + uint32_t(d.x)), *b2 = gsh<float>(vel + uint32_t(d.y));
     const uint32_t wofs = 4 * g.nbmax;
-    float* pm = reinterpret_cast<float*>(g.pmut + (active ? d.w : 0)) + id.role;
-    float* mm = reinterpret_cast<float*>(g.mmut + (active ? d.z : 0));
+    float* pm = gsh<float>(g.pmut + 8 * uint32_t(d.w) + 4 * id.role);
+    float* mm = gsh<float>(g.mmut + (uint32_t(d.z) >> 8 << 4));
     const float *mq = reinterpret_cast<const float*>(sl->rows.mq), *pq = reinterpret_cast<const float*>(sl->rows.pq);
     float imp[4], f[3];
+    // a point's impulse behind the island's last is the next array's: read and discarded
 #pragma unroll
-    for (uint32_t k = 0; k < 4; k++) imp[k] = k < nb ? pm[2 * k] : 0.0f;
+    for (uint32_t k = 0; k < 4; k++) imp[k] = pm[2 * k];
     f[0] = mm[0]; f[1] = mm[1]; f[2] = mm[2];
     if (warm) lanes_warm(mq, pq, nb, nbw, active, id, b1, b2, wofs, imp, f);
     else lanes_solve(a.split != 0, mq, pq, nb, nbw, active, id, b1, b2, wofs, imp, f);
-    if (active && (lane & 3u) == 0 && (id.role == 0 || (!warm && a.split))) {
-#pragma unroll
-        for (uint32_t k = 0; k < 4; k++)
-            if (k < nb) pm[2 * k] = imp[k];
-        if (id.role == 0) { mm[0] = f[0]; mm[1] = f[1]; mm[2] = f[2]; }
-    }
+    const bool keep = active && (id.role == 0 || (!warm && a.split));
+    st_shared_if(keep && id.q < nb, pm + 2 * id.q, lane_pick(id.q, imp));
+    st_shared_if(active && id.writer && id.role == 0, mm + id.c, id.c == 0 ? f[0] : (id.c == 1 ? f[1] : f[2]));
 }
 
 // All warps: stage, solve and write back one island.
 RD void giant_solve(const DynArgs& a, uint32_t m0, uint32_t cnt, const GiantStage& g, uint32_t warp,
                     uint32_t lane, uint32_t depth, uint32_t nslots, uint32_t p0) {
-    const uint32_t np = g.pofs[cnt - 1] + g.npt[cnt - 1];
+    const uint32_t np = gsh<uint32_t>(g.pofs)[cnt - 1] + gsh<uint8_t>(g.npt)[cnt - 1];
     const uint32_t tid = warp * 32 + lane;
+    float4 *vel = gsh<float4>(g.vel), *mmut = gsh<float4>(g.mmut);
+    float2* pmut = gsh<float2>(g.pmut);
+    const int32_t* slot_body = gsh<int32_t>(g.slot_body);
     for (uint32_t s = tid; s < nslots; s += GIANT_THREADS) {
-        const int32_t e = g.slot_body[s], b = e < 0 ? -1 - e : e;
-        g.vel[s] = a.cv[b];
-        g.vel[g.nbmax + s] = a.cw[b];
-        g.vel[2 * g.nbmax + s] = a.sv[b];
-        g.vel[3 * g.nbmax + s] = a.sw[b];
+        const int32_t e = slot_body[s], b = e < 0 ? -1 - e : e;
+        vel[s] = a.cv[b];
+        vel[g.nbmax + s] = a.cw[b];
+        vel[2 * g.nbmax + s] = a.sv[b];
+        vel[3 * g.nbmax + s] = a.sw[b];
     }
-    for (uint32_t k = tid; k < cnt; k += GIANT_THREADS) g.mmut[k] = a.mrec[m0 + k].mut;
-    for (uint32_t p = tid; p < np; p += GIANT_THREADS) g.pmut[p] = *reinterpret_cast<const float2*>(&a.prec[p0 + p].mut);
+    for (uint32_t k = tid; k < cnt; k += GIANT_THREADS) mmut[k] = a.mrec[m0 + k].mut;
+    for (uint32_t p = tid; p < np; p += GIANT_THREADS) {
+        const float4 v = a.prec[p0 + p].mut;
+        pmut[p] = make_float2(v.x, v.y);
+    }
     const uint32_t total = uint32_t(a.iterations + 1) * depth;
-    if (warp == GIANT_SOLVERS) {
+    if (warp == 0) {
         GiantCursor S{0, 0, 0};
         giant_stage_level(a, g, m0, p0, depth, total, S, lane);
         giant_stage_level(a, g, m0, p0, depth, total, S, lane);
@@ -1593,28 +1651,31 @@ RD void giant_solve(const DynArgs& a, uint32_t m0, uint32_t cnt, const GiantStag
         cp_async_wait<0>();
     } else {
         const LaneId id = lane_id(lane);
+        const uint32_t solver = warp - 1;
         cta_bar<GIANT_THREADS>();
         uint32_t ring = 0;
         for (uint32_t t = 0; t < total; t++) {
             const bool warm = t < depth;
-            const GiantLevel* R = g.ring + ring;
-            const uint32_t at = warp * WARP_MANIFOLDS + id.group;
-            const uint32_t nbw = R->nbw[warp], b = R->first, width = R->width, e = b + width;
-            if (nbw) giant_manifold(a, g, id, warm, &R->slot[at], at < width, nbw, lane);
+            const GiantLevel* R = gsh<GiantLevel>(g.ring) + ring;
+            const uint32_t at = solver * WARP_MANIFOLDS + id.group;
+            const uint32_t nbw = R->nbw[solver], b = R->first, width = R->width, e = b + width;
+            const int4 d = R->slot[at].desc;
+            if (nbw) giant_manifold(a, g, id, warm, &R->slot[at], d, at < width, nbw);
             // a level's manifolds beyond the staged ones: one a lane, their rows
             // from global memory
-            for (uint32_t j = b + GIANT_RING + warp * 32 + lane; j < e; j += GIANT_SOLVERS * 32) {
-                const uint32_t kk = g.order[j];
-                const short2 bs = g.slot[kk];
+            if (width > GIANT_RING)
+            for (uint32_t j = b + GIANT_RING + solver * 32 + lane; j < e; j += GIANT_SOLVERS * 32) {
+                const uint32_t kk = gsh<uint16_t>(g.order)[j], npt = gsh<uint8_t>(g.npt)[kk], pofs = gsh<uint32_t>(g.pofs)[kk];
+                const short2 bs = gsh<short2>(g.slot)[kk];
                 BodyVel bv;
                 const uint32_t n = g.nbmax;
-                bv.v1 = g.vel + bs.x; bv.w1 = bv.v1 + n; bv.s1 = bv.w1 + n; bv.t1 = bv.s1 + n;
-                bv.v2 = g.vel + bs.y; bv.w2 = bv.v2 + n; bv.s2 = bv.w2 + n; bv.t2 = bv.s2 + n;
-                RecSrc r = rec_global(a, m0 + kk, int32_t(g.npt[kk] ? p0 + g.pofs[kk] : 0u));
-                r.mmut = g.mmut + kk;
-                r.pm2 = g.pmut + g.pofs[kk];
-                if (warm) warm_core<true, true>(a, r, bv, g.npt[kk]);
-                else solve_core<true, true>(a, r, bv, g.npt[kk]);
+                bv.v1 = vel + bs.x; bv.w1 = bv.v1 + n; bv.s1 = bv.w1 + n; bv.t1 = bv.s1 + n;
+                bv.v2 = vel + bs.y; bv.w2 = bv.v2 + n; bv.s2 = bv.w2 + n; bv.t2 = bv.s2 + n;
+                RecSrc r = rec_global(a, m0 + kk, int32_t(npt ? p0 + pofs : 0u));
+                r.mmut = mmut + kk;
+                r.pm2 = pmut + pofs;
+                if (warm) warm_core<true, true>(a, r, bv, int32_t(npt));
+                else solve_core<true, true>(a, r, bv, int32_t(npt));
             }
             __syncwarp();
             cta_bar<GIANT_THREADS>();
@@ -1623,15 +1684,20 @@ RD void giant_solve(const DynArgs& a, uint32_t m0, uint32_t cnt, const GiantStag
     }
     __syncthreads();
     for (uint32_t s = tid; s < nslots; s += GIANT_THREADS) {
-        const int32_t b = g.slot_body[s];
+        const int32_t b = slot_body[s];
         if (b < 0) continue;
-        a.cv[b] = g.vel[s];
-        a.cw[b] = g.vel[g.nbmax + s];
-        a.sv[b] = g.vel[2 * g.nbmax + s];
-        a.sw[b] = g.vel[3 * g.nbmax + s];
+        a.cv[b] = vel[s];
+        a.cw[b] = vel[g.nbmax + s];
+        a.sv[b] = vel[2 * g.nbmax + s];
+        a.sw[b] = vel[3 * g.nbmax + s];
     }
-    for (uint32_t k = tid; k < cnt; k += GIANT_THREADS) a.mrec[m0 + k].mut = g.mmut[k];
-    for (uint32_t p = tid; p < np; p += GIANT_THREADS) *reinterpret_cast<float2*>(&a.prec[p0 + p].mut) = g.pmut[p];
+    for (uint32_t k = tid; k < cnt; k += GIANT_THREADS) a.mrec[m0 + k].mut = mmut[k];
+    for (uint32_t p = tid; p < np; p += GIANT_THREADS) {
+        float* mut = reinterpret_cast<float*>(&a.prec[p0 + p].mut);
+        const float2 v = pmut[p];
+        mut[0] = v.x;
+        mut[1] = v.y;
+    }
     __syncthreads();
 }
 
@@ -1849,17 +1915,16 @@ RD void stream_solve(const DynArgs& a, uint32_t m0, StreamSlot* ring, uint32_t w
 }
 
 __global__ void __launch_bounds__(GIANT_THREADS, 1) dyn_islands_giant(const DynArgs a) {
-    extern __shared__ __align__(16) unsigned char gsm[];
     __shared__ uint32_t s_island, s_ok, s_depth, s_nslots, s_p0;
     constexpr uint32_t SCHED_WARP = 0;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t n_giant = a.counters[3];
+    const uint32_t n_giant = a.counters[3], n_big = big_on_ctas(a) ? a.counters[0] : 0u;
     for (;;) {
         if (threadIdx.x == 0) s_island = atomicAdd(a.counters + 4, 1u);
         __syncthreads();
         const uint32_t k = s_island;
-        if (k >= n_giant) break;
-        const uint32_t is = a.giant_list[k];
+        if (k >= n_giant + n_big) break;
+        const uint32_t is = k < n_giant ? a.giant_list[k] : a.large_list[k - n_giant];
         if (is == ISLAND_DONE) {
             __syncthreads();
             continue;
@@ -1868,7 +1933,7 @@ __global__ void __launch_bounds__(GIANT_THREADS, 1) dyn_islands_giant(const DynA
         GiantStage g;
         if (warp == SCHED_WARP) {
             uint32_t depth = 0, p0 = 0;
-            const bool ok = giant_schedule(a, m0, cnt, gsm, g, lane, depth, &s_nslots, p0);
+            const bool ok = giant_schedule(a, m0, cnt, g, lane, depth, &s_nslots, p0);
             if (lane == 0) { s_ok = ok ? 1u : 0u; s_depth = depth; s_p0 = p0; }
         }
         __syncthreads();
@@ -1876,7 +1941,7 @@ __global__ void __launch_bounds__(GIANT_THREADS, 1) dyn_islands_giant(const DynA
             if (warp != SCHED_WARP) {
                 // the same layout (a pure function of the island's sizes)
                 const int4 l = man_ids(a, m0 + cnt - 1);
-                giant_layout(a, cnt, uint32_t(int64_t(l.w) + int64_t(l.z) - int64_t(s_p0)), gsm, g);
+                giant_layout(a, cnt, uint32_t(int64_t(l.w) + int64_t(l.z) - int64_t(s_p0)), g);
             }
             giant_solve(a, m0, cnt, g, warp, lane, s_depth, s_nslots, s_p0);
         } else if (size_t(GIANT_LEVELS) * STREAM_RING * sizeof(StreamSlot) + GIANT_LEVELS * sizeof(int2) <= a.giant_smem) {
