@@ -12,10 +12,11 @@ namespace rp3dg {
 // The world's dynamic AABB tree as RayNode records (rp3dg_internal.h): a
 // leaf has child 0 = -2 - collider index.
 // Per collider (creation order): x device row of its world transform,
-// y body index, z shape index, w collision category bits.
+// y body index, z shape index, w collision category bits | shape kind << 16.
 struct RayArgs {
     const RayNode* nodes;
     int32_t root;
+    int32_t finite_nodes;          // every node's bounds are finite numbers
     const int4* colliders;
     const float4* c_wpos;          // collider local-to-world position, by row
     const float4* c_wori;          // and orientation
@@ -31,9 +32,10 @@ struct RayArgs {
     uint32_t max_hits;
     rp3dg_raycast_hit* hits;       // n * max_hits
     uint32_t* nb_hits;             // n
+    uint32_t* queue;               // rays handed out so far, 0 before the launch
     uint32_t* error;               // bit 0: a traversal stack overflowed (world or mesh tree)
 };
 
-cudaError_t launch_world_raycast(const RayArgs& a, cudaStream_t stream);
+cudaError_t launch_world_raycast(const RayArgs& a, int num_sms, cudaStream_t stream);
 
 }  // namespace rp3dg

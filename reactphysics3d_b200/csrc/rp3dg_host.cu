@@ -380,6 +380,7 @@ int get_shapes_host(rp3dg_ctx* ctx, std::vector<rp3dg_shape>* out) {
     return 0;
 }
 // the device shape table and its local bounds (2 float4 per shape)
+int get_num_sms(const rp3dg_ctx* ctx) { return ctx->num_sms; }
 int get_shape_device(rp3dg_ctx* ctx, const rp3dg_shape** shapes, const float4** bounds) {
     if (!ctx) return RP3DG_EINVAL;
     *shapes = ctx->d_shapes;

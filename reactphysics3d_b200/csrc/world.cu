@@ -78,6 +78,7 @@ int get_mesh_arena_device(rp3dg_ctx* ctx, const uint32_t** words);
 int get_mesh_mass(rp3dg_ctx* ctx, int32_t instance, float* volume, float* extent);
 int get_mesh_face_counts(rp3dg_ctx* ctx, int32_t instance, std::vector<uint32_t>* counts);
 int get_cmeshes(rp3dg_ctx* ctx, std::vector<CmDesc>* out);
+int get_num_sms(const rp3dg_ctx* ctx);
 int get_shape_device(rp3dg_ctx* ctx, const rp3dg_shape** shapes, const float4** bounds);
 int narrowphase_tri_device(rp3dg_ctx* ctx, int algorithm, const rp3dg_pair_batch* p, const rp3dg_contact_batch* out,
                            const float4* tri);
@@ -950,12 +951,14 @@ struct rp3dg_world {
     uint32_t ray_world = 0;
     rp3dg::RayNode *h_rnodes = nullptr, *d_rnodes = nullptr;
     int4 *h_rcols = nullptr, *d_rcols = nullptr;
-    size_t cap_rnodes = 0, cap_rcols = 0, cap_rhf = 0, cap_rays = 0, cap_rhits = 0, cap_rcount = 0;
+    size_t cap_rnodes = 0, cap_rcols = 0, cap_rhf = 0, cap_rays = 0, cap_rhits = 0, cap_rcount = 0, cap_rwork = 0;
     rp3dg::HfDesc* d_rhf = nullptr;
     uint32_t nb_rhf = 0;
     rp3dg_ray* d_rays = nullptr;
     rp3dg_raycast_hit* d_rhits = nullptr;
-    uint32_t* d_rcount = nullptr;    // n counts, then the error word
+    uint32_t* d_rcount = nullptr;    // n counts
+    uint32_t* d_rwork = nullptr;     // error word, rays handed out
+    bool ray_finite = false;         // every node of the tables has finite bounds
     cudaEvent_t ev_r0 = nullptr, ev_r1 = nullptr;
     // manifold packing
     size_t cap_m = 0, cap_i = 0;
@@ -2358,7 +2361,7 @@ void destroy_group(Group* g) {
     cudaFree(g->d_tree); cudaFree(g->d_tree_base); cudaFree(g->d_tree_hdr);
     cudaFreeHost(g->h_gq); cudaFree(g->d_gq);
     cudaFreeHost(g->h_rnodes); cudaFree(g->d_rnodes); cudaFreeHost(g->h_rcols); cudaFree(g->d_rcols);
-    cudaFree(g->d_rhf); cudaFree(g->d_rays); cudaFree(g->d_rhits); cudaFree(g->d_rcount);
+    cudaFree(g->d_rhf); cudaFree(g->d_rays); cudaFree(g->d_rhits); cudaFree(g->d_rcount); cudaFree(g->d_rwork);
     if (g->ev_r0) cudaEventDestroy(g->ev_r0);
     if (g->ev_r1) cudaEventDestroy(g->ev_r1);
     if (g->ev_rect) cudaEventDestroy(g->ev_rect);
@@ -3650,8 +3653,10 @@ int ray_tables(Group* g, uint32_t world) {
     if (!pair_grow(&g->h_rnodes, &g->d_rnodes, &g->cap_rnodes, nn) ||
         !pair_grow(&g->h_rcols, &g->d_rcols, &g->cap_rcols, nc))
         return wfail(g, RP3DG_ENOMEM, "allocation of raycast tables");
+    bool finite = true;
     for (size_t k = 0; k < w.tree.nodes.size(); k++) {
         const rp3dg::order::Tree::Node& N = w.tree.nodes[k];
+        for (int i = 0; i < 3; i++) finite = finite && std::fabs(N.box.mn[i]) <= FLT_MAX && std::fabs(N.box.mx[i]) <= FLT_MAX;
         rp3dg::RayNode& R = g->h_rnodes[k];
         const bool leaf = N.height == 0;
         const int c0 = leaf ? -2 - N.data : N.child[0];
@@ -3661,7 +3666,8 @@ int ray_tables(Group* g, uint32_t world) {
     }
     for (size_t c = 0; c < w.colliders.size(); c++) {
         const ColliderH& C = w.colliders[c];
-        g->h_rcols[c] = make_int4(int(w.c0) + w.ccomp.slot[c], C.body, C.shape, int(C.category));
+        g->h_rcols[c] = make_int4(int(w.c0) + w.ccomp.slot[c], C.body, C.shape,
+                                  int(uint32_t(C.category) | uint32_t(g->shapes[size_t(C.shape)].kind) << 16));
     }
     std::vector<rp3dg::HfDesc> hf;
     rp3dg::get_heightfields(g->ctx, &hf);
@@ -3677,6 +3683,7 @@ int ray_tables(Group* g, uint32_t world) {
     if (e != cudaSuccess) return wcuda(g, e, "raycast tables");
     g->ray_version = g->state_version;
     g->ray_world = world;
+    g->ray_finite = finite;
     return 0;
 }
 
@@ -3685,7 +3692,7 @@ int raycast_device(Group* g, uint32_t world, const rp3dg_ray* rays, uint32_t n, 
                    rp3dg_raycast_hit* hits, uint32_t* nb_hits, float* kernel_ms) {
     int rc = ray_tables(g, world);
     if (rc) return rc;
-    if (dev_grow(&g->d_rcount, &g->cap_rcount, 1))
+    if (dev_grow(&g->d_rwork, &g->cap_rwork, 2))
         return wfail(g, RP3DG_ENOMEM, "allocation of the raycast error word");
     if (!g->ev_r0 && (cudaEventCreate(&g->ev_r0) != cudaSuccess || cudaEventCreate(&g->ev_r1) != cudaSuccess))
         return wfail(g, RP3DG_ECUDA, "cudaEventCreate(raycast)");
@@ -3694,6 +3701,7 @@ int raycast_device(Group* g, uint32_t world, const rp3dg_ray* rays, uint32_t n, 
     rp3dg::RayArgs a{};
     a.nodes = g->d_rnodes;
     a.root = w.tree.root;
+    a.finite_nodes = g->ray_finite ? 1 : 0;
     a.colliders = g->d_rcols;
     a.c_wpos = g->ccol[g->cur_c][CC_WPOS];
     a.c_wori = g->ccol[g->cur_c][CC_WORI];
@@ -3710,14 +3718,15 @@ int raycast_device(Group* g, uint32_t world, const rp3dg_ray* rays, uint32_t n, 
     a.max_hits = max_hits;
     a.hits = hits;
     a.nb_hits = nb_hits;
-    a.error = g->d_rcount;
-    cudaMemsetAsync(g->d_rcount, 0, sizeof(uint32_t), st);
+    a.error = g->d_rwork;
+    a.queue = g->d_rwork + 1;
+    cudaMemsetAsync(g->d_rwork, 0, 2 * sizeof(uint32_t), st);
     cudaEventRecord(g->ev_r0, st);
-    cudaError_t e = rp3dg::launch_world_raycast(a, st);
+    cudaError_t e = rp3dg::launch_world_raycast(a, rp3dg::get_num_sms(g->ctx), st);
     cudaEventRecord(g->ev_r1, st);
     if (e != cudaSuccess) return wcuda(g, e, "raycast kernel");
     uint32_t err = 0;
-    cudaMemcpyAsync(&err, g->d_rcount, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(&err, g->d_rwork, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return wcuda(g, e, "raycast");
     if (kernel_ms) cudaEventElapsedTime(kernel_ms, g->ev_r0, g->ev_r1);
@@ -3748,12 +3757,11 @@ int rp3dg_world_raycast(rp3dg_world* g, uint32_t world, const rp3dg_ray* rays, u
     if (rc || n == 0) return rc;
     const size_t nh = size_t(n) * max_hits;
     if (dev_grow(&g->d_rays, &g->cap_rays, n) || dev_grow(&g->d_rhits, &g->cap_rhits, std::max<size_t>(nh, 1)) ||
-        dev_grow(&g->d_rcount, &g->cap_rcount, size_t(n) + 1))
+        dev_grow(&g->d_rcount, &g->cap_rcount, n))
         return wfail(g, RP3DG_ENOMEM, "allocation of raycast buffers");
     cudaStream_t st = g->stream;
     cudaMemcpyAsync(g->d_rays, rays, size_t(n) * sizeof(rp3dg_ray), cudaMemcpyHostToDevice, st);
-    // the error word sits after the counts
-    uint32_t* counts = g->d_rcount + 1;
+    uint32_t* counts = g->d_rcount;
     rc = raycast_device(g, world, g->d_rays, n, mode, max_hits, g->d_rhits, counts, nullptr);
     if (rc) return rc;
     if (nh) cudaMemcpyAsync(hits, g->d_rhits, nh * sizeof(rp3dg_raycast_hit), cudaMemcpyDeviceToHost, st);
