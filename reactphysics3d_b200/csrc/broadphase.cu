@@ -12,13 +12,12 @@
 // which is when its fat AABB changes).  Here that set is computed directly,
 // two ways:
 //   - LBVH (the default): 30-bit Morton codes of the fat-AABB centres with
-//     the group (world) in the bits above, an LSD radix sort, a Karras tree
-//     over the sorted keys (ties broken by sorted position), a bottom-up refit
-//     with one atomic visit counter per node, and a traversal in which the 32
-//     lanes of a warp hold 32 Morton-consecutive colliders and walk one shared
-//     stack (a node is opened when any lane's fat AABB overlaps it; a lane
-//     only looks for partners later in the sorted order, so each pair is
-//     found once), with a count pass, an exclusive scan and a write pass;
+//     the group (world) in the bits above, an LSD radix sort, the radix tree
+//     over the sorted keys (ties broken by sorted position) built and boxed
+//     bottom-up in one pass, and one walk per collider (32 Morton-consecutive
+//     ones a warp) that looks for partners later in the sorted order, so each
+//     pair is found once; the partners found are kept and written out at the
+//     collider's offset by a second kernel;
 //   - sort and sweep along one axis: an LSD radix sort of the colliders by
 //     (group, fat min on the sweep axis), then each collider scans forward
 //     while the next minimum is within its maximum.
@@ -70,28 +69,6 @@ __global__ void __launch_bounds__(128) bp_update_kernel(const BpArgs a) {
     a.moved[i] = 1;
 }
 
-// ---- radix sort of 64-bit keys with 32-bit values (LSD, 8-bit digits) ---
-constexpr int SORT_THREADS = 256;
-constexpr int SORT_ITEMS = 8;
-constexpr uint32_t SORT_TILE = SORT_THREADS * SORT_ITEMS;   // 2048 keys per block
-constexpr int SORT_WARPS = SORT_THREADS / 32;
-
-RD uint32_t digit_of(unsigned long long k, int shift) { return uint32_t(k >> shift) & 0xffu; }
-
-__global__ void __launch_bounds__(SORT_THREADS) sort_hist(const unsigned long long* __restrict__ keys, uint32_t n,
-                                                          int shift, uint32_t nblocks, uint32_t* __restrict__ hist) {
-    __shared__ uint32_t h[256];
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    const uint32_t base = blockIdx.x * SORT_TILE;
-    for (int k = 0; k < SORT_ITEMS; k++) {
-        const uint32_t idx = base + k * SORT_THREADS + threadIdx.x;
-        if (idx < n) atomicAdd(&h[digit_of(keys[idx], shift)], 1u);
-    }
-    __syncthreads();
-    hist[threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
-}
-
 // Exclusive scan of n uint32 in place, one block of 1024 threads (each
 // thread scans a contiguous segment).
 __global__ void __launch_bounds__(1024) scan_small(uint32_t* __restrict__ v, uint32_t n, uint32_t* __restrict__ total) {
@@ -117,52 +94,150 @@ __global__ void __launch_bounds__(1024) scan_small(uint32_t* __restrict__ v, uin
     if (total && threadIdx.x == 1023) *total = part[1023];
 }
 
+// ---- radix sort of 64-bit keys with 32-bit values (LSD, 10-bit digits) ---
+//
+// Two kernels a pass: digit counts per tile of 2,048 keys (tile-major), and a
+// scatter whose blocks add up the counts of the tiles before theirs
+// themselves: a row of 1,024 counts a tile, read coalesced, 49 rows for
+// 100,000 keys (a one-block scan between the two took 17 us a pass).  Above
+// SORT_SUM_TILES tiles, where the rows read grow with the square, a kernel
+// turns the counts into running sums first.  Ten bits make three passes of a
+// 30-bit Morton code: 18 us a pass for 100,000 keys, latency of the rows and
+// of the ranking; tiles of 1,024 keys took 23.
+constexpr int SORT_BITS = 10;
+constexpr uint32_t SORT_RADIX = 1u << SORT_BITS;
+constexpr int SORT_THREADS = 256;
+constexpr int SORT_ITEMS = 8;
+constexpr uint32_t SORT_TILE = SORT_THREADS * SORT_ITEMS;   // 2048 keys per block
+constexpr int SORT_WARPS = SORT_THREADS / 32;
+constexpr uint32_t SORT_SUM_TILES = 512;
+static_assert(SORT_RADIX == 4 * SORT_THREADS, "four digits a thread");
+
+RD uint32_t digit_of(unsigned long long k, int shift) { return uint32_t(k >> shift) & (SORT_RADIX - 1u); }
+
+__global__ void __launch_bounds__(SORT_THREADS) sort_hist(const unsigned long long* __restrict__ keys, uint32_t n,
+                                                          int shift, uint32_t* __restrict__ hist) {
+    __shared__ __align__(16) uint32_t h[SORT_RADIX];
+    for (uint32_t d = threadIdx.x; d < SORT_RADIX; d += SORT_THREADS) h[d] = 0;
+    __syncthreads();
+    const uint32_t base = blockIdx.x * SORT_TILE;
+#pragma unroll
+    for (int k = 0; k < SORT_ITEMS; k++) {
+        const uint32_t idx = base + k * SORT_THREADS + threadIdx.x;
+        if (idx < n) atomicAdd(&h[digit_of(keys[idx], shift)], 1u);
+    }
+    __syncthreads();
+    reinterpret_cast<uint4*>(hist + size_t(blockIdx.x) * SORT_RADIX)[threadIdx.x] = reinterpret_cast<uint4*>(h)[threadIdx.x];
+}
+
+// Many tiles: each digit's counts become running sums over the tiles, its
+// total goes to `totals`; one digit a thread.
+__global__ void __launch_bounds__(32) sort_tile_sums(uint32_t* __restrict__ hist, uint32_t ntiles, uint32_t* __restrict__ totals) {
+    const uint32_t d = blockIdx.x * 32u + threadIdx.x;
+    uint32_t run = 0;
+#pragma unroll 8
+    for (uint32_t t = 0; t < ntiles; t++) {
+        const uint32_t v = hist[size_t(t) * SORT_RADIX + d];
+        hist[size_t(t) * SORT_RADIX + d] = run;
+        run += v;
+    }
+    totals[d] = run;
+}
+
 // Stable scatter: each warp ranks its 256 consecutive keys of the tile in
 // order (lanes with equal digits via __match_any_sync), warps are ordered by
-// the per-digit counts of the warps before them.
-__global__ void __launch_bounds__(SORT_THREADS) sort_scatter(const unsigned long long* __restrict__ keys_in,
+// the per-digit counts of the warps before them, tiles by the counts of the
+// tiles before them.
+template <bool SUMMED>
+__global__ void __launch_bounds__(SORT_THREADS, 2) sort_scatter(const unsigned long long* __restrict__ keys_in,
                                                              const uint32_t* __restrict__ vals_in,
                                                              unsigned long long* __restrict__ keys_out,
                                                              uint32_t* __restrict__ vals_out, uint32_t n, int shift,
-                                                             uint32_t nblocks, const uint32_t* __restrict__ offs) {
-    __shared__ uint32_t cnt[SORT_WARPS][256];
+                                                             const uint32_t* __restrict__ hist, uint32_t ntiles,
+                                                             const uint32_t* __restrict__ totals) {
+    __shared__ uint16_t cnt[SORT_WARPS][SORT_RADIX];
+    __shared__ __align__(16) uint32_t offs[SORT_RADIX];
+    __shared__ uint32_t wsum[SORT_WARPS];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (uint32_t d = lane; d < 256; d += 32) cnt[warp][d] = 0;
+    for (uint32_t d = lane; d < SORT_RADIX; d += 32) cnt[warp][d] = 0;
     __syncwarp();
     const uint32_t base = blockIdx.x * SORT_TILE + warp * (SORT_ITEMS * 32);
     unsigned long long k_[SORT_ITEMS];
     uint32_t v_[SORT_ITEMS], rank[SORT_ITEMS], dg[SORT_ITEMS];
     const uint32_t lt = (1u << lane) - 1u;
+    // this thread's four digits: keys before this tile, keys in all
+    {
+        const uint4* rows = reinterpret_cast<const uint4*>(hist) + threadIdx.x;
+        uint4 pre = make_uint4(0, 0, 0, 0), tot = pre;
+        if (SUMMED) {
+            pre = rows[size_t(blockIdx.x) * (SORT_RADIX / 4)];
+            tot = reinterpret_cast<const uint4*>(totals)[threadIdx.x];
+        } else {
+            // 16 rows in flight
+            for (uint32_t t0 = 0; t0 < ntiles; t0 += 16) {
+                uint4 v[16];
+#pragma unroll
+                for (uint32_t k = 0; k < 16; k++)
+                    v[k] = t0 + k < ntiles ? rows[size_t(t0 + k) * (SORT_RADIX / 4)] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+                for (uint32_t k = 0; k < 16; k++) {
+                    const uint32_t m = t0 + k < blockIdx.x ? 0xffffffffu : 0u;
+                    tot.x += v[k].x; tot.y += v[k].y; tot.z += v[k].z; tot.w += v[k].w;
+                    pre.x += v[k].x & m; pre.y += v[k].y & m; pre.z += v[k].z & m; pre.w += v[k].w & m;
+                }
+            }
+        }
+        const uint32_t sum = tot.x + tot.y + tot.z + tot.w;
+        uint32_t inc = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= uint32_t(o)) inc += x;
+        }
+        if (lane == 31) wsum[warp] = inc;
+        __syncthreads();
+        uint32_t run = inc - sum;
+        for (uint32_t w = 0; w < warp; w++) run += wsum[w];
+        uint4 o;
+        o.x = run + pre.x; run += tot.x;
+        o.y = run + pre.y; run += tot.y;
+        o.z = run + pre.z; run += tot.z;
+        o.w = run + pre.w;
+        reinterpret_cast<uint4*>(offs)[threadIdx.x] = o;
+    }
+#pragma unroll
     for (int r = 0; r < SORT_ITEMS; r++) {
         const uint32_t idx = base + r * 32 + lane;
-        const bool valid = idx < n;
-        k_[r] = valid ? keys_in[idx] : 0ull;
-        v_[r] = valid ? vals_in[idx] : 0u;
-        const uint32_t d = valid ? digit_of(k_[r], shift) : 256u;
+        k_[r] = idx < n ? keys_in[idx] : 0ull;
+        v_[r] = idx < n ? vals_in[idx] : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < SORT_ITEMS; r++) {
+        const bool valid = base + r * 32 + lane < n;
+        const uint32_t d = valid ? digit_of(k_[r], shift) : SORT_RADIX;
         dg[r] = d;
         const uint32_t peers = __match_any_sync(0xffffffffu, d);
         const uint32_t before = valid ? cnt[warp][d] : 0u;
         rank[r] = before + __popc(peers & lt);
         __syncwarp();
-        if (valid && (peers & lt) == 0) cnt[warp][d] = before + __popc(peers);
+        if (valid && (peers & lt) == 0) cnt[warp][d] = uint16_t(before + __popc(peers));
         __syncwarp();
     }
     __syncthreads();
     // per digit: counts of the earlier warps of this block
-    __shared__ uint32_t woff[SORT_WARPS][256];
-    {
-        const uint32_t d = threadIdx.x;  // 256 threads, one digit each
+    for (uint32_t d = threadIdx.x; d < SORT_RADIX; d += SORT_THREADS) {
         uint32_t run = 0;
         for (int w = 0; w < SORT_WARPS; w++) {
-            woff[w][d] = run;
-            run += cnt[w][d];
+            const uint32_t c = cnt[w][d];
+            cnt[w][d] = uint16_t(run);
+            run += c;
         }
     }
     __syncthreads();
+#pragma unroll
     for (int r = 0; r < SORT_ITEMS; r++) {
         const uint32_t d = dg[r];
-        if (d < 256u) {
-            const uint32_t pos = offs[d * nblocks + blockIdx.x] + woff[warp][d] + rank[r];
+        if (d < SORT_RADIX) {
+            const uint32_t pos = offs[d] + cnt[warp][d] + rank[r];
             keys_out[pos] = k_[r];
             vals_out[pos] = v_[r];
         }
@@ -253,27 +328,29 @@ RD float3 aabb_centre(const float4 mn, const float4 mx) {
     return make_float3(0.5f * (mn.x + mx.x), 0.5f * (mn.y + mx.y), 0.5f * (mn.z + mx.z));
 }
 
-// Scene bounds of the centres (ordered-bit atomics: min in [0..2], max in [3..5]).
-__global__ void __launch_bounds__(128) lbvh_bounds(const BpArgs a, uint32_t* __restrict__ bounds) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t lo[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, hi[3] = {0u, 0u, 0u};
-    if (i < a.n) {
+// Scene bounds of the centres, as ordered bits: maxima in [3..5], minima
+// complemented in [0..2] (so that zero is the start of both).  A few blocks
+// with one atomic a value each: with one a warp, 100,000 centres queued 19,000
+// atomics on six words (15 us).
+constexpr uint32_t BOUNDS_BLOCKS = 148;
+__global__ void __launch_bounds__(256) lbvh_bounds(const BpArgs a, uint32_t* __restrict__ bounds) {
+    __shared__ uint32_t part[8][6];
+    uint32_t m[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
         const float3 c = aabb_centre(a.fat_min[i], a.fat_max[i]);
-        lo[0] = hi[0] = ordered_bits(c.x);
-        lo[1] = hi[1] = ordered_bits(c.y);
-        lo[2] = hi[2] = ordered_bits(c.z);
+        const uint32_t x = ordered_bits(c.x), y = ordered_bits(c.y), z = ordered_bits(c.z);
+        m[0] = max(m[0], ~x); m[1] = max(m[1], ~y); m[2] = max(m[2], ~z);
+        m[3] = max(m[3], x); m[4] = max(m[4], y); m[5] = max(m[5], z);
     }
-    for (int k = 0; k < 3; k++) {
-        for (int o = 16; o; o >>= 1) {
-            lo[k] = min(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
-            hi[k] = max(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
-        }
+    for (int k = 0; k < 6; k++) {
+        m[k] = __reduce_max_sync(0xffffffffu, m[k]);
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][k] = m[k];
     }
-    if ((threadIdx.x & 31) == 0) {
-        for (int k = 0; k < 3; k++) {
-            atomicMin(bounds + k, lo[k]);
-            atomicMax(bounds + 3 + k, hi[k]);
-        }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        uint32_t v = 0;
+        for (int w = 0; w < 8; w++) v = max(v, part[w][threadIdx.x]);
+        atomicMax(bounds + threadIdx.x, v);
     }
 }
 
@@ -299,7 +376,7 @@ __global__ void __launch_bounds__(128) lbvh_keys(const BpArgs a, const uint32_t*
     if (i >= a.n) return;
     float lo[3], inv[3];
     for (int k = 0; k < 3; k++) {
-        lo[k] = from_ordered_bits(bounds[k]);
+        lo[k] = from_ordered_bits(~bounds[k]);
         const float ext = from_ordered_bits(bounds[3 + k]) - lo[k];
         inv[k] = ext > 0.0f ? 1023.0f / ext : 0.0f;
     }
@@ -315,76 +392,63 @@ __global__ void __launch_bounds__(128) lbvh_keys(const BpArgs a, const uint32_t*
     a.vals[i] = i;
 }
 
-// Common-prefix length of sorted keys i and j (Karras 2012), with the sorted
-// position breaking ties; -1 outside [0, n).
-RD int lbvh_delta(const unsigned long long* __restrict__ k, int64_t n, int64_t i, int64_t j) {
-    if (j < 0 || j >= n) return -1;
-    const unsigned long long ki = k[i], kj = k[j];
-    if (ki == kj) return 64 + __clz(uint32_t(i) ^ uint32_t(j));
-    return __clzll(ki ^ kj);
-}
-
-// Internal node i of the n - 1: its sorted range and its two children
-// (internal index, or n - 1 + sorted position for a leaf); node 0 is the root.
-__global__ void __launch_bounds__(128) lbvh_build(const unsigned long long* __restrict__ keys, uint32_t n,
-                                                  int2* __restrict__ child, int2* __restrict__ range,
-                                                  int32_t* __restrict__ parent) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t N = n;
-    if (i >= N - 1) return;
-    const int d = (lbvh_delta(keys, N, i, i + 1) - lbvh_delta(keys, N, i, i - 1)) >= 0 ? 1 : -1;
-    const int dmin = lbvh_delta(keys, N, i, i - d);
-    int64_t lmax = 2;
-    while (lbvh_delta(keys, N, i, i + lmax * d) > dmin) lmax <<= 1;
-    int64_t l = 0;
-    for (int64_t t = lmax >> 1; t >= 1; t >>= 1)
-        if (lbvh_delta(keys, N, i, i + (l + t) * d) > dmin) l += t;
-    const int64_t j = i + l * d;
-    const int dnode = lbvh_delta(keys, N, i, j);
-    int64_t s = 0, t = l;
-    for (;;) {
-        t = (t + 1) >> 1;
-        if (lbvh_delta(keys, N, i, i + (s + t) * d) > dnode) s += t;
-        if (t <= 1) break;
-    }
-    const int64_t gamma = i + s * d + (d < 0 ? -1 : 0);
-    const int64_t first = i < j ? i : j, last = i < j ? j : i;
-    const int32_t left = int32_t(first == gamma ? (N - 1) + gamma : gamma);
-    const int32_t right = int32_t(last == gamma + 1 ? (N - 1) + gamma + 1 : gamma + 1);
-    child[i] = make_int2(left, right);
-    range[i] = make_int2(int32_t(first), int32_t(last));
-    parent[left] = int32_t(i);
-    parent[right] = int32_t(i);
-    if (i == 0) parent[0] = -1;
-}
-
-// Bottom-up refit: a leaf's thread walks up; at each node the first arriving
-// child stops and the second computes the node's box (its sibling's box is
-// visible: written before the fence that precedes the counter increment).
-__global__ void __launch_bounds__(128) lbvh_refit(const float4* __restrict__ s_lo, const float4* __restrict__ s_hi,
-                                                  uint32_t n, const int2* __restrict__ child,
-                                                  const int32_t* __restrict__ parent, uint32_t* __restrict__ visits,
-                                                  float4* __restrict__ nlo, float4* __restrict__ nhi) {
+// The radix tree over the sorted keys, bottom-up in one pass (after Apetrei,
+// "Fast and Simple Agglomerative LBVH Construction", 2014): a leaf's thread
+// walks up, and joins the range it covers, [l, r], with the neighbour it
+// shares the longer prefix with.  Internal node s lies between the sorted
+// positions s and s + 1.  A child leaves its box, its id (leaf at sorted
+// position p: n - 1 + p) and its last position in its half of the parent's
+// record; the first to arrive stops, the second goes on with both (the other
+// half was written before the fence that precedes the counter's increment).
+// Equal prefixes of equal keys are told apart by the positions.
+__global__ void __launch_bounds__(128) lbvh_build(const unsigned long long* __restrict__ keys, const float4* __restrict__ s_lo,
+                                                  const float4* __restrict__ s_hi, uint32_t n, LbvhNode* __restrict__ nodes,
+                                                  uint32_t* __restrict__ first, uint32_t* __restrict__ visits,
+                                                  uint32_t* __restrict__ root) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n || n < 2) return;
-    const int32_t nl = int32_t(n) - 1;
-    int32_t x = parent[nl + int32_t(p)];
-    while (x >= 0) {
+    uint32_t l = p, r = p;
+    int32_t id = int32_t(n) - 1 + int32_t(p);
+    float4 lo = s_lo[p], hi = s_hi[p];
+    unsigned long long kl = keys[p], kr = kl;
+    while (l != 0 || r != n - 1) {
+        bool right;   // join the neighbour on the right
+        if (l == 0) right = true;
+        else if (r == n - 1) right = false;
+        else {
+            const unsigned long long xr = kr ^ keys[r + 1], xl = keys[l - 1] ^ kl;
+            right = xr != xl ? xr < xl : (r ^ (r + 1)) < ((l - 1) ^ l);
+        }
+        const uint32_t parent = right ? r : l - 1;
+        LbvhNode* nd = nodes + parent;
+        lo.w = __int_as_float(id);
+        hi.w = __int_as_float(int32_t(r));
+        __stcg(right ? &nd->lo0 : &nd->lo1, lo);
+        __stcg(right ? &nd->hi0 : &nd->hi1, hi);
+        if (right) __stcg(first + parent, l);
         __threadfence();
-        if (atomicAdd(visits + x, 1u) == 0u) return;
-        const int2 c = child[x];
-        float4 lo0, hi0, lo1, hi1;
-        if (c.x >= nl) { lo0 = s_lo[c.x - nl]; hi0 = s_hi[c.x - nl]; }
-        else { lo0 = __ldcg(nlo + c.x); hi0 = __ldcg(nhi + c.x); }
-        if (c.y >= nl) { lo1 = s_lo[c.y - nl]; hi1 = s_hi[c.y - nl]; }
-        else { lo1 = __ldcg(nlo + c.y); hi1 = __ldcg(nhi + c.y); }
-        __stcg(nlo + x, make_float4(fminf(lo0.x, lo1.x), fminf(lo0.y, lo1.y), fminf(lo0.z, lo1.z), 0.0f));
-        __stcg(nhi + x, make_float4(fmaxf(hi0.x, hi1.x), fmaxf(hi0.y, hi1.y), fmaxf(hi0.z, hi1.z), 0.0f));
-        x = parent[x];
+        if (atomicAdd(visits + parent, 1u) == 0u) return;
+        __threadfence();
+        const float4 olo = __ldcg(right ? &nd->lo1 : &nd->lo0), ohi = __ldcg(right ? &nd->hi1 : &nd->hi0);
+        if (right) {
+            r = uint32_t(__float_as_int(ohi.w));
+            kr = keys[r];
+        } else {
+            l = __ldcg(first + parent);
+            kl = keys[l];
+        }
+        lo = make_float4(fminf(lo.x, olo.x), fminf(lo.y, olo.y), fminf(lo.z, olo.z), 0.0f);
+        hi = make_float4(fmaxf(hi.x, ohi.x), fmaxf(hi.y, ohi.y), fmaxf(hi.z, ohi.z), 0.0f);
+        id = int32_t(parent);
     }
+    *root = uint32_t(id);
 }
 
 constexpr int LBVH_STACK = 128;   // > the deepest tree 96-bit keys can give
+constexpr uint32_t LBVH_BLOCK = 128;
+// Up to this many blocks the writing kernel's blocks add up the totals before
+// theirs; above it they are scanned first.
+constexpr uint32_t LBVH_SUM_BLOCKS = 2048;
 
 // AABB::testCollision (AABB.h:179-187): inclusive on every axis
 RD bool aabb_overlap(const float4 alo, const float4 ahi, const float4 blo, const float4 bhi) {
@@ -394,75 +458,154 @@ RD bool aabb_overlap(const float4 alo, const float4 ahi, const float4 blo, const
     return true;
 }
 
-template <bool WRITE>
-__global__ void __launch_bounds__(128) lbvh_query(const BpArgs a, const int2* __restrict__ child,
-                                                  const int2* __restrict__ range, const float4* __restrict__ nlo,
-                                                  const float4* __restrict__ nhi) {
-    __shared__ int32_t stack[4][LBVH_STACK];
+// The partners of the collider at sorted position p that lie behind it, in
+// ascending position: the walk takes left children first, and both children
+// of a node are tested from its one record.  With groups only positions up to
+// the group's end are looked at.
+template <class Found>
+RD void lbvh_walk(const BpArgs& a, uint32_t p, uint32_t root, Found found) {
     const uint32_t n = a.n;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (blockIdx.x * blockDim.x + warp * 32u >= n) return;   // whole warp past the end
-    const bool active = p < n;
     const int32_t nl = int32_t(n) - 1;
-    float4 qlo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), qhi = qlo;
-    int32_t g = 0;
-    if (active) { qlo = a.s_lo[p]; qhi = a.s_hi[p]; g = a.s_group[p]; }
+    const float4 qlo = a.s_lo[p], qhi = a.s_hi[p];
     const int32_t body = __float_as_int(qlo.w);
     const uint32_t bits = __float_as_uint(qhi.w);
     const uint32_t cat = bits >> 16, msk = bits & 0xffffu;
-    uint32_t count = 0;
-    uint32_t out = (WRITE && active) ? a.pair_offset[p] : 0u;
-    const uint32_t ci = active ? a.vals[p] : 0u;
-    int32_t* st = stack[warp];
+    int32_t g = 0;
+    uint32_t end = n - 1;   // last position of the group
+    if (a.group) {
+        g = a.s_group[p];
+        uint32_t lo = p, hi = n - 1;
+        while (lo < hi) {
+            const uint32_t m = lo + (hi - lo + 1) / 2;
+            if (a.s_group[m] > g) hi = m - 1;
+            else lo = m;
+        }
+        end = lo;
+    }
+    auto leaf = [&](uint32_t j) {
+        const int32_t body2 = __float_as_int(a.s_lo[j].w);
+        const uint32_t bits2 = __float_as_uint(a.s_hi[j].w);
+        if (body2 != body && (msk & (bits2 >> 16)) != 0u && (cat & (bits2 & 0xffffu)) != 0u && (!a.group || a.s_group[j] == g))
+            found(j);
+    };
+    int32_t stack[LBVH_STACK];
     int sp = 0;
-    if (n >= 2) { if (lane == 0) st[0] = 0; sp = 1; }
-    __syncwarp();
-    while (sp > 0) {
-        const int32_t node = st[--sp];
-        __syncwarp();
-        if (node >= nl) {
-            // a leaf: sorted position j
-            const int32_t j = node - nl;
-            bool hit = active && j > int32_t(p);
-            if (hit) {
-                const float4 lo2 = a.s_lo[j], hi2 = a.s_hi[j];
-                const uint32_t bits2 = __float_as_uint(hi2.w);
-                hit = a.s_group[j] == g && aabb_overlap(qlo, qhi, lo2, hi2) && __float_as_int(lo2.w) != body &&
-                      (msk & (bits2 >> 16)) != 0u && (cat & (bits2 & 0xffffu)) != 0u;
+    int32_t node = int32_t(root);
+    for (;;) {
+        if (node < 0) {
+            if (sp == 0) break;
+            node = stack[--sp];
+            if (node >= nl) {
+                leaf(uint32_t(node - nl));
+                node = -1;
+                continue;
             }
-            if (hit) {
-                if (WRITE) {
-                    if (out < a.capacity) {
-                        const uint32_t cj = a.vals[j];
-                        a.pairs[2 * out] = int32_t(ci < cj ? ci : cj);
-                        a.pairs[2 * out + 1] = int32_t(ci < cj ? cj : ci);
-                    }
-                    out++;
-                } else {
-                    count++;
+        }
+        const LbvhNode* nd = a.lbvh_nodes + node;
+        const float4 lo0 = nd->lo0, hi0 = nd->hi0, lo1 = nd->lo1, hi1 = nd->hi1;
+        const int32_t c0 = __float_as_int(lo0.w), last0 = __float_as_int(hi0.w), c1 = __float_as_int(lo1.w);
+        const int32_t last1 = __float_as_int(hi1.w);
+        const bool hit0 = last0 > int32_t(p) && aabb_overlap(qlo, qhi, lo0, hi0);
+        const bool hit1 = last1 > int32_t(p) && uint32_t(last0) < end && aabb_overlap(qlo, qhi, lo1, hi1);
+        node = -1;
+        if (hit0 && c0 >= nl) leaf(uint32_t(c0 - nl));
+        if (hit0 && c0 < nl) {
+            node = c0;
+            if (hit1) {
+                if (sp == LBVH_STACK) {
+                    atomicOr(a.error, 16u);   // cannot happen for trees of 96-bit keys
+                    break;
                 }
+                stack[sp++] = c1;
             }
-            continue;
-        }
-        const int2 r = range[node];
-        bool hit = active && r.y > int32_t(p);
-        if (hit) {
-            // the node's sorted range holds groups s_group[r.x] .. s_group[r.y]
-            hit = g >= a.s_group[r.x] && g <= a.s_group[r.y] && aabb_overlap(qlo, qhi, nlo[node], nhi[node]);
-        }
-        if (__any_sync(0xffffffffu, hit)) {
-            if (sp + 2 > LBVH_STACK) {
-                if (lane == 0) atomicOr(a.error, 16u);   // cannot happen for trees of 96-bit keys
-                break;
-            }
-            const int2 c = child[node];
-            if (lane == 0) { st[sp] = c.y; st[sp + 1] = c.x; }
-            sp += 2;
-            __syncwarp();
+        } else if (hit1) {
+            if (c1 >= nl) leaf(uint32_t(c1 - nl));
+            else node = c1;
         }
     }
-    if (!WRITE && active) a.pair_offset[p] = count;
+}
+
+// Bound: the latency of the dependent node reads.  100,000 colliders: 44 us,
+// plus 9 to write the pairs (a count and a write walk of 32-lane packets took
+// 138 + 137 us, the whole search 560 us; 174 now).
+//
+// Search: a collider's partners, the first LBVH_KEEP of them to `found`
+// (entry k of position p at k * n + p), their number to pair_offset[p], each
+// block's total to block_pairs.
+__global__ void __launch_bounds__(LBVH_BLOCK) lbvh_search(const BpArgs a) {
+    const uint32_t p = blockIdx.x * LBVH_BLOCK + threadIdx.x;
+    uint32_t count = 0;
+    if (p < a.n) {
+        if (a.n >= 2)
+            lbvh_walk(a, p, *a.lbvh_root, [&](uint32_t j) {
+                if (count < LBVH_KEEP) a.lbvh_found[size_t(count) * a.n + p] = j;
+                count++;
+            });
+        a.pair_offset[p] = count;
+    }
+    __shared__ uint32_t part[LBVH_BLOCK / 32];
+    const uint32_t sum = __reduce_add_sync(0xffffffffu, count);
+    if ((threadIdx.x & 31u) == 0) part[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t t = 0;
+        for (uint32_t w = 0; w < LBVH_BLOCK / 32; w++) t += part[w];
+        a.block_pairs[blockIdx.x] = t;
+    }
+}
+
+// The pairs in order of sorted position: every block adds up the totals of
+// the blocks before it (SCANNED: they are running sums already), scans its
+// own counts and writes its pairs; a collider with more than LBVH_KEEP
+// partners walks again for the rest.
+template <bool SCANNED>
+__global__ void __launch_bounds__(LBVH_BLOCK) lbvh_emit(const BpArgs a) {
+    __shared__ uint32_t part[LBVH_BLOCK / 32], s_base;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t p = blockIdx.x * LBVH_BLOCK + threadIdx.x;
+    if (SCANNED) {
+        if (threadIdx.x == 0) s_base = a.block_pairs[blockIdx.x];
+    } else {
+        uint32_t before = 0;
+        for (uint32_t b = threadIdx.x; b < blockIdx.x; b += LBVH_BLOCK) before += a.block_pairs[b];
+        before = __reduce_add_sync(0xffffffffu, before);
+        if (lane == 0) part[warp] = before;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t t = 0;
+            for (uint32_t w = 0; w < LBVH_BLOCK / 32; w++) t += part[w];
+            s_base = t;
+        }
+        __syncthreads();
+    }
+    const uint32_t count = p < a.n ? a.pair_offset[p] : 0u;
+    uint32_t inc = count;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= uint32_t(o)) inc += x;
+    }
+    if (lane == 31) part[warp] = inc;
+    __syncthreads();
+    uint32_t out = s_base + inc - count;
+    for (uint32_t w = 0; w < warp; w++) out += part[w];
+    if (!SCANNED && blockIdx.x == gridDim.x - 1 && threadIdx.x == LBVH_BLOCK - 1) *a.pair_count = out + count;
+    if (count == 0) return;
+    const uint32_t ci = a.vals[p];
+    auto put = [&](uint32_t j) {
+        if (out < a.capacity) {
+            const uint32_t cj = a.vals[j];
+            a.pairs[2 * size_t(out)] = int32_t(ci < cj ? ci : cj);
+            a.pairs[2 * size_t(out) + 1] = int32_t(ci < cj ? cj : ci);
+        }
+        out++;
+    };
+    for (uint32_t k = 0; k < count && k < LBVH_KEEP; k++) put(a.lbvh_found[size_t(k) * a.n + p]);
+    if (count > LBVH_KEEP) {
+        uint32_t k = 0;
+        lbvh_walk(a, p, *a.lbvh_root, [&](uint32_t j) {
+            if (k++ >= LBVH_KEEP) put(j);
+        });
+    }
 }
 
 }  // namespace
@@ -474,7 +617,8 @@ cudaError_t launch_bp_update(const BpArgs& a, cudaStream_t s, uint64_t* launches
     return cudaGetLastError();
 }
 
-size_t sort_scratch_words(uint32_t n) { return size_t(256) * ((n + SORT_TILE - 1) / SORT_TILE) + 1; }
+size_t sort_scratch_words(uint32_t n) { return size_t(SORT_RADIX) * ((n + SORT_TILE - 1) / SORT_TILE + 1); }
+size_t lbvh_block_words(uint32_t n) { return (n + LBVH_BLOCK - 1) / LBVH_BLOCK; }
 
 cudaError_t launch_exclusive_scan(uint32_t* v, uint32_t n, uint32_t* total, cudaStream_t s) {
     if (n == 0) return total ? cudaMemsetAsync(total, 0, sizeof(uint32_t), s) : cudaSuccess;
@@ -486,11 +630,11 @@ cudaError_t launch_bp_pairs(const BpArgs& a, int axis, cudaStream_t s, uint64_t*
     if (a.n == 0) return cudaMemsetAsync(a.pair_count, 0, sizeof(uint32_t), s);
     const bool lbvh = axis < 0;
     if (lbvh) {
-        cudaError_t e = cudaMemsetAsync(a.lbvh_bounds, 0xff, 3 * sizeof(uint32_t), s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(a.lbvh_bounds + 3, 0, 3 * sizeof(uint32_t), s);
-        if (e == cudaSuccess && a.n > 1) e = cudaMemsetAsync(a.lbvh_visits, 0, size_t(a.n) * sizeof(uint32_t), s);
+        // centre bounds, then the visit counters
+        const cudaError_t e = cudaMemsetAsync(a.lbvh_bounds, 0, (8 + size_t(a.n)) * sizeof(uint32_t), s);
         if (e != cudaSuccess) return e;
-        lbvh_bounds<<<blocks128(a.n), 128, 0, s>>>(a, a.lbvh_bounds);
+        const uint32_t nb = (a.n + 255) / 256;
+        lbvh_bounds<<<nb < BOUNDS_BLOCKS ? nb : BOUNDS_BLOCKS, 256, 0, s>>>(a, a.lbvh_bounds);
         lbvh_keys<<<blocks128(a.n), 128, 0, s>>>(a, a.lbvh_bounds);
         *launches += 2;
     } else {
@@ -499,15 +643,21 @@ cudaError_t launch_bp_pairs(const BpArgs& a, int axis, cudaStream_t s, uint64_t*
     }
     // radix sort: (group, Morton code) = 30 + group bits, or (group, min) =
     // 32 float bits + the group bits in use
-    const uint32_t nblocks = (a.n + SORT_TILE - 1) / SORT_TILE;
+    const uint32_t ntiles = (a.n + SORT_TILE - 1) / SORT_TILE;
+    uint32_t* totals = a.sort_hist + size_t(ntiles) * SORT_RADIX;
     unsigned long long *kin = a.keys, *kout = a.keys_tmp;
     uint32_t *vin = a.vals, *vout = a.vals_tmp;
     const int end_bit = (lbvh ? 30 : 32) + a.group_bits;
-    for (int shift = 0; shift < end_bit; shift += 8) {
-        sort_hist<<<nblocks, SORT_THREADS, 0, s>>>(kin, a.n, shift, nblocks, a.sort_hist);
-        scan_small<<<1, 1024, 0, s>>>(a.sort_hist, 256 * nblocks, nullptr);
-        sort_scatter<<<nblocks, SORT_THREADS, 0, s>>>(kin, vin, kout, vout, a.n, shift, nblocks, a.sort_hist);
-        *launches += 3;
+    for (int shift = 0; shift < end_bit; shift += SORT_BITS) {
+        sort_hist<<<ntiles, SORT_THREADS, 0, s>>>(kin, a.n, shift, a.sort_hist);
+        if (ntiles > SORT_SUM_TILES) {
+            sort_tile_sums<<<SORT_RADIX / 32, 32, 0, s>>>(a.sort_hist, ntiles, totals);
+            sort_scatter<true><<<ntiles, SORT_THREADS, 0, s>>>(kin, vin, kout, vout, a.n, shift, a.sort_hist, ntiles, totals);
+            (*launches)++;
+        } else {
+            sort_scatter<false><<<ntiles, SORT_THREADS, 0, s>>>(kin, vin, kout, vout, a.n, shift, a.sort_hist, ntiles, nullptr);
+        }
+        *launches += 2;
         unsigned long long* tk = kin; kin = kout; kout = tk;
         uint32_t* tv = vin; vin = vout; vout = tv;
     }
@@ -518,15 +668,20 @@ cudaError_t launch_bp_pairs(const BpArgs& a, int axis, cudaStream_t s, uint64_t*
     *launches += 1;
     if (lbvh) {
         if (a.n > 1) {
-            lbvh_build<<<blocks128(a.n - 1), 128, 0, s>>>(kin, a.n, a.lbvh_child, a.lbvh_range, a.lbvh_parent);
-            lbvh_refit<<<blocks128(a.n), 128, 0, s>>>(b.s_lo, b.s_hi, a.n, a.lbvh_child, a.lbvh_parent, a.lbvh_visits,
-                                                      a.lbvh_nlo, a.lbvh_nhi);
-            *launches += 2;
+            lbvh_build<<<blocks128(a.n), 128, 0, s>>>(kin, b.s_lo, b.s_hi, a.n, a.lbvh_nodes, a.lbvh_first, a.lbvh_visits,
+                                                      a.lbvh_root);
+            (*launches)++;
         }
-        lbvh_query<false><<<blocks128(a.n), 128, 0, s>>>(b, a.lbvh_child, a.lbvh_range, a.lbvh_nlo, a.lbvh_nhi);
-        scan_small<<<1, 1024, 0, s>>>(b.pair_offset, a.n, a.pair_count);
-        lbvh_query<true><<<blocks128(a.n), 128, 0, s>>>(b, a.lbvh_child, a.lbvh_range, a.lbvh_nlo, a.lbvh_nhi);
-        *launches += 3;
+        const uint32_t nb = uint32_t(lbvh_block_words(a.n));
+        lbvh_search<<<nb, LBVH_BLOCK, 0, s>>>(b);
+        if (nb > LBVH_SUM_BLOCKS) {
+            scan_small<<<1, 1024, 0, s>>>(b.block_pairs, nb, a.pair_count);
+            lbvh_emit<true><<<nb, LBVH_BLOCK, 0, s>>>(b);
+            (*launches)++;
+        } else {
+            lbvh_emit<false><<<nb, LBVH_BLOCK, 0, s>>>(b);
+        }
+        *launches += 2;
         return cudaGetLastError();
     }
     sap_sweep<false><<<blocks128(a.n), 128, 0, s>>>(b);

@@ -8,6 +8,16 @@
 
 namespace rp3dg {
 
+// An internal node of the pair search's tree: its children's boxes with, in the
+// w components, each child's id (lo) and last sorted position (hi).
+struct __align__(64) LbvhNode {
+    float4 lo0, hi0, lo1, hi1;
+};
+// Partners per collider that the search keeps for the writing kernel (a second
+// walk for the rest costs its warp a whole walk's latency: with 8 the writing
+// kernel of a 100,000-collider lattice took 36 us, with 16 it takes 9).
+constexpr uint32_t LBVH_KEEP = 16;
+
 struct BpArgs {
     uint32_t n;           // colliders in the broad phase
     uint32_t n_update;    // colliders [0, n_update) get new AABBs
@@ -35,14 +45,17 @@ struct BpArgs {
     int32_t* pairs;
     uint32_t capacity;
     uint32_t* pair_count;
-    // LBVH (sweep axis < 0): centre bounds (6 words), per internal node its
-    // children, sorted range, box and visit counter, per node its parent
+    // LBVH (sweep axis < 0): centre bounds (6 words), the root's index (word
+    // 7 of the same 8), then the nodes' visit counters (n words); per internal
+    // node its record and the first sorted position it covers; per collider
+    // its first LBVH_KEEP partners; per block of colliders its pairs
     uint32_t* lbvh_bounds;
-    int2* lbvh_child;
-    int2* lbvh_range;
-    int32_t* lbvh_parent;     // 2n - 1 entries
+    uint32_t* lbvh_root;
     uint32_t* lbvh_visits;
-    float4 *lbvh_nlo, *lbvh_nhi;
+    LbvhNode* lbvh_nodes;
+    uint32_t* lbvh_first;
+    uint32_t* lbvh_found;
+    uint32_t* block_pairs;
 };
 
 cudaError_t launch_bp_update(const BpArgs& a, cudaStream_t s, uint64_t* launches);
@@ -50,6 +63,8 @@ cudaError_t launch_bp_update(const BpArgs& a, cudaStream_t s, uint64_t* launches
 cudaError_t launch_bp_pairs(const BpArgs& a, int axis, cudaStream_t s, uint64_t* launches);
 // uint32 words of sort histogram scratch for n keys
 size_t sort_scratch_words(uint32_t n);
+// words of the pair search's block totals for n colliders
+size_t lbvh_block_words(uint32_t n);
 // Exclusive scan of n words in place (one CTA); *total (device, or null) gets the sum.
 cudaError_t launch_exclusive_scan(uint32_t* v, uint32_t n, uint32_t* total, cudaStream_t s);
 

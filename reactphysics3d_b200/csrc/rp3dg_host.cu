@@ -2158,13 +2158,11 @@ int rp3dg_broadphase_pairs_device(rp3dg_ctx* ctx, const rp3dg_broadphase* bp, in
     const size_t o_grp = off; off += al(n * 4);
     const size_t o_poff = off; off += al(n * 4 + 4);
     const bool lbvh = axis == RP3DG_BROADPHASE_LBVH;
-    const size_t o_lb = off; off += lbvh ? al(8 * 4) : 0;
-    const size_t o_lchild = off; off += lbvh ? al(n * 8) : 0;
-    const size_t o_lrange = off; off += lbvh ? al(n * 8) : 0;
-    const size_t o_lparent = off; off += lbvh ? al(2 * n * 4) : 0;
-    const size_t o_lvisit = off; off += lbvh ? al(n * 4) : 0;
-    const size_t o_lnlo = off; off += lbvh ? al(n * 16) : 0;
-    const size_t o_lnhi = off; off += lbvh ? al(n * 16) : 0;
+    const size_t o_lb = off; off += lbvh ? al((8 + n) * 4) : 0;
+    const size_t o_lnode = off; off += lbvh ? al(n * sizeof(rp3dg::LbvhNode)) : 0;
+    const size_t o_lfirst = off; off += lbvh ? al(n * 4) : 0;
+    const size_t o_lfound = off; off += lbvh ? al(n * rp3dg::LBVH_KEEP * 4) : 0;
+    const size_t o_lblock = off; off += lbvh ? al(rp3dg::lbvh_block_words(uint32_t(n)) * 4) : 0;
     cudaSetDevice(ctx->device);
     rc = grow(ctx, &ctx->d_bp, &ctx->cap_bp, off + 256, "cudaMalloc(broad-phase scratch)");
     if (rc) return rc;
@@ -2195,12 +2193,12 @@ int rp3dg_broadphase_pairs_device(rp3dg_ctx* ctx, const rp3dg_broadphase* bp, in
     a.error = ctx->d_error;
     if (lbvh) {
         a.lbvh_bounds = reinterpret_cast<uint32_t*>(s + o_lb);
-        a.lbvh_child = reinterpret_cast<int2*>(s + o_lchild);
-        a.lbvh_range = reinterpret_cast<int2*>(s + o_lrange);
-        a.lbvh_parent = reinterpret_cast<int32_t*>(s + o_lparent);
-        a.lbvh_visits = reinterpret_cast<uint32_t*>(s + o_lvisit);
-        a.lbvh_nlo = reinterpret_cast<float4*>(s + o_lnlo);
-        a.lbvh_nhi = reinterpret_cast<float4*>(s + o_lnhi);
+        a.lbvh_root = a.lbvh_bounds + 7;
+        a.lbvh_visits = a.lbvh_bounds + 8;
+        a.lbvh_nodes = reinterpret_cast<rp3dg::LbvhNode*>(s + o_lnode);
+        a.lbvh_first = reinterpret_cast<uint32_t*>(s + o_lfirst);
+        a.lbvh_found = reinterpret_cast<uint32_t*>(s + o_lfound);
+        a.block_pairs = reinterpret_cast<uint32_t*>(s + o_lblock);
     }
     cudaError_t e = rp3dg::launch_bp_pairs(a, axis, ctx->stream, &ctx->launches);
     return e == cudaSuccess ? 0 : cuda_fail(ctx, e, "broad-phase pairs");
