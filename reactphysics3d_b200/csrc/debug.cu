@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(128) debug_colliders(const DebugArgs a) {
             const MeshHdr* h = reinterpret_cast<const MeshHdr*>(a.mesh_words) + sh.mesh;
             const uint32_t* w = a.mesh_words;
             auto vtx = [&](uint32_t v) {
-                const uint32_t o = h->off_sverts + 3 * v;
+                const uint32_t o = h->off_sverts + 4 * v;
                 return V(__uint_as_float(w[o]), __uint_as_float(w[o + 1]), __uint_as_float(w[o + 2]));
             };
             uint32_t tri = J.tri;
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(128) debug_colliders(const DebugArgs a) {
                 if (normal) {
                     const float nfv = float(fc);
                     centroid = V(centroid.x / nfv, centroid.y / nfv, centroid.z / nfv);
-                    const uint32_t o = h->off_normals + 3 * f;
+                    const uint32_t o = h->off_normals + 4 * f;
                     const v3 fn = qrot(T.q, V(__uint_as_float(w[o]), __uint_as_float(w[o + 1]), __uint_as_float(w[o + 2])));
                     const v3 normalPoint = vadd(centroid, V(fn.x * 1.0f, fn.y * 1.0f, fn.z * 1.0f));
                     put_line(a.lines + line++, centroid, normalPoint, COLOR_SHAPE_NORMAL);

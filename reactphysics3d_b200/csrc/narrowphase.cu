@@ -12,9 +12,11 @@
 // Kernel tuning knobs (compile time): resident CTAs per SM requested from the
 // register allocator, for the closed-form/GJK kernels, the warp-per-pair
 // polyhedron kernels (one per shape combination, each with one SAT
-// instantiation: 5 CTAs of 96 registers without spills, 7% faster on the
-// hull-box batch than 4 CTAs) and the thread-per-pair polyhedron kernel
-// (box-box only: 103 registers at 4 CTAs; at 5 it spills and is slower).
+// instantiation; mesh-box: 5 CTAs of 96 registers without spills, 12% faster
+// on the hull-box batch than 4 CTAs; with a mesh as shape 2: 4 CTAs, at 5 it
+// spills and is 6% slower on hull-hull pairs) and the thread-per-pair
+// polyhedron kernel (box-box only: 104 registers at 4 CTAs; at 5 it spills
+// and is slower).
 #ifndef RP3DG_NP_MIN_BLOCKS
 #define RP3DG_NP_MIN_BLOCKS 4
 #endif
@@ -29,8 +31,11 @@ namespace rp3dg {
 
 // Internal kernel id: the per-thread half of the polyhedron schedule.
 constexpr int ALGO_POLY_PER_THREAD = 7;
+// Internal kernel ids of the warp-per-pair launches, plus the COMBO_*.
+constexpr int WARP_KERNEL = 8, WARP_KERNEL_STAGED = 12;
 constexpr int NP_MIN_BLOCKS = RP3DG_NP_MIN_BLOCKS;
 constexpr int NP_MIN_BLOCKS_POLY_WARP = RP3DG_NP_MIN_BLOCKS_POLY_WARP;
+constexpr int NP_MIN_BLOCKS_MESH_WARP = 4;
 constexpr int NP_MIN_BLOCKS_POLY_THREAD = RP3DG_NP_MIN_BLOCKS_POLY_THREAD;
 
 __constant__ BoxTables c_box_tables;
@@ -278,8 +283,12 @@ constexpr int COMBO_MESH_BOX = 1, COMBO_BOX_MESH = 2, COMBO_MESH_MESH = 3;
 // Convex polyhedron vs convex polyhedron, one warp per pair, for pairs of
 // shape combination COMBO.
 template <int COMBO>
+struct ComboScratch { typedef WarpScratchMesh type; };
+template <>
+struct ComboScratch<COMBO_MESH_BOX> { typedef WarpScratch type; };
+template <int COMBO>
 RD uint32_t process_pair_warp(const NpArgs& a, uint32_t i, int lane, const BoxTables* box, const uint32_t* mesh_words,
-                              WarpScratch& stage, uint32_t proposal) {
+                              typename ComboScratch<COMBO>::type& stage, uint32_t proposal) {
     const int32_t i1 = a.shape1[i], i2 = a.shape2[i];
     if (uint32_t(i1) >= a.nb_shapes || uint32_t(i2) >= a.nb_shapes) {
         if (lane == 0) {
@@ -344,7 +353,7 @@ struct MinBlocks<ALGO_POLY_PER_THREAD> { static constexpr int value = NP_MIN_BLO
 
 template <int ALGO>
 __global__ void __launch_bounds__(NP_BLOCK, MinBlocks<ALGO>::value) narrowphase_kernel(const NpArgs a) {
-    extern __shared__ uint32_t s_mesh[];
+    extern __shared__ __align__(16) uint32_t s_mesh[];
     __shared__ BoxTables s_box;
     constexpr bool uses_poly = ALGO >= RP3DG_ALGO_SPHERE_VS_CONVEX_POLYHEDRON;
     const uint32_t* mesh_words = a.mesh_words;
@@ -415,28 +424,36 @@ __global__ void __launch_bounds__(NP_BLOCK, MinBlocks<ALGO>::value) narrowphase_
 // The pairs with a convex mesh of one shape combination, listed by the
 // thread-per-pair launch: persistent warps take them one at a time (so the
 // launch ends within one pair's time of its average), faces over lanes
-// (ballot / arg-min), edge staging in shared memory, the Gauss-map pass and
-// the edge distances 32 at a time, warp-parallel clipping.
-template <int COMBO>
-__global__ void __launch_bounds__(NP_BLOCK, NP_MIN_BLOCKS_POLY_WARP) narrowphase_warp_kernel(const NpArgs a) {
-    extern __shared__ uint32_t s_mesh[];
+// (ballot / arg-min), the edge pairs that can pass the Gauss-map test from bit
+// masks (EdgePairs), their distances 32 at a time, warp-parallel clipping.
+// Bound by instruction issue and dependent latency.  149,796 hull-box pairs
+// 736 -> 414 us, 20,011 hull-hull pairs 1,145 -> 212 us against one Gauss-map
+// test per edge pair from staged edges.
+// STAGED: every CTA holds the mesh tables in its own shared memory (arenas up
+// to MESH_STAGE_MAX_BYTES).  A parameter and not a run-time choice of the
+// pointer, so that the compiler knows the address space: 265 -> 231 us for
+// 20,011 hull-hull pairs.
+template <int COMBO, bool STAGED>
+__global__ void __launch_bounds__(NP_BLOCK, COMBO == COMBO_MESH_BOX ? NP_MIN_BLOCKS_POLY_WARP : NP_MIN_BLOCKS_MESH_WARP)
+    narrowphase_warp_kernel(const NpArgs a) {
+    extern __shared__ __align__(16) uint32_t s_mesh[];
     __shared__ BoxTables s_box;
-    __shared__ WarpScratch s_stage[NP_BLOCK / 32];
+    typedef typename ComboScratch<COMBO>::type Scratch;
+    __shared__ __align__(16) Scratch s_stage[NP_BLOCK / 32];
     const uint32_t total = __ldcg(a.work + (COMBO - 1));
     if (total == 0) return;   // uniform: nothing of this combination in the batch
-    const uint32_t* mesh_words = a.mesh_words;
+    const uint32_t* mesh_words = STAGED ? s_mesh : a.mesh_words;
     {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(&c_box_tables);
         uint32_t* dst = reinterpret_cast<uint32_t*>(&s_box);
         for (uint32_t k = threadIdx.x; k < sizeof(BoxTables) / 4; k += blockDim.x) dst[k] = src[k];
-        if (a.stage_mesh) {
+        if constexpr (STAGED) {
             for (uint32_t k = threadIdx.x; k < a.mesh_nwords; k += blockDim.x) s_mesh[k] = __ldg(a.mesh_words + k);
-            mesh_words = s_mesh;
         }
         __syncthreads();
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    WarpScratch& ws = s_stage[warp];
+    Scratch& ws = s_stage[warp];
     const uint32_t* list = a.plist + size_t(COMBO - 1) * a.n;
     uint32_t tested = 0, confirmed = 0;
     for (;;) {
@@ -460,7 +477,7 @@ __global__ void __launch_bounds__(NP_BLOCK, NP_MIN_BLOCKS_POLY_WARP) narrowphase
 
 template <int ALGO>
 __global__ void __launch_bounds__(NP_BLOCK, NP_MIN_BLOCKS) narrowphase_tri_kernel(const NpArgs a) {
-    extern __shared__ uint32_t s_mesh[];
+    extern __shared__ __align__(16) uint32_t s_mesh[];
     __shared__ BoxTables s_box;
     const uint32_t* mesh_words = a.mesh_words;
     {
@@ -707,9 +724,12 @@ static const void* kernel_ptr(int algo) {
         case 3: return reinterpret_cast<const void*>(&narrowphase_kernel<3>);
         case 4: return reinterpret_cast<const void*>(&narrowphase_kernel<4>);
         case 5: return reinterpret_cast<const void*>(&narrowphase_kernel<5>);
-        case 8 + COMBO_MESH_BOX: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_MESH_BOX>);
-        case 8 + COMBO_BOX_MESH: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_BOX_MESH>);
-        case 8 + COMBO_MESH_MESH: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_MESH_MESH>);
+        case WARP_KERNEL + COMBO_MESH_BOX: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_MESH_BOX, false>);
+        case WARP_KERNEL + COMBO_BOX_MESH: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_BOX_MESH, false>);
+        case WARP_KERNEL + COMBO_MESH_MESH: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_MESH_MESH, false>);
+        case WARP_KERNEL_STAGED + COMBO_MESH_BOX: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_MESH_BOX, true>);
+        case WARP_KERNEL_STAGED + COMBO_BOX_MESH: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_BOX_MESH, true>);
+        case WARP_KERNEL_STAGED + COMBO_MESH_MESH: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_MESH_MESH, true>);
         case ALGO_POLY_PER_THREAD: return reinterpret_cast<const void*>(&narrowphase_kernel<ALGO_POLY_PER_THREAD>);
     }
     return nullptr;
@@ -718,7 +738,7 @@ static const void* kernel_ptr(int algo) {
 #ifdef RP3DG_PROFILE_PHASES
 // Profiling builds only: per-phase cycles (summed over warps) and counts of the
 // warp-cooperative SAT; phases 0 = setup + temporal coherence, 1 = faces of
-// polyhedron 1, 2 = faces of polyhedron 2, 3 = edge staging, 4 = edge pairs,
+// polyhedron 1, 2 = faces of polyhedron 2, 3 = edge masks, 4 = edge pairs,
 // 5 = contact generation.  clear != 0 zeroes the counters after reading.
 extern "C" int rp3dg_profile_phases(unsigned long long* cycles, unsigned long long* counts, int clear) {
     cudaMemcpyFromSymbol(cycles, g_phase_cycles, sizeof(unsigned long long) * 8);
@@ -747,7 +767,7 @@ cudaError_t launch_narrowphase(int algo, const NpArgs& args, int num_sms, cudaSt
         if (e != cudaSuccess) return e;
         ++*launches;
         for (int c = COMBO_MESH_BOX; c <= COMBO_MESH_MESH; c++) {
-            e = launch_one(8 + c, args, num_sms, stream);
+            e = launch_one((args.stage_mesh ? WARP_KERNEL_STAGED : WARP_KERNEL) + c, args, num_sms, stream);
             if (e != cudaSuccess) return e;
             ++*launches;
         }
@@ -770,7 +790,7 @@ struct LaunchCache {
 static cudaError_t launch_one(int algo, const NpArgs& args, int num_sms, cudaStream_t stream) {
     const void* k = kernel_ptr(algo);
     if (!k) return cudaErrorInvalidValue;
-    const bool warp_list = algo > 8;   // narrowphase_warp_kernel<algo - 8>
+    const bool warp_list = algo > WARP_KERNEL;
     size_t smem = (args.stage_mesh && algo != ALGO_POLY_PER_THREAD) ? size_t(args.mesh_nwords) * 4 : 0;
     static thread_local LaunchCache cache[16];
     LaunchCache& lc = cache[algo & 15];

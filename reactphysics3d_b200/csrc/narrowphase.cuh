@@ -92,21 +92,24 @@ struct MeshPoly {
     const MeshHdr* h;
     const uint32_t* w;
     RD float margin() const { return 0.0f; }
-    RD float f(uint32_t off) const { return __uint_as_float(w[off]); }
+    RD v3 row(uint32_t off, uint32_t i) const {
+        const float4 r = *reinterpret_cast<const float4*>(w + off + 4 * i);
+        return V(r.x, r.y, r.z);
+    }
     RD uint32_t nfaces() const { return h->nf; }
     RD uint32_t nhe() const { return h->nhe; }
     RD hedge edge(uint32_t e) const {
-        const uint32_t* c = w + h->off_edges + 4 * e;
-        hedge r; r.vertex = c[0]; r.twin = c[1]; r.face = c[2]; r.next = c[3];
+        const uint4 c = *reinterpret_cast<const uint4*>(w + h->off_edges + 4 * e);
+        hedge r; r.vertex = c.x; r.twin = c.y; r.face = c.z; r.next = c.w;
         return r;
     }
     RD uint32_t face_edge(uint32_t fi) const { return w[h->off_face_edge + fi]; }
     RD uint32_t face_count(uint32_t fi) const { return w[h->off_face_count + fi]; }
     RD uint32_t face_vertex(uint32_t fi, uint32_t i) const { return w[h->off_face_verts + w[h->off_face_start + fi] + i]; }
     // ConvexMeshShape::getVertexPosition (ConvexMeshShape.h:214-217), pre-scaled
-    RD v3 vertex(uint32_t v) const { const uint32_t o = h->off_sverts + 3 * v; return V(f(o), f(o + 1), f(o + 2)); }
+    RD v3 vertex(uint32_t v) const { return row(h->off_sverts, v); }
     // ConvexMeshShape::getFaceNormal (ConvexMeshShape.h:220-223)
-    RD v3 normal(uint32_t fi) const { const uint32_t o = h->off_normals + 3 * fi; return V(f(o), f(o + 1), f(o + 2)); }
+    RD v3 normal(uint32_t fi) const { return row(h->off_normals, fi); }
     RD v3 centroid() const { return V(h->centroid[0], h->centroid[1], h->centroid[2]); }
     // ConvexMeshShape::getLocalSupportPointWithoutMargin (ConvexMeshShape.cpp:80-102):
     // brute force over the unscaled vertices, strict '>' keeps the first maximum
@@ -116,7 +119,7 @@ struct MeshPoly {
         const uint32_t nv = h->nv;
         const uint32_t o = h->off_verts;
         for (uint32_t i = 0; i < nv; i++) {
-            const float dp = vdot(d, V(f(o + 3 * i), f(o + 3 * i + 1), f(o + 3 * i + 2)));
+            const float dp = vdot(d, row(o, i));
             if (dp > maxd) { imax = i; maxd = dp; }
         }
         return vertex(imax);
@@ -1374,7 +1377,8 @@ RD void capsule_poly(Item& it, bool cap1, CapsuleS cap, const P& poly) {
 // bit-identical to the sequential loops.
 // ===========================================================================
 constexpr unsigned FULL_MASK = 0xffffffffu;
-constexpr uint32_t WARP_EDGE_CAP = 128;  // even half-edges of polyhedron 1 staged per warp
+constexpr uint32_t WARP_EDGE_CAP = MAX_MESH_HALF_EDGES / 2;  // edges (even half-edges) of a polyhedron
+constexpr uint32_t WARP_FACE_CAP = MAX_MESH_HALF_EDGES / 3;  // faces: a closed mesh has three half-edges or more a face
 
 // Optional per-phase cycle counters (the device counterpart of the
 // reference's RP3D_PROFILE scopes), compiled in with -DRP3DG_PROFILE_PHASES.
@@ -1404,41 +1408,58 @@ struct PhaseTimer {
 };
 #endif
 
-// Per-edge data of polyhedron 1 in polyhedron-2 space, staged in shared memory.
-struct Edge1Stage {
-    float e1A[3], dir1[3], a[3], b[3], bxa[3];
-};
-// Shared-memory scratch of one warp: staged edges, the list of edge pairs
-// that pass the Gauss-map test (in visiting order) and the clip polygon.
+// Shared-memory scratch of one warp: the face normals of polyhedron 1 rotated
+// into polyhedron-2 space, the edge pairs that pass the Gauss-map test
+// (i * 128 + j, in visiting order) and the clip polygon.
 constexpr uint32_t WARP_CAND_CAP = 512;
 struct WarpScratch {
-    union {
-        Edge1Stage stage[WARP_EDGE_CAP];
-        float feat[32][32];  // a tile's MLP input rows (consumed before the SAT starts)
-    };
+    float4 nr[WARP_FACE_CAP + 1];
+    float4 bn[6];       // a box's rotated face normals (faces of a box against a mesh)
     uint16_t cand[WARP_CAND_CAP];
     v3 poly[CLIP_MAX];
-    uint32_t cls[32];
 };
+// With a mesh as polyhedron 2 also, per face of either polyhedron, a bit per
+// edge of the other one: the side of the edge's plane the normal lies on.
+struct WarpScratchMesh : WarpScratch {
+    uint4 side1[WARP_FACE_CAP + 1], side2[WARP_FACE_CAP + 1];
+};
+static_assert(sizeof(WarpScratch) % 16 == 0 && sizeof(WarpScratchMesh) % 16 == 0, "rows stay aligned");
+
+// A key that orders like the float (no NaN; the two zeros alike): the warp's
+// minimum or maximum is then one reduction instruction instead of five
+// shuffle steps.
+RD uint32_t order_key(float x) {
+    const uint32_t u = __float_as_uint(x + 0.0f);
+    return u ^ (uint32_t(int32_t(u) >> 31) | 0x80000000u);
+}
+RD float order_value(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? k ^ 0x80000000u : ~k); }
 
 RD void warp_argmin(float& d, uint32_t& idx) {
-    for (int o = 16; o; o >>= 1) {
-        const float od = __shfl_xor_sync(FULL_MASK, d, o);
-        const uint32_t oi = __shfl_xor_sync(FULL_MASK, idx, o);
-        if (od < d || (od == d && oi < idx)) { d = od; idx = oi; }
-    }
+    const uint32_t key = order_key(d), m = __reduce_min_sync(FULL_MASK, key);
+    idx = __reduce_min_sync(FULL_MASK, key == m ? idx : 0xffffffffu);
+    d = order_value(m);
 }
 
-// testFacesDirectionPolyhedronVsPolyhedron (SATAlgorithm.cpp:1113-1142), faces spread over lanes
-template <class PA, class PB>
-RD float warp_sat_faces(const PA& pa, const PB& pb, const xform& a2b, uint32_t& minFace, int lane) {
+// testFacesDirectionPolyhedronVsPolyhedron (SATAlgorithm.cpp:1113-1142), faces
+// spread over lanes; nr keeps the rotated normals for the edge pairs.
+template <class PB>
+RD float warp_sat_faces(const MeshPoly& pa, const PB& pb, const xform& a2b, uint32_t& minFace, int lane, WarpScratch&,
+                        float4* nr = nullptr) {
     const uint32_t nf = pa.nfaces();
     float best = DECIMAL_LARGEST;
     uint32_t bestF = 0xffffffffu;
     for (uint32_t base = 0; base < nf; base += 32) {
         const uint32_t f = base + lane;
         const bool valid = f < nf;
-        const float d = valid ? sat_single_face(pa, pb, a2b, f) : DECIMAL_LARGEST;
+        float d = DECIMAL_LARGEST;
+        if (valid) {
+            // testSingleFaceDirectionPolyhedronVsPolyhedron, as sat_single_face
+            const v3 fn2 = qrot(a2b.q, pa.normal(f));
+            if (nr) nr[f] = make_float4(fn2.x, fn2.y, fn2.z, 0.0f);
+            const v3 sp = pb.support(vneg(fn2));
+            const v3 fv = xapply(a2b, pa.vertex(pa.face_vertex(f, 0)));
+            d = vdot(vsub(fv, sp), fn2);
+        }
         const unsigned sep = __ballot_sync(FULL_MASK, valid && d <= 0.0f);
         if (sep) {
             const int l = __ffs(sep) - 1;
@@ -1448,71 +1469,64 @@ RD float warp_sat_faces(const PA& pa, const PB& pb, const xform& a2b, uint32_t& 
         if (valid && d < best) { best = d; bestF = f; }
     }
     warp_argmin(best, bestF);
-    minFace = bestF;
+    minFace = bestF == 0xffffffffu ? 0u : bestF;
     return best;
 }
 
-// Support point of a convex mesh with the vertices spread over lanes
-// (ConvexMeshShape::getLocalSupportPointWithoutMargin, ConvexMeshShape.cpp:80-102):
-// the first vertex with the largest dot product; a dot product only counts
-// when it beats DECIMAL_SMALLEST, exactly like the reference's running maximum.
-RD v3 warp_mesh_support(const MeshPoly& m, v3 d, int lane) {
-    float best = DECIMAL_SMALLEST;
-    uint32_t bi = 0xffffffffu;
-    const uint32_t nv = m.h->nv, o = m.h->off_verts;
-    for (uint32_t i = lane; i < nv; i += 32) {
-        const float dp = vdot(d, V(m.f(o + 3 * i), m.f(o + 3 * i + 1), m.f(o + 3 * i + 2)));
-        if (dp > best) { best = dp; bi = i; }
+// The same for the faces of a box against a convex mesh: lane f (0..5) holds
+// face f, every lane searches its share of the mesh's vertices for the
+// support points of all six (ConvexMeshShape::getLocalSupportPointWithoutMargin,
+// ConvexMeshShape.cpp:80-102: the first vertex with the largest dot product
+// that beats DECIMAL_SMALLEST).
+RD float warp_sat_faces(const BoxPoly& pa, const MeshPoly& pb, const xform& a2b, uint32_t& minFace, int lane,
+                        WarpScratch& ws, float4* nr = nullptr) {
+    const uint32_t face = lane < 6 ? uint32_t(lane) : 5u;
+    const v3 fn2 = qrot(a2b.q, pa.normal(face));
+    __syncwarp();
+    if (lane < 6) {
+        ws.bn[lane] = make_float4(fn2.x, fn2.y, fn2.z, 0.0f);
+        if (nr) nr[lane] = make_float4(fn2.x, fn2.y, fn2.z, 0.0f);
     }
-    for (int s = 16; s; s >>= 1) {
-        const float ob = __shfl_xor_sync(FULL_MASK, best, s);
-        const uint32_t oi = __shfl_xor_sync(FULL_MASK, bi, s);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-    }
-    return m.vertex(bi == 0xffffffffu ? 0u : bi);
-}
-
-// testFacesDirectionPolyhedronVsPolyhedron for the faces of a box against a
-// convex mesh: faces in order (first separating face, strict minimum), the
-// mesh support search spread over the lanes.
-RD float warp_sat_faces(const BoxPoly& pa, const MeshPoly& pb, const xform& a2b, uint32_t& minFace, int lane) {
-    // the six support searches run side by side (independent accumulators)
+    __syncwarp();
     v3 dir[6];
     float best[6];
     uint32_t bi[6];
 #pragma unroll
     for (uint32_t f = 0; f < 6; f++) {
-        dir[f] = vneg(qrot(a2b.q, pa.normal(f)));
+        const float4 n = ws.bn[f];
+        dir[f] = V(-n.x, -n.y, -n.z);
         best[f] = DECIMAL_SMALLEST;
         bi[f] = 0xffffffffu;
     }
     const uint32_t nv = pb.h->nv, o = pb.h->off_verts;
     for (uint32_t i = lane; i < nv; i += 32) {
-        const v3 v = V(pb.f(o + 3 * i), pb.f(o + 3 * i + 1), pb.f(o + 3 * i + 2));
+        const v3 v = pb.row(o, i);
 #pragma unroll
         for (uint32_t f = 0; f < 6; f++) {
             const float dp = vdot(dir[f], v);
             if (dp > best[f]) { best[f] = dp; bi[f] = i; }
         }
     }
+    uint32_t sel = 0xffffffffu;
 #pragma unroll
-    for (int sft = 16; sft; sft >>= 1) {
-#pragma unroll
-        for (uint32_t f = 0; f < 6; f++) {
-            const float ob = __shfl_xor_sync(FULL_MASK, best[f], sft);
-            const uint32_t oi = __shfl_xor_sync(FULL_MASK, bi[f], sft);
-            if (ob > best[f] || (ob == best[f] && oi < bi[f])) { best[f] = ob; bi[f] = oi; }
-        }
-    }
-    float minDepth = DECIMAL_LARGEST;
     for (uint32_t f = 0; f < 6; f++) {
-        const v3 fn2 = qrot(a2b.q, pa.normal(f));
-        const v3 sp = pb.vertex(bi[f] == 0xffffffffu ? 0u : bi[f]);
-        const v3 fv = xapply(a2b, pa.vertex(pa.face_vertex(f, 0)));
-        const float d = vdot(vsub(fv, sp), fn2);
-        if (d <= 0.0f) { minFace = f; return d; }
-        if (d < minDepth) { minDepth = d; minFace = f; }
+        const uint32_t key = order_key(best[f]), m = __reduce_max_sync(FULL_MASK, key);
+        const uint32_t i = __reduce_min_sync(FULL_MASK, key == m ? bi[f] : 0xffffffffu);
+        if (face == f) sel = i;
     }
+    const v3 sp = pb.vertex(sel == 0xffffffffu ? 0u : sel);
+    const v3 fv = xapply(a2b, pa.vertex(pa.face_vertex(face, 0)));
+    const float d = vdot(vsub(fv, sp), fn2);
+    const unsigned sep = __ballot_sync(FULL_MASK, lane < 6 && d <= 0.0f);
+    if (sep) {
+        minFace = uint32_t(__ffs(sep)) - 1u;
+        return __shfl_sync(FULL_MASK, d, int(minFace));
+    }
+    const bool counts = lane < 6 && d < DECIMAL_LARGEST;
+    float minDepth = counts ? d : DECIMAL_LARGEST;
+    uint32_t bestF = counts ? uint32_t(lane) : 0xffffffffu;
+    warp_argmin(minDepth, bestF);
+    minFace = bestF == 0xffffffffu ? 0u : bestF;
     return minDepth;
 }
 
@@ -1538,21 +1552,11 @@ RD uint32_t warp_most_antiparallel_face(const P& p, v3 dir, int lane) {
     return bestF == 0xffffffffu ? 0u : bestF;
 }
 
-RD uint32_t warp_exclusive_scan(uint32_t v, int lane, uint32_t& total) {
-    uint32_t x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(FULL_MASK, x, o);
-        if (lane >= o) x += y;
-    }
-    total = __shfl_sync(FULL_MASK, x, 31);
-    return x - v;
-}
-
 // computePolyhedronVsPolyhedronFaceContactPoints (SATAlgorithm.cpp:893-1036)
 // on a whole warp.  Each Sutherland-Hodgman pass (clipPolygonWithPlane,
 // mathematics_functions.h:332-393) gives lane l the polygon edge that ends at
-// vertex l; its 0, 1 or 2 output points go to position (exclusive prefix sum
-// of the counts), which is exactly the sequential output order.  Vertex dot
+// vertex l; its 0, 1 or 2 output points go to the position that the counts of
+// the lanes before it give (two ballots), which is exactly the sequential output order.  Vertex dot
 // products are the same expressions as in the sequential pass.  Contacts are
 // appended in clipped-vertex order.  All lanes return the same value.
 // Functions a pair runs at most once or twice (the clipping of the contact
@@ -1593,31 +1597,24 @@ RD_COLD bool warp_face_contacts(bool ref1, const PR& refP, const PI& incP, const
         const int src = lane == 0 ? int(n) - 1 : lane - 1;
         const v3 S = V(__shfl_sync(FULL_MASK, P.x, src), __shfl_sync(FULL_MASK, P.y, src), __shfl_sync(FULL_MASK, P.z, src));
         const float vsn = __shfl_sync(FULL_MASK, ven, src);
-        v3 o0 = V(0.0f, 0.0f, 0.0f), o1 = V(0.0f, 0.0f, 0.0f);
-        uint32_t cnt = 0;
-        if (active) {
-            if (ven >= 0.0f) {
-                if (vsn < 0.0f) {
-                    const float t = plane_segment_intersection(S, P, pnpp, pn);
-                    o0 = (t >= 0.0f && t <= 1.0f) ? vadd(S, vmul(vsub(P, S), t)) : P;
-                    o1 = P;
-                    cnt = 2;
-                } else {
-                    o0 = P;
-                    cnt = 1;
-                }
-            } else if (vsn >= 0.0f) {
-                const float t = plane_segment_intersection(S, P, -pnpp, vneg(pn));
-                o0 = (t >= 0.0f && t <= 1.0f) ? vadd(S, vmul(vsub(P, S), t)) : S;
-                cnt = 1;
-            }
+        // an edge that enters the plane's inner side gives the intersection
+        // and its end, one that leaves it the intersection with the plane
+        // turned round, one inside its end: one intersection for both signs
+        const bool in = ven >= 0.0f;
+        const bool enters = active && in && vsn < 0.0f, leaves = active && !in && vsn >= 0.0f;
+        v3 o0 = P;
+        if (enters || leaves) {
+            const float t = plane_segment_intersection(S, P, in ? pnpp : -pnpp, in ? pn : vneg(pn));
+            o0 = (t >= 0.0f && t <= 1.0f) ? vadd(S, vmul(vsub(P, S), t)) : (in ? P : S);
         }
         NP_EV(it, EV_CLIP_INTERSECT, __popc(__ballot_sync(FULL_MASK, active && (ven >= 0.0f) != (vsn >= 0.0f))));
-        uint32_t total;
-        const uint32_t pos = warp_exclusive_scan(cnt, lane, total);
-        __syncwarp();
-        if (cnt >= 1 && pos < CLIP_MAX) poly[pos] = o0;
-        if (cnt == 2 && pos + 1 < CLIP_MAX) poly[pos + 1] = o1;
+        const bool one = active && (in || leaves);
+        const unsigned m1 = __ballot_sync(FULL_MASK, one), m2 = __ballot_sync(FULL_MASK, enters);
+        const unsigned before = (1u << lane) - 1u;
+        const uint32_t pos = uint32_t(__popc(m1 & before) + __popc(m2 & before));
+        const uint32_t total = uint32_t(__popc(m1) + __popc(m2));
+        if (one && pos < CLIP_MAX) poly[pos] = o0;
+        if (enters && pos + 1 < CLIP_MAX) poly[pos + 1] = P;
         __syncwarp();
         n = total < CLIP_MAX ? total : CLIP_MAX;
         if (uint32_t(lane) < n) P = poly[lane];
@@ -1655,83 +1652,247 @@ RD bool warp_poly_face_contacts(bool ref1, const P1& p1, const P2& p2, const xfo
     return warp_face_contacts(false, p2, p1, p2to1, p1to2, minFace, it, lane, poly);
 }
 
-// Walks the edge pairs (i, j) of the reference's double loop in visiting
-// order, a round at a time; lane `offset` of a round holds pair base + offset.
-// Generic polyhedron 2: 32 consecutive pairs per round.
-template <class P2>
-struct EdgePairWalker {
-    const P2& p2;
-    uint32_t n2h, ih, jh, qstep, rstep, offset, per_round;
-    bool active;
-    RD EdgePairWalker(const P2& p, uint32_t n2, int lane) : p2(p), n2h(n2) {
-        ih = uint32_t(lane) / n2h;
-        jh = uint32_t(lane) - ih * n2h;
-        qstep = 32u / n2h;
-        rstep = 32u - qstep * n2h;
-        offset = uint32_t(lane);
-        per_round = 32;
-        active = true;
+// One edge of polyhedron 1 in polyhedron-2 space, from the staged normals.
+template <class P1>
+RD Edge1Gauss warp_edge1_gauss(const P1& p1, uint32_t i, const xform& p1to2, const float4* nr) {
+    const hedge e1 = p1.edge(2 * i);
+    const hedge tw = p1.edge(e1.twin);
+    const float4 a = nr[e1.face], b = nr[tw.face];
+    Edge1Gauss g;
+    g.a = V(a.x, a.y, a.z);
+    g.b = V(b.x, b.y, b.z);
+    g.bxa = qrot(p1to2.q, vsub(p1.vertex(e1.vertex), p1.vertex(tw.vertex)));
+    return g;
+}
+
+// The products of testGaussMapArcsIntersect between one edge and the edges of
+// a box (see edges_minkowski for a box) have one magnitude for the four box
+// edges along an axis k, and signs that the box edge's own three signs turn:
+//   adc * bdc = (a_k 2h)(b_k 2h)          bits 0..2: negative
+//   cba * dba = +/- bxa_m bxa_n           bits 3..5: negative, 6..8: positive
+//   cba * bdc = +/- bxa_m (b_k 2h)        bits 9..14: positive, 15..20: negative
+// Negating a factor negates the product exactly, so box edge j passes exactly
+// when all bits of BoxTables::edge_need[j] are set: nine products an edge
+// instead of five for each of its twelve pairs.
+RD uint32_t box_edge_bits(const Edge1Gauss& g, v3 he) {
+    const float a[3] = {g.a.x, g.a.y, g.a.z}, b[3] = {g.b.x, g.b.y, g.b.z}, x[3] = {g.bxa.x, g.bxa.y, g.bxa.z};
+    const float h[3] = {he.x + he.x, he.y + he.y, he.z + he.z};
+    uint32_t bits = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int k1 = (k + 1) % 3, k2 = (k + 2) % 3;
+        const float adc = a[k] * h[k], bdc = b[k] * h[k];
+        const float ab = adc * bdc, xx = x[k1] * x[k2], q1 = x[k1] * bdc, q2 = x[k2] * bdc;
+        if (ab < 0.0f) bits |= 1u << k;
+        if (xx < 0.0f) bits |= 1u << (3 + k);
+        if (xx > 0.0f) bits |= 1u << (6 + k);
+        if (q1 > 0.0f) bits |= 1u << (9 + 2 * k);
+        if (q2 > 0.0f) bits |= 1u << (10 + 2 * k);
+        if (q1 < 0.0f) bits |= 1u << (15 + 2 * k);
+        if (q2 < 0.0f) bits |= 1u << (16 + 2 * k);
     }
-    RD bool test(const Edge1Stage* stage) const {
-        const Edge1Stage& s = stage[ih];
-        Edge1Gauss g;
-        g.a = V(s.a[0], s.a[1], s.a[2]);
-        g.b = V(s.b[0], s.b[1], s.b[2]);
-        g.bxa = V(s.bxa[0], s.bxa[1], s.bxa[2]);
-        return edges_minkowski(g, p2, p2.edge(2 * jh), 2 * jh);
+    return bits;
+}
+
+// Appends each lane's edges (lane's row i, set bits of w as j) to a list, in
+// the order of the lanes; a lane whose edges no longer fit keeps them in w
+// and so do the lanes after it.  Returns whether all fitted.
+template <int WORDS>
+RD bool warp_append_rows(uint32_t (&w)[WORDS], uint32_t i, uint16_t* list, uint32_t& n, int lane) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int k = 0; k < WORDS; k++) c += uint32_t(__popc(w[k]));
+    uint32_t incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL_MASK, incl, o);
+        if (lane >= o) incl += y;
     }
-    RD void advance() {
-        jh += rstep; ih += qstep;
-        if (jh >= n2h) { jh -= n2h; ih++; }
+    const bool fits = n + incl <= WARP_CAND_CAP;
+    if (fits) {
+        uint32_t p = n + incl - c;
+#pragma unroll
+        for (int k = 0; k < WORDS; k++) {
+            for (uint32_t m = w[k]; m; m &= m - 1u) list[p++] = uint16_t(i * WARP_EDGE_CAP + 32 * k + __ffs(m) - 1);
+            w[k] = 0;
+        }
     }
-    static constexpr int UNROLL = 1;
-    RD bool test_ahead(const Edge1Stage* stage, int) const { return test(stage); }
-    RD void advance_by(int u) { for (int k = 0; k < u; k++) advance(); }
+    const int nfit = __popc(__ballot_sync(FULL_MASK, fits));   // the counts only grow: the first lanes
+    if (nfit > 0) n += __shfl_sync(FULL_MASK, incl, nfit - 1);
+    return nfit == 32;
+}
+
+// Two products or sums in one instruction, each rounded as the single one.
+RD uint64_t pack2(float a, float b) { return (uint64_t(__float_as_uint(b)) << 32) | __float_as_uint(a); }
+RD uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+RD uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Per face normal (row f of `rows`) a bit per edge: whether the normal's dot
+// product with the edge vector is positive.  Lane l holds the vectors of the
+// edges l + 32 k, k < 2 PAIRS, two to a register pair.
+template <int PAIRS>
+RD void warp_face_sides(const float4* rows, uint32_t nf, const v3 (&e)[4], uint4* sides, int lane) {
+    uint64_t x[PAIRS], y[PAIRS], z[PAIRS];
+#pragma unroll
+    for (int p = 0; p < PAIRS; p++) {
+        x[p] = pack2(e[2 * p].x, e[2 * p + 1].x);
+        y[p] = pack2(e[2 * p].y, e[2 * p + 1].y);
+        z[p] = pack2(e[2 * p].z, e[2 * p + 1].z);
+    }
+#pragma unroll 2
+    for (uint32_t f = 0; f < nf; f++) {
+        const float4 n = rows[f];
+        const uint64_t nx = pack2(n.x, n.x), ny = pack2(n.y, n.y), nz = pack2(n.z, n.z);
+        uint32_t m[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int p = 0; p < PAIRS; p++) {
+            const uint64_t s = add2(add2(mul2(nx, x[p]), mul2(ny, y[p])), mul2(nz, z[p]));
+            m[2 * p] = __ballot_sync(FULL_MASK, __uint_as_float(uint32_t(s)) > 0.0f);
+            m[2 * p + 1] = __ballot_sync(FULL_MASK, __uint_as_float(uint32_t(s >> 32)) > 0.0f);
+        }
+        if (lane == 0) sides[f] = make_uint4(m[0], m[1], m[2], m[3]);
+    }
+}
+
+// Transposes a 32 x 32 bit matrix, row = lane.
+RD uint32_t warp_transpose_bits(uint32_t x, int lane) {
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        const uint32_t m = s == 16 ? 0x0000ffffu : s == 8 ? 0x00ff00ffu : s == 4 ? 0x0f0f0f0fu : s == 2 ? 0x33333333u : 0x55555555u;
+        const uint32_t y = __shfl_xor_sync(FULL_MASK, x, s);
+        const bool low = (lane & s) == 0;
+        const uint32_t keep = low ? m : ~m;
+        const uint32_t t = __funnelshift_l(y, y, low ? s : 32 - s);
+        x = (x & keep) | (t & ~keep);
+    }
+    return x;
+}
+
+// The edge pairs (i, j) of the reference's double loop that may pass the
+// Gauss-map test, in visiting order, appended to ws.cand until it could
+// overflow; more() tells whether any are left, test() is the test itself
+// where the list holds pairs that may still fail it.
+//
+// Polyhedron 2 a box: lane = edge i, its twelve tests from 21 sign bits.
+template <class P1, class P2>
+struct EdgePairs {
+    typedef WarpScratch Scratch;
+    const P1& p1;
+    const BoxPoly& p2;
+    uint32_t base, n1h;
+    RD EdgePairs(const P1& a, const BoxPoly& b, uint32_t n1, uint32_t, const xform&, Scratch&, int)
+        : p1(a), p2(b), base(0), n1h(n1) {}
+    RD bool more() const { return base < n1h; }
+    RD void fill(Scratch& ws, uint32_t& ncand, const xform& p1to2, int lane) {
+        while (base < n1h && ncand + 12 * 32 <= WARP_CAND_CAP) {
+            const uint32_t i = base + lane;
+            uint32_t w[1] = {0};
+            if (i < n1h) {
+                const uint32_t bits = box_edge_bits(warp_edge1_gauss(p1, i, p1to2, ws.nr), p2.he);
+#pragma unroll
+                for (int j = 0; j < 12; j++) {
+                    const uint32_t need = p2.t->edge_need[j];
+                    if ((bits & need) == need) w[0] |= 1u << j;
+                }
+            }
+            warp_append_rows(w, i, ws.cand, ncand, lane);   // fits: at most twelve a lane
+            base += 32;
+        }
+    }
+    RD bool test(uint32_t, const xform&, const Scratch&) const { return true; }
 };
-// Box polyhedron 2: its 12 even half-edges are fixed per lane (lanes 0..23 =
-// two rows i of the loop), so each lane keeps its box edge's Gauss-map data in
-// registers and reads only the three components of the staged edge it needs.
-template <>
-struct EdgePairWalker<BoxPoly> {
-    uint32_t ih, offset, per_round;
-    bool active;
-    uint32_t k, m, n;
-    bool negC, negD2;
-    float D;
-    RD EdgePairWalker(const BoxPoly& p2, uint32_t, int lane) {
-        active = lane < 24;
-        const uint32_t jh = uint32_t(lane) % 12u, half = uint32_t(lane) / 12u;
-        ih = half;
-        offset = uint32_t(lane);
-        per_round = 24;
-        const uint8_t* gi = p2.t->gauss[2 * jh];
-        k = gi[0] & 3u; m = gi[1] & 3u; n = gi[2] & 3u;
-        negC = (gi[1] & 4u) != 0;
-        negD2 = (gi[2] & 4u) != 0;
-        const float hk = axis_component(p2.he, k);
-        D = (gi[0] & 4u) ? -(hk + hk) : (hk + hk);
+
+// Polyhedron 2 a mesh.  The test asks among other things that the normals of
+// edge i's faces lie strictly on opposite sides of the plane across edge j
+// (adc * bdc < 0), and those of edge j's faces of the plane across edge i
+// (cba * dba < 0).  A normal's side is the same for all edges of its face, so
+// the sides are computed once per face and edge of the other polyhedron, as
+// bit masks (80 x 120 dot products either way for two 42-vertex hulls, four
+// edges a lane), instead of in each of the 120 x 120 pairs; a pair is left
+// when both its masks differ (about one in a hundred), and takes the whole
+// test.  One pass over all pairs took 89 % of the kernel's cycles.
+template <class P1>
+struct EdgePairs<P1, MeshPoly> {
+    typedef WarpScratchMesh Scratch;
+    const P1& p1;
+    const MeshPoly& p2;
+    uint32_t base, n1h, n2h;
+    uint32_t w[4];
+    uint32_t faces2[4];   // of edge j = 32 k + lane
+    bool rows_left;
+    RD EdgePairs(const P1& a, const MeshPoly& b, uint32_t n1, uint32_t n2, const xform& p1to2, Scratch& ws, int lane)
+        : p1(a), p2(b), base(0), n1h(n1), n2h(n2), rows_left(false) {
+        v3 e[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) {
+            const uint32_t j = 32 * k + lane;
+            e[k] = V(0.0f, 0.0f, 0.0f);   // gives no bits
+            faces2[k] = 0;
+            if (j < n2h) {
+                const hedge e2 = p2.edge(2 * j), tw = p2.edge(e2.twin);
+                e[k] = vsub(p2.vertex(e2.vertex), p2.vertex(tw.vertex));
+                faces2[k] = e2.face | (tw.face << 16);
+            }
+        }
+        if (n2h > 64) warp_face_sides<2>(ws.nr, p1.nfaces(), e, ws.side1, lane);
+        else warp_face_sides<1>(ws.nr, p1.nfaces(), e, ws.side1, lane);
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) {
+            const uint32_t i = 32 * k + lane;
+            e[k] = V(0.0f, 0.0f, 0.0f);
+            if (i < n1h) {
+                const hedge e1 = p1.edge(2 * i), tw = p1.edge(e1.twin);
+                e[k] = qrot(p1to2.q, vsub(p1.vertex(e1.vertex), p1.vertex(tw.vertex)));
+            }
+        }
+        const float4* normals2 = reinterpret_cast<const float4*>(p2.w + p2.h->off_normals);
+        if (n1h > 64) warp_face_sides<2>(normals2, p2.nfaces(), e, ws.side2, lane);
+        else warp_face_sides<1>(normals2, p2.nfaces(), e, ws.side2, lane);
+        __syncwarp();
     }
-    RD bool test(const Edge1Stage* stage) const { return test_ahead(stage, 0); }
-    RD bool test_ahead(const Edge1Stage* stage, int u) const {
-        const Edge1Stage& s = stage[ih + 2 * u];
-        const float bm = s.bxa[m], bn = s.bxa[n];
-        const float cba = negC ? -bm : bm;
-        const float dba = negD2 ? -bn : bn;
-        const float adc = s.a[k] * D;
-        const float bdc = s.b[k] * D;
-        return cba * dba < 0.0f && adc * bdc < 0.0f && cba * bdc > 0.0f;
+    RD bool more() const { return rows_left || base < n1h; }
+    RD void fill(Scratch& ws, uint32_t& ncand, const xform&, int lane) {
+        while (rows_left || base < n1h) {
+            if (!rows_left) {
+                // rows i = base + lane over the words of j
+                uint4 s = make_uint4(0, 0, 0, 0);
+                if (base + lane < n1h) {
+                    const hedge e1 = p1.edge(2 * (base + lane));
+                    const uint4 a = ws.side1[e1.face], b = ws.side1[p1.edge(e1.twin).face];
+                    s = make_uint4(a.x ^ b.x, a.y ^ b.y, a.z ^ b.z, a.w ^ b.w);
+                }
+                w[0] = s.x; w[1] = s.y; w[2] = s.z; w[3] = s.w;
+                const uint32_t* sides2 = &ws.side2[0].x + base / 32;
+#pragma unroll
+                for (uint32_t k = 0; k < 4; k++)
+                    if (32 * k < n2h)
+                        w[k] &= warp_transpose_bits(sides2[4 * (faces2[k] & 0xffffu)] ^ sides2[4 * (faces2[k] >> 16)], lane);
+            }
+            rows_left = !warp_append_rows(w, base + lane, ws.cand, ncand, lane);
+            if (rows_left) return;
+            base += 32;
+        }
     }
-    RD void advance() { ih += 2; }
-    static constexpr int UNROLL = 4;
-    RD void advance_by(int u) { ih += 2 * u; }
+    RD bool test(uint32_t pair, const xform& p1to2, const Scratch& ws) const {
+        return edges_minkowski(warp_edge1_gauss(p1, pair / WARP_EDGE_CAP, p1to2, ws.nr), p2,
+                               p2.edge(2 * (pair % WARP_EDGE_CAP)));
+    }
 };
 
 // testCollisionConvexPolyhedronVsConvexPolyhedron (SATAlgorithm.cpp:485-889), one warp per pair.
 // Every lane holds the same pair state; contacts and outputs are produced by lane 0.
 template <class P1, class P2>
-RD void warp_sat_poly_poly(Item& it, const P1& p1, const P2& p2, bool clipPrev, int lane, WarpScratch& ws) {
+RD void warp_sat_poly_poly(Item& it, const P1& p1, const P2& p2, bool clipPrev, int lane,
+                           typename EdgePairs<P1, P2>::Scratch& ws) {
     NP_EV(it, EV_POLY_SETUP, 1);
-    Edge1Stage* stage = ws.stage;
     PhaseTimer timer(lane);
     const xform p1to2 = xmul(xinv(it.t2), it.t1);
     const xform p2to1 = xinv(p1to2);
@@ -1800,14 +1961,14 @@ RD void warp_sat_poly_poly(Item& it, const P1& p1, const P2& p2, bool clipPrev, 
     }
     timer.mark(0);
     uint32_t f1 = 0, f2 = 0;
-    const float d1 = warp_sat_faces(p1, p2, p1to2, f1, lane);
+    const float d1 = warp_sat_faces(p1, p2, p1to2, f1, lane, ws, ws.nr);
     ev_face_tests(it, p2, d1 <= 0.0f ? f1 + 1 : p1.nfaces());
     timer.mark(1);
     if (d1 <= 0.0f) {
         lf.set(RP3DG_LF_SAT_FACE_POLY1, true); lf.set(RP3DG_LF_SAT_FACE_POLY2, false); lf.sat_face = f1;
         return;
     }
-    const float d2 = warp_sat_faces(p2, p1, p2to1, f2, lane);
+    const float d2 = warp_sat_faces(p2, p1, p2to1, f2, lane, ws);
     ev_face_tests(it, p1, d2 <= 0.0f ? f2 + 1 : p2.nfaces());
     timer.mark(2);
     if (d2 <= 0.0f) {
@@ -1820,107 +1981,64 @@ RD void warp_sat_poly_poly(Item& it, const P1& p1, const P2& p2, bool clipPrev, 
     if (d1 < d2 * SAT_REL_TOL + SAT_ABS_TOL) { minFace = f1; isFace1 = true; }
     else { minFace = f2; isFace1 = false; }
 
-    // stage the even half-edges of polyhedron 1 (in polyhedron-2 space)
     const uint32_t n1h = (p1.nhe() + 1) / 2, n2h = (p2.nhe() + 1) / 2;
     const v3 c1 = xapply(p1to2, p1.centroid());
-    for (uint32_t ih = lane; ih < n1h; ih += 32) {
-        const hedge e1 = p1.edge(2 * ih);
-        const v3 e1A = xapply(p1to2, p1.vertex(e1.vertex));
-        const v3 e1B = xapply(p1to2, p1.vertex(p1.edge(e1.next).vertex));
-        const v3 dir1 = vsub(e1B, e1A);
-        const Edge1Gauss g = edge1_gauss(p1, e1, p1to2);
-        Edge1Stage& s = stage[ih];
-        s.e1A[0] = e1A.x; s.e1A[1] = e1A.y; s.e1A[2] = e1A.z;
-        s.dir1[0] = dir1.x; s.dir1[1] = dir1.y; s.dir1[2] = dir1.z;
-        s.a[0] = g.a.x; s.a[1] = g.a.y; s.a[2] = g.a.z;
-        s.b[0] = g.b.x; s.b[1] = g.b.y; s.b[2] = g.b.z;
-        s.bxa[0] = g.bxa.x; s.bxa[1] = g.bxa.y; s.bxa[2] = g.bxa.z;
-    }
-    __syncwarp();
+    __syncwarp();   // the rotated normals are in place
+    EdgePairs<P1, P2> pairs(p1, p2, n1h, n2h, p1to2, ws, lane);
     timer.mark(3);
-    const uint32_t total = n1h * n2h;
     float best = DECIMAL_LARGEST;
     uint32_t bestIdx = 0xffffffffu;
-    // Pass 1 walks the edge pairs in visiting order and appends the ones that
-    // pass the Gauss-map test to ws.cand; pass 2 (run whenever the list could
-    // overflow, and at the end) computes their distances 32 at a time.  The
-    // list keeps visiting order, so the first separating pair and the
-    // first arg-min are those of the sequential loop.
+    // The pairs are listed in visiting order, and their distances computed 32
+    // at a time whenever the list could overflow, and at the end.  The first
+    // separating pair and the first arg-min are those of the sequential loop.
     uint32_t ncand = 0;
-    bool separated = false;
-    NP_EV_ONLY(uint32_t cand_before = 0;)
-    EdgePairWalker<P2> walk(p2, n2h, lane);
-    for (uint32_t base = 0; base < total || ncand > 0;) {
-        if (EdgePairWalker<P2>::UNROLL > 1 && base < total && ncand + 32 * EdgePairWalker<P2>::UNROLL <= WARP_CAND_CAP) {
-            // several rounds at once: independent loads and tests, then the
-            // ballots in round order (keeps the visiting order)
-            constexpr int U = EdgePairWalker<P2>::UNROLL;
-            bool pass[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const uint32_t idx = base + u * walk.per_round + walk.offset;
-                pass[u] = walk.active && idx < total && walk.test_ahead(stage, u);
-            }
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const uint32_t idx = base + u * walk.per_round + walk.offset;
-                const unsigned m = __ballot_sync(FULL_MASK, pass[u]);
-                if (pass[u]) ws.cand[ncand + __popc(m & ((1u << lane) - 1u))] = uint16_t(idx);
-                ncand += __popc(m);
-            }
-            base += U * walk.per_round;
-            walk.advance_by(U);
-            continue;
-        }
-        if (base < total && ncand + 32 <= WARP_CAND_CAP) {
-            const uint32_t idx = base + walk.offset;
-            const bool pass = walk.active && idx < total && walk.test(stage);
-            const unsigned m = __ballot_sync(FULL_MASK, pass);
-            if (pass) ws.cand[ncand + __popc(m & ((1u << lane) - 1u))] = uint16_t(idx);
-            ncand += __popc(m);
-            base += walk.per_round;
-            walk.advance();
-            continue;
-        }
+    NP_EV_ONLY(uint32_t tested = 0;)
+    do {
+        pairs.fill(ws, ncand, p1to2, lane);
         __syncwarp();
-        for (uint32_t c0 = 0; c0 < ncand && !separated; c0 += 32) {
+        for (uint32_t c0 = 0; c0 < ncand; c0 += 32) {
             const uint32_t c = c0 + lane;
             float d = DECIMAL_LARGEST;
             uint32_t idx = 0xffffffffu;
+            bool pass = false;
             if (c < ncand) {
                 idx = ws.cand[c];
-                const uint32_t ci = idx / n2h, cj = idx - ci * n2h;
-                const Edge1Stage& s = stage[ci];
-                hedge e2;
-                v3 e2A, dir2, axis;
-                edge2_data(p2, 2 * cj, e2, e2A, dir2);
-                d = sat_edge_distance(V(s.e1A[0], s.e1A[1], s.e1A[2]), e2A, c1, V(s.dir1[0], s.dir1[1], s.dir1[2]),
-                                      dir2, axis);
+                pass = pairs.test(idx, p1to2, ws);
+                if (pass) {
+                    const hedge e1 = p1.edge(2 * (idx / WARP_EDGE_CAP));
+                    const v3 e1A = xapply(p1to2, p1.vertex(e1.vertex));
+                    const v3 dir1 = vsub(xapply(p1to2, p1.vertex(p1.edge(e1.next).vertex)), e1A);
+                    hedge e2;
+                    v3 e2A, dir2, axis;
+                    edge2_data(p2, 2 * (idx % WARP_EDGE_CAP), e2, e2A, dir2);
+                    d = sat_edge_distance(e1A, e2A, c1, dir1, dir2, axis);
+                }
             }
-            const unsigned sep = __ballot_sync(FULL_MASK, c < ncand && d <= 0.0f);
+            NP_EV_ONLY(const unsigned passed = __ballot_sync(FULL_MASK, pass);)
+            const unsigned sep = __ballot_sync(FULL_MASK, pass && d <= 0.0f);
             if (sep) {
-                const uint32_t first = __shfl_sync(FULL_MASK, idx, __ffs(sep) - 1);
-                const uint32_t fi = first / n2h;
+                const int l = __ffs(sep) - 1;
+                const uint32_t first = __shfl_sync(FULL_MASK, idx, l);
+                const uint32_t fi = first / WARP_EDGE_CAP, fj = first % WARP_EDGE_CAP;
                 // the reference's loop stops at this pair
                 NP_EV(it, EV_EDGE1, fi + 1);
-                NP_EV(it, EV_GAUSS, first + 1);
-                NP_EV(it, EV_EDGE_DIST, cand_before + c0 + uint32_t(__ffs(sep)));
+                NP_EV(it, EV_GAUSS, fi * n2h + fj + 1);
+                NP_EV(it, EV_EDGE_DIST, tested + uint32_t(__popc(passed & ((2u << l) - 1u))));
                 lf.set(RP3DG_LF_SAT_FACE_POLY1, false); lf.set(RP3DG_LF_SAT_FACE_POLY2, false);
                 lf.sat_e1 = 2 * fi;
-                lf.sat_e2 = 2 * (first - fi * n2h);
-                separated = true;
-            } else if (c < ncand && d < best) {
-                best = d; bestIdx = idx;
+                lf.sat_e2 = 2 * fj;
+                __syncwarp();
+                return;
             }
+            NP_EV_ONLY(tested += uint32_t(__popc(passed));)
+            if (pass && d < best) { best = d; bestIdx = idx; }
         }
         __syncwarp();
-        if (separated) return;
-        NP_EV_ONLY(cand_before += ncand;)
         ncand = 0;
-    }
+    } while (pairs.more());
     NP_EV(it, EV_EDGE1, n1h);
-    NP_EV(it, EV_GAUSS, total);
-    NP_EV(it, EV_EDGE_DIST, cand_before);
+    NP_EV(it, EV_GAUSS, n1h * n2h);
+    NP_EV(it, EV_EDGE_DIST, tested);
     warp_argmin(best, bestIdx);
     __syncwarp();
     timer.mark(4);
@@ -1931,7 +2049,7 @@ RD void warp_sat_poly_poly(Item& it, const P1& p1, const P2& p2, bool clipPrev, 
         lf.set(RP3DG_LF_SAT_FACE_POLY1, isFace1); lf.set(RP3DG_LF_SAT_FACE_POLY2, !isFace1); lf.sat_face = minFace;
         if (!found) return;
     } else {
-        const uint32_t ih = bestIdx / n2h, jh = bestIdx - ih * n2h;
+        const uint32_t ih = bestIdx / WARP_EDGE_CAP, jh = bestIdx % WARP_EDGE_CAP;
         if (it.report) {
             NP_EV(it, EV_EDGE_CONTACT, 1);
             const hedge e1 = p1.edge(2 * ih);

@@ -11,7 +11,7 @@ namespace rp3dg {
 
 constexpr int NP_BLOCK = 128;
 // Mesh arenas up to this size are staged in shared memory by every CTA.
-constexpr uint32_t MESH_STAGE_MAX_BYTES = 96 * 1024;
+constexpr uint32_t MESH_STAGE_MAX_BYTES = 108 * 1024;
 
 struct NpArgs {
     uint32_t n;

@@ -204,10 +204,10 @@ RD bool ray_mesh(v3 p1, v3 p2, float maxf, const MeshHdr* H, const uint32_t* w, 
     bool found = false;
     const uint32_t nf = H->nf;
     for (uint32_t f = 0; f < nf; f++) {
-        const uint32_t on = H->off_normals + 3 * f;
+        const uint32_t on = H->off_normals + 4 * f;
         const v3 nrm = V(__uint_as_float(w[on]), __uint_as_float(w[on + 1]), __uint_as_float(w[on + 2]));
         const uint32_t v0 = w[H->off_face_verts + w[H->off_face_start + f]];
-        const uint32_t ov = H->off_verts + 3 * v0;
+        const uint32_t ov = H->off_verts + 4 * v0;
         const v3 fp = V(__uint_as_float(w[ov]), __uint_as_float(w[ov + 1]), __uint_as_float(w[ov + 2]));
         const float denom = vdot(nrm, d);
         const float planeD = vdot(nrm, fp);

@@ -183,6 +183,11 @@ BoxTables make_box_tables() {
     for (int e = 0; e < 24; e += 2) {
         const int k = t.gauss[e][0] & 3;
         if (fillc[k] < 4) t.axis_edges[k][fillc[k]++] = uint8_t(e);
+        // see box_edge_bits: c = s1 e_m, d = s2 e_n, D = s3 2h_k
+        const int m = t.gauss[e][1] & 3;
+        const bool neg_c = (t.gauss[e][1] & 4) != 0, neg_d = (t.gauss[e][2] & 4) != 0, neg_D = (t.gauss[e][0] & 4) != 0;
+        const int q = 2 * k + (m == (k + 1) % 3 ? 0 : 1);
+        t.edge_need[e / 2] = (1u << k) | (1u << ((neg_c == neg_d ? 3 : 6) + k)) | (1u << ((neg_c == neg_D ? 9 : 15) + q));
     }
     // PhysicsCommon::initTriangleShapeHalfEdgeStructure (reference
     // src/engine/PhysicsCommon.cpp:111-130): the two faces of a triangle
@@ -319,7 +324,16 @@ void rebuild_arena(rp3dg_ctx* ctx) {
     const uint32_t nin = uint32_t(ctx->instances.size());
     const uint32_t hdr_words = nin * (sizeof(MeshHdr) / 4);
     w.assign(hdr_words, 0u);
-    auto push_f = [&](float x) { uint32_t u; std::memcpy(&u, &x, 4); w.push_back(u); };
+    auto align4 = [&]() { w.resize((w.size() + 3) & ~size_t(3), 0u); };
+    align4();
+    auto push_rows = [&](const std::vector<float>& v) {
+        for (size_t k = 0; k < v.size(); k++) {
+            uint32_t u;
+            std::memcpy(&u, &v[k], 4);
+            w.push_back(u);
+            if (k % 3 == 2) w.push_back(0u);
+        }
+    };
     for (uint32_t k = 0; k < nin; k++) {
         const MeshInstance& in = ctx->instances[k];
         const MeshTopo& m = ctx->meshes[in.mesh];
@@ -327,11 +341,11 @@ void rebuild_arena(rp3dg_ctx* ctx) {
         std::memset(&h, 0, sizeof(h));
         h.nv = m.nv; h.nf = m.nf; h.nhe = uint32_t(m.edges.size());
         h.off_verts = uint32_t(w.size());
-        for (float x : m.verts) push_f(x);
+        push_rows(m.verts);
         h.off_sverts = uint32_t(w.size());
-        for (float x : in.sverts) push_f(x);
+        push_rows(in.sverts);
         h.off_normals = uint32_t(w.size());
-        for (float x : in.snormals) push_f(x);
+        push_rows(in.snormals);
         h.off_face_start = uint32_t(w.size());
         for (uint32_t x : m.face_start) w.push_back(x);
         h.off_face_count = uint32_t(w.size());
@@ -340,6 +354,7 @@ void rebuild_arena(rp3dg_ctx* ctx) {
         for (uint32_t x : m.face_verts) w.push_back(x);
         h.off_face_edge = uint32_t(w.size());
         for (uint32_t x : m.face_edge) w.push_back(x);
+        align4();
         h.off_edges = uint32_t(w.size());
         for (const HalfEdge& e : m.edges) { w.push_back(e.vertex); w.push_back(e.twin); w.push_back(e.face); w.push_back(e.next); }
         h.centroid[0] = in.scentroid[0]; h.centroid[1] = in.scentroid[1]; h.centroid[2] = in.scentroid[2];

@@ -19,9 +19,10 @@ constexpr uint32_t MAX_MESH_VERTICES = 4096;
 // All offsets are in 32-bit words from the start of the arena.
 struct MeshHdr {
     uint32_t nv, nf, nhe, pad0;
-    uint32_t off_verts;       // nv * 3 floats, unscaled (used by the support search)
-    uint32_t off_sverts;      // nv * 3 floats, vertex * scale
-    uint32_t off_normals;     // nf * 3 floats, scaled unit normals
+    // rows of four words (x, y, z, 0) on 16-byte boundaries: one 128-bit load each
+    uint32_t off_verts;       // nv rows, unscaled (used by the support search)
+    uint32_t off_sverts;      // nv rows, vertex * scale
+    uint32_t off_normals;     // nf rows, scaled unit normals
     uint32_t off_face_start;  // nf uint32: first index in face_verts
     uint32_t off_face_count;  // nf uint32
     uint32_t off_face_verts;  // sum(face_count) uint32
@@ -50,6 +51,9 @@ struct BoxTables {
     uint8_t tri_edges[6][4];   // vertex, twin, face, next
     uint8_t tri_face_edge[2];
     uint8_t pad2[2];
+    // Per even half-edge: the bits that box_edge_bits() must all have for an
+    // edge of the other polyhedron to pass the Gauss-map test against it.
+    uint32_t edge_need[12];
 };
 
 // Steps of the reference's narrow-phase code paths, counted per batch by the
