@@ -376,8 +376,8 @@ __global__ void __launch_bounds__(NP_BLOCK, MinBlocks<ALGO>::value) narrowphase_
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const uint32_t nwarps = gridDim.x * (NP_BLOCK / 32);
         uint32_t tested = 0, confirmed = 0;
-        for (uint32_t tile = blockIdx.x * (NP_BLOCK / 32) + warp; tile * 32u < a.n; tile += nwarps) {
-            const uint32_t t = tile * 32u + lane;
+        for (uint32_t tile = blockIdx.x * (NP_BLOCK / 32) + warp; tile * a.lanes < a.n; tile += nwarps) {
+            const uint32_t t = uint32_t(lane) < a.lanes ? tile * a.lanes + lane : a.n;
             const uint32_t i = (a.perm && t < a.n) ? a.perm[t] : t;
             int combo = 0;   // box-box, or a pair whose check fails in process_pair
             if (t < a.n) {
@@ -415,8 +415,10 @@ __global__ void __launch_bounds__(NP_BLOCK, MinBlocks<ALGO>::value) narrowphase_
             atomicAdd(&a.mlp_stats[1], (unsigned long long)confirmed);
         }
     } else {
-        const uint32_t stride = gridDim.x * blockDim.x;
-        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += stride)
+        const uint32_t lane = threadIdx.x & 31u;
+        if (lane >= a.lanes) return;
+        const uint32_t stride = gridDim.x * (NP_BLOCK / 32) * a.lanes;
+        for (uint32_t i = (blockIdx.x * (NP_BLOCK / 32) + (threadIdx.x >> 5)) * a.lanes + lane; i < a.n; i += stride)
             process_pair<ALGO>(a, i, &s_box, mesh_words);
     }
 }
@@ -490,9 +492,28 @@ __global__ void __launch_bounds__(NP_BLOCK, NP_MIN_BLOCKS) narrowphase_tri_kerne
         }
         __syncthreads();
     }
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += stride)
+    const uint32_t lane = threadIdx.x & 31u;
+    if (lane >= a.lanes) return;
+    const uint32_t stride = gridDim.x * (NP_BLOCK / 32) * a.lanes;
+    for (uint32_t i = (blockIdx.x * (NP_BLOCK / 32) + (threadIdx.x >> 5)) * a.lanes + lane; i < a.n; i += stride)
         process_tri<ALGO>(a, i, &s_box, mesh_words);
+}
+
+// Pairs that one warp takes at once in the thread-per-pair kernels.  The pairs
+// of a warp take different paths (GJK steps, SAT exits, clipping), and the
+// warp's time is that of all of them together; so a batch that cannot fill the
+// device spreads over more warps with fewer pairs each, up to WARPS_PER_SM
+// (two a scheduler), and a large one fills its warps.  42 capsule-box pairs
+// 52 -> 41 us, ~1,000 box-box pairs of a terrain world 68 -> 34 us.
+constexpr uint32_t WARPS_PER_SM = 8;
+static uint32_t pairs_per_warp(uint32_t n, int num_sms) {
+    const uint32_t warps = uint32_t(num_sms) * WARPS_PER_SM;
+    const uint32_t p = (n + warps - 1) / warps;
+    return p < 32u ? p : 32u;
+}
+static uint32_t blocks_for(uint32_t n, uint32_t lanes) {
+    const uint32_t per_block = (NP_BLOCK / 32) * lanes;
+    return (n + per_block - 1) / per_block;
 }
 
 cudaError_t launch_narrowphase_tri(int algo, const NpArgs& args, int num_sms, cudaStream_t stream) {
@@ -513,10 +534,12 @@ cudaError_t launch_narrowphase_tri(int algo, const NpArgs& args, int num_sms, cu
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
     }
-    const uint32_t blocks_needed = (args.n + NP_BLOCK - 1) / NP_BLOCK;
+    NpArgs a = args;
+    a.lanes = pairs_per_warp(args.n, num_sms);
+    const uint32_t blocks_needed = blocks_for(args.n, a.lanes);
     const uint32_t cap = uint32_t(num_sms) * 16u;
     const uint32_t blocks = blocks_needed < cap ? blocks_needed : cap;
-    void* params[] = {const_cast<NpArgs*>(&args)};
+    void* params[] = {&a};
     return cudaLaunchKernel(k, dim3(blocks), dim3(NP_BLOCK), params, smem, stream);
 }
 
@@ -528,23 +551,6 @@ cudaError_t launch_narrowphase_tri(int algo, const NpArgs& args, int num_sms, cu
 // the results do not depend on it; the order inside a class follows the
 // atomics.  Rank of class c: 15 first, then 0..14.
 __device__ __forceinline__ uint32_t class_rank(uint32_t c) { return c >= 15u ? 0u : c + 1u; }
-__global__ void __launch_bounds__(256) partition_count(const NpArgs a, const uint8_t* __restrict__ cls,
-                                                       uint32_t* __restrict__ counts) {
-    const uint32_t n = a.n;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t r = i < n ? class_rank(cls[i]) : 16u;
-    // a batch with a convex mesh keeps its order: its pairs go one per warp,
-    // where grouping gains nothing
-    if (i < n) {
-        const int32_t i1 = a.shape1[i], i2 = a.shape2[i];
-        const bool box = uint32_t(i1) < a.nb_shapes && uint32_t(i2) < a.nb_shapes &&
-                         load_shape(a.shapes, i1).kind == RP3DG_SHAPE_BOX && load_shape(a.shapes, i2).kind == RP3DG_SHAPE_BOX;
-        if (!box) counts[31] = 1u;
-    }
-    const uint32_t peers = __match_any_sync(0xffffffffu, r);
-    const uint32_t lane = threadIdx.x & 31u;
-    if (r < 16u && (peers & ((1u << lane) - 1u)) == 0) atomicAdd(counts + r, uint32_t(__popc(peers)));
-}
 __global__ void __launch_bounds__(256) partition_scatter(const uint8_t* __restrict__ cls, uint32_t n,
                                                          uint32_t* __restrict__ counts, uint32_t* __restrict__ perm) {
     __shared__ uint32_t base[16];
@@ -570,13 +576,8 @@ __global__ void __launch_bounds__(256) partition_scatter(const uint8_t* __restri
 }
 cudaError_t launch_partition_by_class(const NpArgs& a, const uint8_t* cls, uint32_t* counts, uint32_t* perm,
                                       cudaStream_t stream) {
-    const uint32_t n = a.n;
-    if (n == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(counts, 0, 32 * sizeof(uint32_t), stream);
-    if (e != cudaSuccess) return e;
-    const uint32_t nb = (n + 255) / 256;
-    partition_count<<<nb, 256, 0, stream>>>(a, cls, counts);
-    partition_scatter<<<nb, 256, 0, stream>>>(cls, n, counts, perm);
+    if (a.n == 0) return cudaSuccess;
+    partition_scatter<<<(a.n + 255) / 256, 256, 0, stream>>>(cls, a.n, counts, perm);
     return cudaGetLastError();
 }
 
@@ -592,17 +593,18 @@ cudaError_t launch_partition_by_class(const NpArgs& a, const uint8_t* cls, uint3
 //     features and runs the MLP on the bf16 tensor cores (mma.sync
 //     m16n8k16, 112 MMAs per tile) and writes each pair's proposed feature
 //     (15 = none) to `proposals`, which the SAT kernels test exactly.
-// `key` receives the order class that partition_count / partition_scatter
-// sort by (class 15 first, then 0..14): certainly colliding (15), uncertain
-// (0), certainly separated (1) and mesh pairs (2); the learned proposals do
-// not change the order.  Only the order in which the pairs are processed
+// `key` receives the order class that partition_scatter sorts by (class 15
+// first, then 0..14): certainly colliding (15), uncertain (0), certainly
+// separated (1) and mesh pairs (2); counts the pairs of each class.  The
+// learned proposals do not change the order.  Only the order in which the pairs are processed
 // depends on the key.
+constexpr uint8_t NOT_BOXES = 2;
 RD uint8_t box_pair_class(const NpArgs& a, uint32_t i) {
     if (i >= a.n) return 0;
     const int32_t i1 = a.shape1[i], i2 = a.shape2[i];
-    if (uint32_t(i1) >= a.nb_shapes || uint32_t(i2) >= a.nb_shapes) return 0;
+    if (uint32_t(i1) >= a.nb_shapes || uint32_t(i2) >= a.nb_shapes) return NOT_BOXES;
     const ShapeRec r1 = load_shape(a.shapes, i1), r2 = load_shape(a.shapes, i2);
-    if (r1.kind != RP3DG_SHAPE_BOX || r2.kind != RP3DG_SHAPE_BOX) return 2;   // a mesh pair: its own tiles
+    if (r1.kind != RP3DG_SHAPE_BOX || r2.kind != RP3DG_SHAPE_BOX) return NOT_BOXES;   // a mesh pair: its own tiles
     const float4 p1 = a.pos1[i], p2 = a.pos2[i];
     const float dx = p2.x - p1.x, dy = p2.y - p1.y, dz = p2.z - p1.z;
     const float d2 = dx * dx + dy * dy + dz * dz;
@@ -613,7 +615,8 @@ RD uint8_t box_pair_class(const NpArgs& a, uint32_t i) {
 }
 
 __global__ void __launch_bounds__(NP_BLOCK) classify_pairs(const NpArgs a, uint8_t* __restrict__ key,
-                                                           uint8_t* __restrict__ proposals) {
+                                                           uint8_t* __restrict__ proposals,
+                                                           uint32_t* __restrict__ counts) {
     __shared__ float s_feat[NP_BLOCK / 32][32][MLP_KPAD];
     __shared__ uint32_t s_cls[NP_BLOCK / 32][32];
     __shared__ BoxTables s_box;
@@ -659,6 +662,12 @@ __global__ void __launch_bounds__(NP_BLOCK) classify_pairs(const NpArgs a, uint8
             if (i < a.n) proposals[i] = uint8_t(c);
         }
         if (i < a.n) key[i] = k;
+        // a batch with a convex mesh keeps its order: its pairs go one per
+        // warp, where grouping gains nothing
+        if (i < a.n && geo == NOT_BOXES) counts[31] = 1u;
+        const uint32_t r = i < a.n ? class_rank(k) : 16u;
+        const uint32_t peers = __match_any_sync(FULL_MASK, r);
+        if (r < 16u && (peers & ((1u << lane) - 1u)) == 0) atomicAdd(counts + r, uint32_t(__popc(peers)));
     }
 }
 
@@ -708,12 +717,14 @@ cudaError_t launch_compact_contacts(const CompactArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_classify_pairs(const NpArgs& args, uint8_t* key, uint8_t* proposals, int num_sms,
+cudaError_t launch_classify_pairs(const NpArgs& args, uint8_t* key, uint8_t* proposals, uint32_t* counts, int num_sms,
                                   cudaStream_t stream) {
     if (args.n == 0) return cudaSuccess;
+    cudaError_t e = cudaMemsetAsync(counts, 0, 32 * sizeof(uint32_t), stream);
+    if (e != cudaSuccess) return e;
     const uint32_t blocks_needed = (args.n + NP_BLOCK - 1) / NP_BLOCK;
     const uint32_t cap = uint32_t(num_sms) * 16u;
-    classify_pairs<<<blocks_needed < cap ? blocks_needed : cap, NP_BLOCK, 0, stream>>>(args, key, proposals);
+    classify_pairs<<<blocks_needed < cap ? blocks_needed : cap, NP_BLOCK, 0, stream>>>(args, key, proposals, counts);
     return cudaGetLastError();
 }
 
@@ -815,8 +826,10 @@ static cudaError_t launch_one(int algo, const NpArgs& args, int num_sms, cudaStr
         }
         lc.smem = smem;
     }
-    // a warp-per-pair launch can use a warp per pair (4 per CTA), the others a thread
-    const uint32_t blocks_needed = warp_list ? (args.n + 3) / 4 : (args.n + NP_BLOCK - 1) / NP_BLOCK;
+    // a warp-per-pair launch can use a warp per pair (4 per CTA), the others pairs_per_warp
+    NpArgs a = args;
+    a.lanes = pairs_per_warp(args.n, num_sms);
+    const uint32_t blocks_needed = warp_list ? (args.n + 3) / 4 : blocks_for(args.n, a.lanes);
     // Enough CTAs to fill every SM several times; the grid-stride loop covers the rest.
     const uint32_t cap = uint32_t(num_sms) * 16u;
     uint32_t blocks = blocks_needed < cap ? blocks_needed : cap;
@@ -825,7 +838,7 @@ static cudaError_t launch_one(int algo, const NpArgs& args, int num_sms, cudaStr
         const uint32_t resident = uint32_t(num_sms) * uint32_t(lc.per_sm > 0 ? lc.per_sm : 1);
         blocks = blocks_needed < resident ? blocks_needed : resident;
     }
-    void* params[] = {const_cast<NpArgs*>(&args)};
+    void* params[] = {&a};
     return cudaLaunchKernel(k, dim3(blocks), dim3(NP_BLOCK), params, smem, stream);
 }
 

@@ -15,6 +15,7 @@ constexpr uint32_t MESH_STAGE_MAX_BYTES = 108 * 1024;
 
 struct NpArgs {
     uint32_t n;
+    uint32_t lanes;   // pairs a warp takes at once (set by the launch, see pairs_per_warp)
     uint32_t nb_shapes;
     uint32_t* error;  // device word: bit 0 = a pair named a shape outside the table
     uint32_t max_contacts;
@@ -77,16 +78,16 @@ struct CompactArgs {
 cudaError_t launch_compact_contacts(const CompactArgs& a, cudaStream_t s);
 // Launches the kernels of one algorithm batch; *launches receives how many.
 cudaError_t launch_narrowphase(int algo, const NpArgs& args, int num_sms, cudaStream_t stream, int* launches);
-// Pairs of an all-box polyhedron batch grouped by their learned class
-// (colliding first, then the proposed features): perm receives the order
-// (the identity when a pair holds a convex mesh); counts is scratch for 32
-// words.
+// Order key of every pair of a polyhedron batch and how many pairs have each
+// (counts: 32 words) and, with args.mlp set and proposals non-null, the
+// learned proposal of every pair (MLP inference on the tensor cores).
+cudaError_t launch_classify_pairs(const NpArgs& a, uint8_t* key, uint8_t* proposals, uint32_t* counts, int num_sms,
+                                  cudaStream_t stream);
+// Pairs of an all-box polyhedron batch grouped by the key of
+// launch_classify_pairs: perm receives the order (the identity when a pair
+// holds a convex mesh).
 cudaError_t launch_partition_by_class(const NpArgs& a, const uint8_t* cls, uint32_t* counts, uint32_t* perm,
                                       cudaStream_t stream);
-// Order key of every pair of a polyhedron batch (launch_partition_by_class
-// then sorts by it) and, with args.mlp set and proposals non-null, the
-// learned proposal of every pair (MLP inference on the tensor cores).
-cudaError_t launch_classify_pairs(const NpArgs& a, uint8_t* key, uint8_t* proposals, int num_sms, cudaStream_t stream);
 // Triangle tests of one algorithm batch (4, 5 or 6), one test per thread.
 cudaError_t launch_narrowphase_tri(int algo, const NpArgs& args, int num_sms, cudaStream_t stream);
 

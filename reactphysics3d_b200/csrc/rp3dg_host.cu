@@ -1131,22 +1131,22 @@ int rp3dg_narrowphase_device(rp3dg_ctx* ctx, int algorithm, const rp3dg_pair_bat
             if (e != cudaSuccess) { ctx->cap_proposals = 0; return cuda_fail(ctx, e, "cudaMalloc(proposals)"); }
             ctx->cap_proposals = c;
         }
-        uint8_t* key = ctx->d_proposals;
-        uint8_t* prop = ctx->d_proposals + p->n;
-        cudaError_t e = rp3dg::launch_classify_pairs(a, key, learned ? prop : nullptr, ctx->num_sms, ctx->stream);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "pair classes");
-        ctx->launches++;
-        if (learned) a.proposals = prop;
         // tiles of one learned class each (the order only, not the results)
         if (p->n > ctx->cap_perm) {
             const uint32_t c = std::max(p->n, 2 * ctx->cap_perm);
             cudaFree(ctx->d_perm);
             ctx->d_perm = nullptr;
-            e = cudaMalloc(&ctx->d_perm, (size_t(c) + 32) * sizeof(uint32_t));
+            cudaError_t e = cudaMalloc(&ctx->d_perm, (size_t(c) + 32) * sizeof(uint32_t));
             if (e != cudaSuccess) { ctx->cap_perm = 0; return cuda_fail(ctx, e, "cudaMalloc(pair order)"); }
             ctx->cap_perm = c;
         }
-        e = rp3dg::launch_partition_by_class(a, key, ctx->d_perm + p->n, ctx->d_perm, ctx->stream);
+        uint8_t* key = ctx->d_proposals;
+        uint8_t* prop = ctx->d_proposals + p->n;
+        uint32_t* counts = ctx->d_perm + p->n;
+        cudaError_t e = rp3dg::launch_classify_pairs(a, key, learned ? prop : nullptr, counts, ctx->num_sms, ctx->stream);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "pair classes");
+        if (learned) a.proposals = prop;
+        e = rp3dg::launch_partition_by_class(a, key, counts, ctx->d_perm, ctx->stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "pair grouping");
         ctx->launches += 2;
         a.perm = ctx->d_perm;

@@ -39,7 +39,10 @@ static_assert(sizeof(MeshHdr) == 64, "MeshHdr layout");
 //                           axis k, negative when negD is set
 //   [1] = m | (negC << 2):  c = -normal(e.face) lies on axis m
 //   [2] = n | (negD2 << 2): d = -normal(twin.face) lies on axis n
-struct BoxTables {
+struct alignas(16) BoxTables {
+    // Per even half-edge: the bits that box_edge_bits() must all have for an
+    // edge of the other polyhedron to pass the Gauss-map test against it.
+    uint32_t edge_need[12];
     uint8_t edges[24][4];  // vertex, twin, face, next
     uint8_t face_verts[24];
     uint8_t face_edge[6];
@@ -51,9 +54,6 @@ struct BoxTables {
     uint8_t tri_edges[6][4];   // vertex, twin, face, next
     uint8_t tri_face_edge[2];
     uint8_t pad2[2];
-    // Per even half-edge: the bits that box_edge_bits() must all have for an
-    // edge of the other polyhedron to pass the Gauss-map test against it.
-    uint32_t edge_need[12];
 };
 
 // Steps of the reference's narrow-phase code paths, counted per batch by the
