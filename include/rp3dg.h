@@ -155,6 +155,11 @@ void rp3dg_destroy(rp3dg_ctx* ctx);
 const char* rp3dg_last_error(const rp3dg_ctx* ctx);
 /* cudaStream_t of the context, as void* (for callers that order work). */
 void* rp3dg_stream(rp3dg_ctx* ctx);
+/* Order the context's stream against another stream of its device (a
+ * cudaStream_t as void*): with out == 0 the context's stream waits for the
+ * work queued on `stream` so far, with out != 0 the other way round.
+ * Nothing to do when they are the same stream.  May be captured. */
+int rp3dg_order_streams(rp3dg_ctx* ctx, void* stream, int out);
 int rp3dg_synchronize(rp3dg_ctx* ctx);
 
 /* ---- shapes (immutable after creation) -------------------------------- */

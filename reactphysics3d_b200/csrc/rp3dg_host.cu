@@ -14,6 +14,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -213,6 +214,8 @@ struct rp3dg_ctx {
     int num_sms = 148;
     int smem_optin = 0;   // cudaDevAttrMaxSharedMemoryPerBlockOptin
     cudaStream_t stream = nullptr;
+    cudaEvent_t order_event = nullptr;   // rp3dg_order_streams
+    std::mutex order_mutex;
     std::string err;
     uint64_t launches = 0;
     // shapes
@@ -485,6 +488,7 @@ void rp3dg_destroy(rp3dg_ctx* ctx) {
     cudaFree(ctx->d_arena);
     cudaFree(ctx->d_stage);
     cudaFree(ctx->d_istage);
+    if (ctx->order_event) cudaEventDestroy(ctx->order_event);
     if (ctx->s_up) cudaStreamDestroy(ctx->s_up);
     if (ctx->s_pub) cudaStreamDestroy(ctx->s_pub);
     if (ctx->s_rec) cudaStreamDestroy(ctx->s_rec);
@@ -518,6 +522,21 @@ void rp3dg_destroy(rp3dg_ctx* ctx) {
 const char* rp3dg_last_error(const rp3dg_ctx* ctx) { return ctx ? ctx->err.c_str() : "null context"; }
 
 void* rp3dg_stream(rp3dg_ctx* ctx) { return ctx ? static_cast<void*>(ctx->stream) : nullptr; }
+
+int rp3dg_order_streams(rp3dg_ctx* ctx, void* stream, int out) {
+    if (!ctx) return RP3DG_EINVAL;
+    cudaStream_t other = static_cast<cudaStream_t>(stream);
+    if (other == ctx->stream) return 0;
+    // a wait takes the event's record of the moment it is queued, so one event
+    // serves every call, as long as no other thread records it in between
+    std::lock_guard<std::mutex> lock(ctx->order_mutex);
+    cudaSetDevice(ctx->device);
+    cudaError_t e = cudaSuccess;
+    if (!ctx->order_event) e = cudaEventCreateWithFlags(&ctx->order_event, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(ctx->order_event, out ? ctx->stream : other);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(out ? other : ctx->stream, ctx->order_event, 0);
+    return e == cudaSuccess ? 0 : cuda_fail(ctx, e, "order streams");
+}
 
 int rp3dg_synchronize(rp3dg_ctx* ctx) {
     if (!ctx) return RP3DG_EINVAL;

@@ -64,6 +64,7 @@ def load_library(path=LIB_PATH):
     L.rp3dg_last_error.restype = C.c_char_p
     L.rp3dg_stream.argtypes = [P]
     L.rp3dg_stream.restype = P
+    L.rp3dg_order_streams.argtypes = [P, P, C.c_int]
     L.rp3dg_synchronize.argtypes = [P]
     L.rp3dg_kernel_launches.argtypes = [P]
     L.rp3dg_kernel_launches.restype = C.c_uint64
@@ -159,9 +160,10 @@ class DevicePairs:
         self.cache = None if h.cache is None else t(h.cache.view(np.uint8).reshape(-1, 16))
 
     def struct(self):
-        p = lambda x: None if x is None else x.data_ptr()
-        return A.PairBatch(self.n, p(self.shape1), p(self.shape2), p(self.pos1), p(self.rot1), p(self.pos2),
-                           p(self.rot2), p(self.report), p(self.cache))
+        return A.PairBatch(self.n, self.shape1.data_ptr(), self.shape2.data_ptr(), self.pos1.data_ptr(),
+                           self.rot1.data_ptr(), self.pos2.data_ptr(), self.rot2.data_ptr(),
+                           None if self.report is None else self.report.data_ptr(),
+                           None if self.cache is None else self.cache.data_ptr())
 
     def host_cache(self):
         return None if self.cache is None else self.cache.cpu().numpy().reshape(-1).view(A.CACHE_DTYPE)
@@ -205,6 +207,7 @@ class Context:
             raise Rp3dgError(rc, "rp3dg_create failed (no CUDA device?)")
         self.h = h
         self.device = device
+        self._torch_ready = False
         self._shapes = None
 
     def close(self):
@@ -232,25 +235,25 @@ class Context:
             self._tstream = torch.cuda.ExternalStream(self.stream_ptr, device=f"cuda:{self.device}")
         return self._tstream
 
+    def _order(self, out):
+        # one native call: an event and a wait through torch's objects take
+        # several times as long on the host, and every call on device arrays
+        # does this twice
+        import torch
+        if not self._torch_ready:
+            torch.cuda.init()
+            self._torch_ready = True
+        self._check(self.lib.rp3dg_order_streams(self.h, torch._C._cuda_getCurrentRawStream(self.device), out))
+
     def order_in(self):
         """Make the context stream wait for work queued on torch's current
         stream (tensors just created or filled there)."""
-        import torch
-        cur = torch.cuda.current_stream(self.device)
-        if cur.cuda_stream != self.stream_ptr:
-            ev = torch.cuda.Event()
-            ev.record(cur)
-            self.torch_stream().wait_event(ev)
+        self._order(0)
 
     def order_out(self):
         """Make torch's current stream wait for the context stream (results
         read or reused there)."""
-        import torch
-        cur = torch.cuda.current_stream(self.device)
-        if cur.cuda_stream != self.stream_ptr:
-            ev = torch.cuda.Event()
-            ev.record(self.torch_stream())
-            cur.wait_event(ev)
+        self._order(1)
 
     def synchronize(self):
         self._check(self.lib.rp3dg_synchronize(self.h))
