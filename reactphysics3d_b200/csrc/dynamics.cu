@@ -615,7 +615,8 @@ RD void store_manifold(const DynArgs& a, uint32_t mi) {
 // results.
 //
 // 3a: one thread per island runs islands of up to small_max manifolds in
-//     the reference's order and queues the larger ones.
+//     the reference's order (none when the stage has few manifolds) and
+//     queues the larger ones.
 // 3b: persistent warps take the queued islands.  Lane 0 gives each manifold a
 //     level (1 + the highest level of an earlier manifold sharing a movable
 //     body) and sorts the island's manifolds by level; every pass (warm

@@ -279,8 +279,9 @@ struct ItemPoints {
 };
 
 __global__ void __launch_bounds__(128) hf_manifolds_kernel(const HfManifoldArgs a) {
-    const uint32_t ci = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ci >= a.n_items) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t ci = (blockIdx.x * 4u + (threadIdx.x >> 5)) * a.lanes + lane;
+    if (lane >= a.lanes || ci >= a.n_items) return;
     const uint32_t st = a.start[ci], cnt = a.start[ci + 1] - st;
     const int4 b = a.batch[ci];
     const uint32_t base = uint32_t(b.x) * MAXC, bn = uint32_t(b.y), first = st - uint32_t(b.x);
@@ -393,7 +394,7 @@ cudaError_t launch_hf_tests(const HfTestArgs& a, cudaStream_t s) {
 
 cudaError_t launch_hf_manifolds(const HfManifoldArgs& a, cudaStream_t s) {
     if (a.n_items == 0) return cudaSuccess;
-    hf_manifolds_kernel<<<(a.n_items + 127) / 128, 128, 0, s>>>(a);
+    hf_manifolds_kernel<<<(a.n_items + 4 * a.lanes - 1) / (4 * a.lanes), 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -78,6 +78,7 @@ struct HfTestArgs {
 
 struct HfManifoldArgs {
     uint32_t n_items;
+    uint32_t lanes;                // items a warp takes (items_per_warp)
     const int4* items;
     const uint32_t* start;
     const int4* batch;             // per item: x = first test of its algorithm batch, y = batch size

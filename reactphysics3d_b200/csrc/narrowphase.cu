@@ -499,18 +499,6 @@ __global__ void __launch_bounds__(NP_BLOCK, NP_MIN_BLOCKS) narrowphase_tri_kerne
         process_tri<ALGO>(a, i, &s_box, mesh_words);
 }
 
-// Pairs that one warp takes at once in the thread-per-pair kernels.  The pairs
-// of a warp take different paths (GJK steps, SAT exits, clipping), and the
-// warp's time is that of all of them together; so a batch that cannot fill the
-// device spreads over more warps with fewer pairs each, up to WARPS_PER_SM
-// (two a scheduler), and a large one fills its warps.  42 capsule-box pairs
-// 52 -> 41 us, ~1,000 box-box pairs of a terrain world 68 -> 34 us.
-constexpr uint32_t WARPS_PER_SM = 8;
-static uint32_t pairs_per_warp(uint32_t n, int num_sms) {
-    const uint32_t warps = uint32_t(num_sms) * WARPS_PER_SM;
-    const uint32_t p = (n + warps - 1) / warps;
-    return p < 32u ? p : 32u;
-}
 static uint32_t blocks_for(uint32_t n, uint32_t lanes) {
     const uint32_t per_block = (NP_BLOCK / 32) * lanes;
     return (n + per_block - 1) / per_block;
@@ -535,7 +523,7 @@ cudaError_t launch_narrowphase_tri(int algo, const NpArgs& args, int num_sms, cu
         if (e != cudaSuccess) return e;
     }
     NpArgs a = args;
-    a.lanes = pairs_per_warp(args.n, num_sms);
+    a.lanes = items_per_warp(args.n, num_sms);
     const uint32_t blocks_needed = blocks_for(args.n, a.lanes);
     const uint32_t cap = uint32_t(num_sms) * 16u;
     const uint32_t blocks = blocks_needed < cap ? blocks_needed : cap;
@@ -826,9 +814,9 @@ static cudaError_t launch_one(int algo, const NpArgs& args, int num_sms, cudaStr
         }
         lc.smem = smem;
     }
-    // a warp-per-pair launch can use a warp per pair (4 per CTA), the others pairs_per_warp
+    // a warp-per-pair launch can use a warp per pair (4 per CTA), the others items_per_warp
     NpArgs a = args;
-    a.lanes = pairs_per_warp(args.n, num_sms);
+    a.lanes = items_per_warp(args.n, num_sms);
     const uint32_t blocks_needed = warp_list ? (args.n + 3) / 4 : blocks_for(args.n, a.lanes);
     // Enough CTAs to fill every SM several times; the grid-stride loop covers the rest.
     const uint32_t cap = uint32_t(num_sms) * 16u;

@@ -15,7 +15,7 @@ constexpr uint32_t MESH_STAGE_MAX_BYTES = 108 * 1024;
 
 struct NpArgs {
     uint32_t n;
-    uint32_t lanes;   // pairs a warp takes at once (set by the launch, see pairs_per_warp)
+    uint32_t lanes;   // pairs a warp takes at once (set by the launch, see items_per_warp)
     uint32_t nb_shapes;
     uint32_t* error;  // device word: bit 0 = a pair named a shape outside the table
     uint32_t max_contacts;

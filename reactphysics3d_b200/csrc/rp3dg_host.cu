@@ -2024,7 +2024,12 @@ int dynamics_step_flags(rp3dg_ctx* ctx, const rp3dg_dynamics_params* pr, const r
     const rp3dg::DynTuning tdef{};
     const rp3dg::DynTuning& tn = tune ? *tune : tdef;
     a.large_ctas = uint32_t(ctx->num_sms) * (tn.large_per_sm ? tn.large_per_sm : 1u);
-    a.small_max = tn.small_max;
+    // A thread an island saves warps, not time: with few manifolds every island
+    // is faster on a warp of kernel 3b.  Warps / threads, us a stage: 192
+    // worlds of 92 manifolds (20 a warp) 822 / 847, 384 worlds 889 / 877,
+    // 4,096 worlds 2,642 / 1,797.
+    const uint32_t warps = a.large_ctas * uint32_t(rp3dg::LARGE_WARPS);
+    a.small_max = a.nm <= 24u * warps ? 0u : tn.small_max;
     a.giant_min = tn.giant_min;
     a.giant_ctas = uint32_t(ctx->num_sms);
     // the opt-in maximum less room for the kernel's static shared memory

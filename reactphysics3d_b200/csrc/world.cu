@@ -3062,6 +3062,7 @@ int update_group(Group* g, float dt) {
         }
         HfManifoldArgs ma;
         ma.n_items = CI;
+        ma.lanes = rp3dg::items_per_warp(CI, rp3dg::get_num_sms(ctx));
         ma.items = g->d_hitems;
         ma.start = g->d_hstart;
         ma.batch = g->d_hbatch;
