@@ -31,8 +31,8 @@ namespace rp3dg {
 
 // Internal kernel id: the per-thread half of the polyhedron schedule.
 constexpr int ALGO_POLY_PER_THREAD = 7;
-// Internal kernel ids of the warp-per-pair launches, plus the COMBO_*.
-constexpr int WARP_KERNEL = 8, WARP_KERNEL_STAGED = 12;
+// Internal kernel ids of the warp-per-pair launches, plus their mask.
+constexpr int WARP_KERNEL = 8, WARP_KERNEL_STAGED = 16;
 constexpr int NP_MIN_BLOCKS = RP3DG_NP_MIN_BLOCKS;
 constexpr int NP_MIN_BLOCKS_POLY_WARP = RP3DG_NP_MIN_BLOCKS_POLY_WARP;
 constexpr int NP_MIN_BLOCKS_MESH_WARP = 4;
@@ -282,13 +282,16 @@ constexpr int COMBO_MESH_BOX = 1, COMBO_BOX_MESH = 2, COMBO_MESH_MESH = 3;
 
 // Convex polyhedron vs convex polyhedron, one warp per pair, for pairs of
 // shape combination COMBO.
-template <int COMBO>
-struct ComboScratch { typedef WarpScratchMesh type; };
+// A warp-per-pair launch takes the pairs of the combinations in a mask (bit
+// COMBO - 1).
+constexpr int WARP_MESH_BOX = 1, WARP_MESH_SECOND = 6, WARP_ALL = 7;
+template <int MASK>
+struct MaskScratch { typedef WarpScratchMesh type; };
 template <>
-struct ComboScratch<COMBO_MESH_BOX> { typedef WarpScratch type; };
-template <int COMBO>
+struct MaskScratch<WARP_MESH_BOX> { typedef WarpScratch type; };
+template <int COMBO, class Scratch>
 RD uint32_t process_pair_warp(const NpArgs& a, uint32_t i, int lane, const BoxTables* box, const uint32_t* mesh_words,
-                              typename ComboScratch<COMBO>::type& stage, uint32_t proposal) {
+                              Scratch& stage, uint32_t proposal) {
     const int32_t i1 = a.shape1[i], i2 = a.shape2[i];
     if (uint32_t(i1) >= a.nb_shapes || uint32_t(i2) >= a.nb_shapes) {
         if (lane == 0) {
@@ -423,7 +426,26 @@ __global__ void __launch_bounds__(NP_BLOCK, MinBlocks<ALGO>::value) narrowphase_
     }
 }
 
-// The pairs with a convex mesh of one shape combination, listed by the
+template <int COMBO, class Scratch>
+RD void warp_list(const NpArgs& a, int lane, const BoxTables* box, const uint32_t* mesh_words, Scratch& ws,
+                  uint32_t& tested, uint32_t& confirmed) {
+    const uint32_t total = __ldcg(a.work + (COMBO - 1));
+    const uint32_t* list = a.plist + size_t(COMBO - 1) * a.n;
+    while (total != 0) {
+        uint32_t k = 0;
+        if (lane == 0) k = atomicAdd(a.work + 3 + (COMBO - 1), 1u);
+        k = __shfl_sync(FULL_MASK, k, 0);
+        if (k >= total) break;
+        const uint32_t i = list[k];
+        uint32_t proposal = a.proposals ? uint32_t(a.proposals[i]) : uint32_t(MLP_NO_PROPOSAL);
+        if (proposal >= MLP_OUT) proposal = MLP_NO_PROPOSAL;
+        const uint32_t r = process_pair_warp<COMBO>(a, i, lane, box, mesh_words, ws, proposal);
+        tested += r & 1u;
+        confirmed += (r >> 1) & 1u;
+        __syncwarp();
+    }
+}
+// The pairs with a convex mesh of the combinations in MASK, listed by the
 // thread-per-pair launch: persistent warps take them one at a time (so the
 // launch ends within one pair's time of its average), faces over lanes
 // (ballot / arg-min), the edge pairs that can pass the Gauss-map test from bit
@@ -435,15 +457,22 @@ __global__ void __launch_bounds__(NP_BLOCK, MinBlocks<ALGO>::value) narrowphase_
 // to MESH_STAGE_MAX_BYTES).  A parameter and not a run-time choice of the
 // pointer, so that the compiler knows the address space: 265 -> 231 us for
 // 20,011 hull-hull pairs.
-template <int COMBO, bool STAGED>
-__global__ void __launch_bounds__(NP_BLOCK, COMBO == COMBO_MESH_BOX ? NP_MIN_BLOCKS_POLY_WARP : NP_MIN_BLOCKS_MESH_WARP)
+// MASK: one launch for all combinations of a small batch, two for a large one
+// (mesh-box with its smaller scratch and fifth CTA, and the others): each
+// launch with nothing to do costs its 2-3 us all the same.  42 hull-box and 42
+// box-box pairs among five other batches 136 -> 128 us, 100,003 box-box pairs
+// 77.0 -> 72.6 us against a launch per combination.
+template <int MASK, bool STAGED>
+__global__ void __launch_bounds__(NP_BLOCK, MASK == WARP_MESH_BOX ? NP_MIN_BLOCKS_POLY_WARP : NP_MIN_BLOCKS_MESH_WARP)
     narrowphase_warp_kernel(const NpArgs a) {
     extern __shared__ __align__(16) uint32_t s_mesh[];
     __shared__ BoxTables s_box;
-    typedef typename ComboScratch<COMBO>::type Scratch;
+    typedef typename MaskScratch<MASK>::type Scratch;
     __shared__ __align__(16) Scratch s_stage[NP_BLOCK / 32];
-    const uint32_t total = __ldcg(a.work + (COMBO - 1));
-    if (total == 0) return;   // uniform: nothing of this combination in the batch
+    uint32_t any = 0;
+    if constexpr ((MASK & 1) != 0) any |= __ldcg(a.work);
+    if constexpr ((MASK & 6) != 0) any |= __ldcg(a.work + 1) | __ldcg(a.work + 2);
+    if (any == 0) return;   // uniform: nothing of these combinations in the batch
     const uint32_t* mesh_words = STAGED ? s_mesh : a.mesh_words;
     {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(&c_box_tables);
@@ -455,22 +484,10 @@ __global__ void __launch_bounds__(NP_BLOCK, COMBO == COMBO_MESH_BOX ? NP_MIN_BLO
         __syncthreads();
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    Scratch& ws = s_stage[warp];
-    const uint32_t* list = a.plist + size_t(COMBO - 1) * a.n;
     uint32_t tested = 0, confirmed = 0;
-    for (;;) {
-        uint32_t k = 0;
-        if (lane == 0) k = atomicAdd(a.work + 3 + (COMBO - 1), 1u);
-        k = __shfl_sync(FULL_MASK, k, 0);
-        if (k >= total) break;
-        const uint32_t i = list[k];
-        uint32_t proposal = a.proposals ? uint32_t(a.proposals[i]) : uint32_t(MLP_NO_PROPOSAL);
-        if (proposal >= MLP_OUT) proposal = MLP_NO_PROPOSAL;
-        const uint32_t r = process_pair_warp<COMBO>(a, i, lane, &s_box, mesh_words, ws, proposal);
-        tested += r & 1u;
-        confirmed += (r >> 1) & 1u;
-        __syncwarp();
-    }
+    if constexpr ((MASK & 4) != 0) warp_list<COMBO_MESH_MESH>(a, lane, &s_box, mesh_words, s_stage[warp], tested, confirmed);
+    if constexpr ((MASK & 2) != 0) warp_list<COMBO_BOX_MESH>(a, lane, &s_box, mesh_words, s_stage[warp], tested, confirmed);
+    if constexpr ((MASK & 1) != 0) warp_list<COMBO_MESH_BOX>(a, lane, &s_box, mesh_words, s_stage[warp], tested, confirmed);
     if (a.mlp_stats && lane == 0 && tested) {
         atomicAdd(&a.mlp_stats[0], (unsigned long long)tested);
         atomicAdd(&a.mlp_stats[1], (unsigned long long)confirmed);
@@ -723,12 +740,12 @@ static const void* kernel_ptr(int algo) {
         case 3: return reinterpret_cast<const void*>(&narrowphase_kernel<3>);
         case 4: return reinterpret_cast<const void*>(&narrowphase_kernel<4>);
         case 5: return reinterpret_cast<const void*>(&narrowphase_kernel<5>);
-        case WARP_KERNEL + COMBO_MESH_BOX: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_MESH_BOX, false>);
-        case WARP_KERNEL + COMBO_BOX_MESH: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_BOX_MESH, false>);
-        case WARP_KERNEL + COMBO_MESH_MESH: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_MESH_MESH, false>);
-        case WARP_KERNEL_STAGED + COMBO_MESH_BOX: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_MESH_BOX, true>);
-        case WARP_KERNEL_STAGED + COMBO_BOX_MESH: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_BOX_MESH, true>);
-        case WARP_KERNEL_STAGED + COMBO_MESH_MESH: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<COMBO_MESH_MESH, true>);
+        case WARP_KERNEL + WARP_MESH_BOX: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<WARP_MESH_BOX, false>);
+        case WARP_KERNEL + WARP_MESH_SECOND: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<WARP_MESH_SECOND, false>);
+        case WARP_KERNEL + WARP_ALL: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<WARP_ALL, false>);
+        case WARP_KERNEL_STAGED + WARP_MESH_BOX: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<WARP_MESH_BOX, true>);
+        case WARP_KERNEL_STAGED + WARP_MESH_SECOND: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<WARP_MESH_SECOND, true>);
+        case WARP_KERNEL_STAGED + WARP_ALL: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<WARP_ALL, true>);
         case ALGO_POLY_PER_THREAD: return reinterpret_cast<const void*>(&narrowphase_kernel<ALGO_POLY_PER_THREAD>);
     }
     return nullptr;
@@ -758,15 +775,20 @@ cudaError_t launch_narrowphase(int algo, const NpArgs& args, int num_sms, cudaSt
     if (args.n == 0) return cudaSuccess;
     if (algo == RP3DG_ALGO_CONVEX_POLYHEDRON_VS_CONVEX_POLYHEDRON) {
         // the thread-per-pair launch (box-box pairs, and the lists of the
-        // mesh pairs), then one warp-per-pair launch per shape combination
+        // mesh pairs), then the warp-per-pair launches of those
         if (!args.plist || !args.work) return cudaErrorInvalidValue;
         cudaError_t e = cudaMemsetAsync(args.work, 0, 6 * sizeof(uint32_t), stream);
         if (e != cudaSuccess) return e;
         e = launch_one(ALGO_POLY_PER_THREAD, args, num_sms, stream);
         if (e != cudaSuccess) return e;
         ++*launches;
-        for (int c = COMBO_MESH_BOX; c <= COMBO_MESH_MESH; c++) {
-            e = launch_one((args.stage_mesh ? WARP_KERNEL_STAGED : WARP_KERNEL) + c, args, num_sms, stream);
+        const int base = args.stage_mesh ? WARP_KERNEL_STAGED : WARP_KERNEL;
+        // a batch that gives no warp a second pair gains nothing from the
+        // mesh-box kernel's fifth CTA: one launch for all combinations
+        const bool all = args.n <= uint32_t(num_sms) * uint32_t(NP_MIN_BLOCKS_MESH_WARP) * (NP_BLOCK / 32);
+        for (int mask : {all ? WARP_ALL : WARP_MESH_BOX, all ? 0 : WARP_MESH_SECOND}) {
+            if (mask == 0) break;
+            e = launch_one(base + mask, args, num_sms, stream);
             if (e != cudaSuccess) return e;
             ++*launches;
         }
@@ -791,8 +813,8 @@ static cudaError_t launch_one(int algo, const NpArgs& args, int num_sms, cudaStr
     if (!k) return cudaErrorInvalidValue;
     const bool warp_list = algo > WARP_KERNEL;
     size_t smem = (args.stage_mesh && algo != ALGO_POLY_PER_THREAD) ? size_t(args.mesh_nwords) * 4 : 0;
-    static thread_local LaunchCache cache[16];
-    LaunchCache& lc = cache[algo & 15];
+    static thread_local LaunchCache cache[32];
+    LaunchCache& lc = cache[algo & 31];
     cudaError_t e = cudaSuccess;
     if (!lc.known) {
         cudaFuncAttributes fa;

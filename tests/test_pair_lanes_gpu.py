@@ -43,3 +43,29 @@ def test_every_batch_size_matches_oracle(cuda_lib, port, per_warp):
                 getattr(part, f)[...] = getattr(exp, f)[:, :n]
             _assert_same(got, part, p.cache, full.cache[:n], f"{name} n={n}")
     ctx.close()
+
+
+@pytest.mark.parametrize("off", [-700, 0, 1, 2000])
+def test_mixed_mesh_combinations_match_oracle(cuda_lib, port, off):
+    """Hulls and boxes in every order in one batch, around the size (one pair a
+    resident warp) at which the combinations get launches of their own."""
+    port.lib.rp3do_reset()
+    _register_hulls(port)
+    ctx = engine.Context(0)
+    _register_hulls(ctx)
+    n = 16 * torch.cuda.get_device_properties(0).multi_processor_count + off
+    sc = scenes.narrowphase_scene(total_pairs=7 * n, seed=9, hull=edgecases.load_hull())
+    ctx.set_shapes(sc.shapes)
+    algo, pairs = sc.batches["hull_box"]
+    pairs = pairs.slice(0, n)
+    rng = np.random.default_rng(4)
+    hull, box, turn = pairs.shape1.copy(), pairs.shape2.copy(), rng.integers(0, 4, n)
+    pairs.shape1[:] = np.where(turn == 0, hull, np.where(turn == 1, box, np.where(turn == 2, hull, np.roll(box, 1))))
+    pairs.shape2[:] = np.where(turn == 0, box, np.where(turn == 1, hull, np.where(turn == 2, np.roll(hull, 1), box)))
+    a, b = pairs.slice(0, n), pairs.slice(0, n)
+    a.cache, b.cache = A.fresh_cache(n), A.fresh_cache(n)
+    exp, _ = port.narrowphase(algo, sc.shapes, a)
+    got = ctx.narrowphase_host(algo, b)
+    _assert_same(got, exp, b.cache, a.cache, f"n={n}")
+    assert len(np.unique(turn)) == 4 and exp.is_colliding.sum() > n // 10
+    ctx.close()
