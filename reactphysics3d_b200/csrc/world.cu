@@ -420,6 +420,7 @@ struct TreeReinsertArgs {
 // that fits is copied into shared memory before its first reinsertion and
 // back after the last (256 worlds of 20 to 200 bodies: 1,090 -> 772 us).
 constexpr int32_t REINSERT_STAGE_BYTES = 48 * 1024;
+constexpr size_t REINSERT_SM_BYTES = 228 * 1024;   // an SM's shared memory (1 KB of it reserved per CTA)
 __global__ void __launch_bounds__(32) world_tree_reinsert(const TreeReinsertArgs a) {
     extern __shared__ uint4 s_tree[];
     const uint32_t k = blockIdx.x;
@@ -2063,6 +2064,10 @@ int reinsert_on_device(Group* g, const uint8_t* moved, const float4* fmin, const
     a.stage_nodes = 0;   // the largest tree that fits sizes the stage
     for (int32_t n : g->tree_nodes)
         if (n <= fit) a.stage_nodes = std::max(a.stage_nodes, n);
+    // a world's chain is the kernel's time, so worlds that would wait for
+    // another's shared memory are better off in global memory, all at once
+    const size_t per_sm = REINSERT_SM_BYTES / (size_t(a.stage_nodes) * sizeof(TreeNode) + 1024);
+    if (nw > size_t(rp3dg::get_num_sms(g->ctx)) * per_sm) a.stage_nodes = 0;
     world_tree_reinsert<<<uint32_t(nw), 32, size_t(a.stage_nodes) * sizeof(TreeNode), g->stream>>>(a);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : wcuda(g, e, "tree reinsertion launch");
