@@ -1955,8 +1955,9 @@ __global__ void __launch_bounds__(GIANT_THREADS, 1) dyn_islands_giant(const DynA
             }
             giant_solve(a, m0, cnt, g, warp, lane, s_depth, s_nslots, s_p0);
         } else if (size_t(GIANT_LEVELS) * STREAM_RING * sizeof(StreamSlot) + GIANT_LEVELS * sizeof(int2) <= a.giant_smem) {
-            // streamed by dyn_islands_stream (queued at the back of giant_list)
-            if (threadIdx.x == 0) a.giant_list[a.ni - 1 - atomicAdd(a.counters + 5, 1u)] = is;
+            // streamed by dyn_islands_stream (giant_list may still hold untaken
+            // islands up to its end)
+            if (threadIdx.x == 0) a.stream_list[atomicAdd(a.counters + 5, 1u)] = is;
             __syncthreads();
             continue;
         } else if (warp == 0) {
@@ -1979,7 +1980,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) dyn_islands_stream(const Dy
         __syncthreads();
         const uint32_t k = s_island;
         if (k >= n_stream) break;
-        const uint32_t is = a.giant_list[a.ni - 1 - k];
+        const uint32_t is = a.stream_list[k];
         const uint32_t m0 = a.i_start[is], cnt = a.i_count[is];
         if (warp == 0) {
             const uint32_t depth = stream_schedule(a, m0, cnt, lane);

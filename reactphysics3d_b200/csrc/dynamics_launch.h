@@ -153,10 +153,11 @@ struct DynArgs {
     int32_t* body_slot;    // nb: shared-memory slot of each movable body (scratch)
     uint32_t* counters;    // [0] big islands queued (front of large_list), [1] islands taken, [2] others queued (back),
                            // [3] giant islands queued, [4] giant islands taken,
-                           // [5] streamed islands queued (back of giant_list), [6] streamed islands taken,
+                           // [5] streamed islands queued, [6] streamed islands taken,
                            // [7] giant islands offered to kernel 3b
     uint32_t* large_list;  // ni: queued islands
     uint32_t* giant_list;  // ni: islands for kernel 3c
+    uint32_t* stream_list; // ni: islands that do not fit kernel 3c's shared memory
     uint32_t large_ctas;   // grid of kernel 3b (persistent)
     uint32_t small_max;    // islands of up to this many manifolds: one thread each (kernel 3a)
     uint32_t giant_min;    // islands above this many manifolds: one CTA each (kernel 3c)

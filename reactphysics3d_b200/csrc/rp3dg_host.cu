@@ -1943,7 +1943,8 @@ int dynamics_step_flags(rp3dg_ctx* ctx, const rp3dg_dynamics_params* pr, const r
     const size_t off_cnt = off_bslot + al(size_t(b->n) * 4);
     const size_t off_list = off_cnt + 256;
     const size_t off_giant = off_list + al(size_t(is->n) * 4);
-    size_t need = off_giant + al(size_t(is->n) * 4) + 256;
+    const size_t off_stream = off_giant + al(size_t(is->n) * 4);
+    size_t need = off_stream + al(size_t(is->n) * 4) + 256;
     // graph-coloured solver scratch
     const bool colored = solver && solver->colored;
     const size_t o_cstart = need; if (colored) need += al((size_t(b->n) + 1) * 4);
@@ -2021,6 +2022,7 @@ int dynamics_step_flags(rp3dg_ctx* ctx, const rp3dg_dynamics_params* pr, const r
     a.counters = reinterpret_cast<uint32_t*>(s + off_cnt);
     a.large_list = reinterpret_cast<uint32_t*>(s + off_list);
     a.giant_list = reinterpret_cast<uint32_t*>(s + off_giant);
+    a.stream_list = reinterpret_cast<uint32_t*>(s + off_stream);
     const rp3dg::DynTuning tdef{};
     const rp3dg::DynTuning& tn = tune ? *tune : tdef;
     a.large_ctas = uint32_t(ctx->num_sms) * (tn.large_per_sm ? tn.large_per_sm : 1u);
