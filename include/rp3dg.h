@@ -908,7 +908,11 @@ int rp3dg_world_get_device_trees(rp3dg_world* world, int* enabled);
  * parameters (islands of up to small_max manifolds: one thread each; above
  * giant_min: one CTA each; persistent CTAs per SM of the warp-per-island
  * kernel: large_per_sm) only decide which kernel takes which island, so
- * results are identical for every candidate.  The tuning takes
+ * results are identical for every candidate.  small_max 8 and giant_min 256,
+ * the defaults, follow the step's islands (a step with few islands gives the
+ * small ones a warp each, one with no more islands above 64 manifolds than SMs
+ * gives each of those a CTA, one with more giant islands than SMs gives them a
+ * warp each); any other value is used as it stands.  The tuning takes
  * 9 x rounds steps. */
 int rp3dg_world_autotune(rp3dg_world* world, int rounds);
 /* out[0..3] = small_max, giant_min, large_per_sm, 1 while tuning. */
@@ -918,6 +922,10 @@ int rp3dg_world_get_phase_times(rp3dg_world* world, double* ms, uint32_t n);
 /* Number of kernels this context launched so far (instrumentation; a
  * convex-polyhedron batch takes two). */
 uint64_t rp3dg_kernel_launches(const rp3dg_ctx* ctx);
+/* Islands without joints that the context's last dynamics stage solved by a
+ * thread each, by a warp each, by a CTA each in shared memory, and streamed
+ * through global memory (instrumentation; waits for the stage). */
+int rp3dg_dynamics_routes(rp3dg_ctx* ctx, uint32_t* out);
 
 #ifdef __cplusplus
 }

@@ -660,6 +660,8 @@ __global__ void __launch_bounds__(128) dyn_islands_small(const DynArgs a) {
         else a.large_list[a.ni - 1 - atomicAdd(a.counters + 2, 1u)] = is;
         return;
     }
+    const unsigned here = __activemask();
+    if ((threadIdx.x & 31u) == uint32_t(__ffs(here)) - 1u) atomicAdd(a.counters + 8, uint32_t(__popc(here)));
     const uint32_t m1 = m0 + cnt;
     for (uint32_t mi = m0; mi < m1; mi++) {
         const int4 id = man_ids(a, mi);
@@ -1316,18 +1318,23 @@ RD void solve_global(const DynArgs& a, uint32_t m0, uint32_t cnt, uint32_t lane)
 // the giant ones: when there is a CTA for each of them.  A CTA takes a level
 // of up to 16 manifolds in one round (a warp four a round) and a chain's level
 // in 1,273-1,841 cycles (a warp 1,697-2,141).
-RD bool big_on_ctas(const DynArgs& a) { return a.giant_smem && a.counters[3] + a.counters[0] <= a.giant_ctas; }
+RD bool big_on_ctas(const DynArgs& a) {
+    return a.giant_auto && a.giant_smem && a.counters[3] + a.counters[0] <= a.giant_ctas;
+}
+// Whether the giant islands that fit a warp's stage go to kernel 3b: when there
+// are more of them than CTAs of kernel 3c (one each): 300 chains of 300
+// manifolds took 6.4 ms as CTAs (three rounds of 148), 2.7 ms as warps; 148 or
+// fewer are faster as CTAs.
+RD bool giants_on_warps(const DynArgs& a) { return a.giant_auto && a.counters[3] > a.giant_ctas; }
 
 __global__ void __launch_bounds__(LARGE_WARPS * 32, 2) dyn_islands_large(const DynArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WarpStage* st = reinterpret_cast<WarpStage*>(smem_raw + size_t(wid) * LARGE_WARP_SMEM);
-    // Giant islands that fit a warp's stage are taken here, the longest work
-    // first, when there are more of them than CTAs of kernel 3c (one each):
-    // 300 chains of 300 manifolds took 6.4 ms as CTAs (three rounds of 148),
-    // 2.7 ms as warps; 148 or fewer are faster as CTAs.
-    const uint32_t n_giant = a.counters[3];
-    if (n_giant > a.giant_ctas) {
+    uint32_t solved = 0;
+    // the longest work first
+    if (giants_on_warps(a)) {
+        const uint32_t n_giant = a.counters[3];
         for (;;) {
             uint32_t k = 0;
             if (lane == 0) k = atomicAdd(a.counters + 7, 1u);
@@ -1341,6 +1348,7 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32, 2) dyn_islands_large(const D
                 __syncwarp();
                 for (uint32_t j = lane; j < cnt; j += 32) store_manifold(a, m0 + j);
                 if (lane == 0) a.giant_list[k] = ISLAND_DONE;
+                solved++;
             }
             __syncwarp();
         }
@@ -1358,8 +1366,10 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32, 2) dyn_islands_large(const D
         else solve_global(a, m0, cnt, lane);
         __syncwarp();
         for (uint32_t j = lane; j < cnt; j += 32) store_manifold(a, m0 + j);
+        solved++;
         __syncwarp();
     }
+    if (lane == 0 && solved) atomicAdd(a.counters + 9, solved);
 }
 
 
@@ -1954,6 +1964,7 @@ __global__ void __launch_bounds__(GIANT_THREADS, 1) dyn_islands_giant(const DynA
                 giant_layout(a, cnt, uint32_t(int64_t(l.w) + int64_t(l.z) - int64_t(s_p0)), g);
             }
             giant_solve(a, m0, cnt, g, warp, lane, s_depth, s_nslots, s_p0);
+            if (threadIdx.x == 0) atomicAdd(a.counters + 10, 1u);
         } else if (size_t(GIANT_LEVELS) * STREAM_RING * sizeof(StreamSlot) + GIANT_LEVELS * sizeof(int2) <= a.giant_smem) {
             // streamed by dyn_islands_stream (giant_list may still hold untaken
             // islands up to its end)
@@ -2299,6 +2310,7 @@ cudaError_t launch_dynamics(const DynArgs& a, cudaStream_t s, uint64_t* launches
     // islands with joints, one thread each: giant_ctas is the number of SMs
     const uint32_t joint_lanes = items_per_warp(a.nji, int(a.giant_ctas));
     const uint32_t joint_blocks = (a.nji + 2 * joint_lanes - 1) / std::max(2 * joint_lanes, 1u);
+    if (a.ni) cudaMemsetAsync(a.counters, 0, DYN_COUNTERS * sizeof(uint32_t), s);
     if (a.nb) { dyn_bodies_pre<<<blocks(a.nb), 128, 0, s>>>(a); (*launches)++; }
     if (a.nm) { dyn_manifold_init<<<blocks(a.nm), 128, 0, s>>>(a); (*launches)++; }
     if (a.nj) { dyn_joints_init<<<blocks(a.nj), 128, 0, s>>>(a); (*launches)++; }
@@ -2309,7 +2321,6 @@ cudaError_t launch_dynamics(const DynArgs& a, cudaStream_t s, uint64_t* launches
     bool colored_done = false;
     if (a.colored && a.color && a.nj == 0 && a.nm) colored_done = colored_islands(a, s, launches);
     if (a.ni && !colored_done) {
-        cudaMemsetAsync(a.counters, 0, 8 * sizeof(uint32_t), s);
         dyn_islands_small<<<blocks(a.ni), 128, 0, s>>>(a);
         (*launches)++;
         const size_t smem = size_t(LARGE_WARPS) * LARGE_WARP_SMEM;

@@ -154,13 +154,15 @@ struct DynArgs {
     uint32_t* counters;    // [0] big islands queued (front of large_list), [1] islands taken, [2] others queued (back),
                            // [3] giant islands queued, [4] giant islands taken,
                            // [5] streamed islands queued, [6] streamed islands taken,
-                           // [7] giant islands offered to kernel 3b
+                           // [7] giant islands offered to kernel 3b,
+                           // islands solved so far: [8] by a thread, [9] by a warp, [10] by a CTA in shared memory
     uint32_t* large_list;  // ni: queued islands
     uint32_t* giant_list;  // ni: islands for kernel 3c
     uint32_t* stream_list; // ni: islands that do not fit kernel 3c's shared memory
     uint32_t large_ctas;   // grid of kernel 3b (persistent)
     uint32_t small_max;    // islands of up to this many manifolds: one thread each (kernel 3a)
     uint32_t giant_min;    // islands above this many manifolds: one CTA each (kernel 3c)
+    int32_t giant_auto;    // giant_min is the default, and big_on_ctas / giants_on_warps move islands across it
     // joints (nj = 0: none).  j_list holds this step's enabled joints island
     // by island, each island's ball-and-socket, fixed, hinge then slider
     // joints, each type in component order: record index, body 1 row, body 2 row, bit 0 / bit 1 =
@@ -204,9 +206,11 @@ struct DynJoints {
 
 // Scheduling of the islands over the kernels (results do not depend on it):
 // thread-per-island limit, one-CTA-per-island threshold and persistent CTAs
-// per SM of the warp-per-island kernel.
+// per SM of the warp-per-island kernel.  With small_auto / giant_auto the limit
+// follows the stage (DynArgs); without, it is used as it stands.
 struct DynTuning {
     uint32_t small_max = 8, giant_min = 256, large_per_sm = 2;
+    bool small_auto = true, giant_auto = true;
 };
 
 // Solver choice of a dynamics stage: the exact-order solver (the drop-in) or
@@ -216,6 +220,9 @@ struct DynSolver {
     int colored = 0;
     SolverStats* stats = nullptr;
 };
+
+// 32-bit words at DynArgs::counters.
+constexpr uint32_t DYN_COUNTERS = 11;
 
 // Launches the kernels in order on stream s; *launches counts them.
 cudaError_t launch_dynamics(const DynArgs& a, cudaStream_t s, uint64_t* launches);

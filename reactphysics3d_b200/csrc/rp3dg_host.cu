@@ -267,6 +267,7 @@ struct rp3dg_ctx {
     // dynamics stage: per-body velocity scratch and solver records
     void* d_dyn = nullptr;
     size_t cap_dyn = 0;
+    size_t dyn_counters = 0;   // offset of the last stage's counters in d_dyn (0: that stage had no islands)
     // staging buffers for rp3dg_dynamics_step_host
     void* d_dyn_stage = nullptr;
     size_t cap_dyn_stage = 0;
@@ -545,6 +546,19 @@ int rp3dg_synchronize(rp3dg_ctx* ctx) {
 }
 
 uint64_t rp3dg_kernel_launches(const rp3dg_ctx* ctx) { return ctx ? ctx->launches : 0; }
+
+int rp3dg_dynamics_routes(rp3dg_ctx* ctx, uint32_t* out) {
+    if (!ctx || !out) return RP3DG_EINVAL;
+    for (int k = 0; k < 4; k++) out[k] = 0;
+    if (!ctx->dyn_counters) return 0;
+    uint32_t c[rp3dg::DYN_COUNTERS];
+    cudaError_t e = cudaMemcpyAsync(c, static_cast<char*>(ctx->d_dyn) + ctx->dyn_counters, sizeof(c),
+                                    cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "read island routes");
+    out[0] = c[8]; out[1] = c[9]; out[2] = c[10]; out[3] = c[5];
+    return 0;
+}
 
 int rp3dg_device_errors(rp3dg_ctx* ctx, uint32_t* flags, int clear) {
     if (!ctx || !flags) return fail(ctx, RP3DG_EINVAL, "null argument");
@@ -2031,8 +2045,9 @@ int dynamics_step_flags(rp3dg_ctx* ctx, const rp3dg_dynamics_params* pr, const r
     // worlds of 92 manifolds (20 a warp) 822 / 847, 384 worlds 889 / 877,
     // 4,096 worlds 2,642 / 1,797.
     const uint32_t warps = a.large_ctas * uint32_t(rp3dg::LARGE_WARPS);
-    a.small_max = a.nm <= 24u * warps ? 0u : tn.small_max;
+    a.small_max = tn.small_auto && a.nm <= 24u * warps ? 0u : tn.small_max;
     a.giant_min = tn.giant_min;
+    a.giant_auto = tn.giant_auto ? 1 : 0;
     a.giant_ctas = uint32_t(ctx->num_sms);
     // the opt-in maximum less room for the kernel's static shared memory
     a.giant_smem = ctx->smem_optin > 2048 ? uint32_t(ctx->smem_optin - 1024) : 0u;
@@ -2050,6 +2065,7 @@ int dynamics_step_flags(rp3dg_ctx* ctx, const rp3dg_dynamics_params* pr, const r
         a.color = &cs;
     }
     a.stats = solver ? solver->stats : nullptr;
+    ctx->dyn_counters = a.ni ? off_cnt : 0;
     cudaError_t e = rp3dg::launch_dynamics(a, ctx->stream, &ctx->launches);
     return e == cudaSuccess ? 0 : cuda_fail(ctx, e, "dynamics launch");
 }

@@ -3402,12 +3402,18 @@ int update_group(Group* g, float dt) {
 
 // The candidates of one autotuner phase: the current scheduling with one
 // parameter varied (0: thread-per-island limit, 1: one-CTA-per-island
-// threshold, 2: warp-kernel CTAs per SM).
+// threshold, 2: warp-kernel CTAs per SM).  The default of a limit is the one
+// that follows the stage; the others run as they stand, so that every
+// candidate of a phase is a schedule of its own.  The default comes first: it
+// is kept when nothing is faster.
 std::vector<rp3dg::DynTuning> tuner_candidates(const rp3dg::DynTuning& base, int phase) {
     std::vector<rp3dg::DynTuning> c;
-    const uint32_t small[] = {4, 8, 16, 32}, giant[] = {128, 256, 512}, per_sm[] = {1, 2};
-    if (phase == 0) for (uint32_t v : small) { rp3dg::DynTuning t = base; t.small_max = v; c.push_back(t); }
-    if (phase == 1) for (uint32_t v : giant) { rp3dg::DynTuning t = base; t.giant_min = v; c.push_back(t); }
+    const rp3dg::DynTuning def{};
+    const uint32_t small[] = {def.small_max, 4, 16, 32}, giant[] = {def.giant_min, 128, 512}, per_sm[] = {1, 2};
+    if (phase == 0)
+        for (uint32_t v : small) { rp3dg::DynTuning t = base; t.small_max = v; t.small_auto = v == def.small_max; c.push_back(t); }
+    if (phase == 1)
+        for (uint32_t v : giant) { rp3dg::DynTuning t = base; t.giant_min = v; t.giant_auto = v == def.giant_min; c.push_back(t); }
     if (phase == 2) for (uint32_t v : per_sm) { rp3dg::DynTuning t = base; t.large_per_sm = v; c.push_back(t); }
     return c;
 }

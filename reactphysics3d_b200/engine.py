@@ -68,6 +68,7 @@ def load_library(path=LIB_PATH):
     L.rp3dg_synchronize.argtypes = [P]
     L.rp3dg_kernel_launches.argtypes = [P]
     L.rp3dg_kernel_launches.restype = C.c_uint64
+    L.rp3dg_dynamics_routes.argtypes = [P, P]
     L.rp3dg_create_convex_mesh.argtypes = [P, P, C.c_uint32, P, P, C.c_uint32, C.POINTER(C.c_int32)]
     L.rp3dg_create_convex_mesh_shape.argtypes = [P, C.c_int32, C.c_float, C.c_float, C.c_float,
                                                  C.POINTER(C.c_int32)]
@@ -265,6 +266,12 @@ class Context:
 
     def kernel_launches(self):
         return int(self.lib.rp3dg_kernel_launches(self.h))
+
+    def dynamics_routes(self):
+        """Islands of the last dynamics stage by the kernel that solved them."""
+        v = np.zeros(4, np.uint32)
+        self._check(self.lib.rp3dg_dynamics_routes(self.h, v.ctypes.data))
+        return dict(zip(("thread", "warp", "cta", "streamed"), map(int, v)))
 
     def create_convex_mesh(self, vertices, faces):
         v = np.ascontiguousarray(vertices, dtype=np.float32)
