@@ -144,10 +144,88 @@ RD bool is_fixed(const DynArgs& a, int32_t b) {
 
 RD float4 F4w(v3 a, float w) { return make_float4(a.x, a.y, a.z, w); }
 
+// ---- island sizes: which islands get a thread each -------------------------
+//
+// An island on a thread costs kernel 3a a chain of its manifolds, however many
+// islands there are; an island on a warp costs one of kernel 3b's warps its
+// time, and the warps share the islands.  A thread each pays when the warps
+// would have several small islands each, so the limit is chosen from the
+// stage's island sizes, by what both sides measured (four-point manifolds, 888
+// warps): a thread 21, 56, 91, 126, 266 us for 1, 2, 3, 4, 8 manifolds, a warp
+// 10, 17, 23, 28, 42 us an island.
+// 12,000 islands of one manifold: warps 208 us a stage, threads 97; 2,500
+// islands of eight: warps 206, threads 341; 192 captured worlds (6,976
+// islands, half of them of one manifold): limit 0 817, 1 804, 8 859; 4,096 of
+// them: 0 2,635, 4 1,846, 8 1,785.
+constexpr uint32_t BIG_ISLAND = 64;   // queued first: the longest islands start first
+constexpr uint32_t SIZE_CLASSES = 8;  // islands of 1 .. 8 manifolds by size
+enum IslandSizes { IS_MID = SIZE_CLASSES, IS_MID_MAX, IS_BIG, IS_BIG_SUM, IS_BIG_MAX, IS_WORDS };   // from counters[10]
+static_assert(10 + IS_WORDS == DYN_COUNTERS, "counters");
+
+RD uint32_t thread_us(uint32_t manifolds) { return 35u * manifolds - 14u; }
+RD uint32_t warp_us(uint32_t manifolds) {
+    return manifolds <= SIZE_CLASSES ? 7u + 5u * manifolds : 47u + (manifolds - SIZE_CLASSES) * 11u / 4u;
+}
+
+// Block `block` counts its 128 islands.
+RD void count_island_sizes(const DynArgs& a, uint32_t block) {
+    __shared__ uint32_t h[IS_WORDS];
+    if (threadIdx.x < IS_WORDS) h[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t is = block * 128u + threadIdx.x;
+    const uint32_t cnt = is < a.ni && !(a.i_jcount && a.i_jcount[is]) ? a.i_count[is] : 0u;
+    if (cnt != 0 && cnt <= a.nm) {
+        if (cnt <= SIZE_CLASSES) {
+            atomicAdd(h + cnt - 1, 1u);
+        } else if (cnt <= BIG_ISLAND) {
+            atomicAdd(h + IS_MID, warp_us(cnt));
+            atomicMax(h + IS_MID_MAX, warp_us(cnt));
+        } else {
+            atomicAdd(h + IS_BIG, 1u);
+            atomicAdd(h + IS_BIG_SUM, warp_us(cnt));
+            atomicMax(h + IS_BIG_MAX, warp_us(cnt));
+        }
+    }
+    __syncthreads();
+    const uint32_t k = threadIdx.x;
+    if (k < IS_WORDS && h[k]) {
+        if (k == IS_MID_MAX || k == IS_BIG_MAX) atomicMax(a.counters + 10 + k, h[k]);
+        else atomicAdd(a.counters + 10 + k, h[k]);
+    }
+}
+
+// The limit whose estimate is the lowest (of two alike the smaller); lane s of
+// a warp estimates limit s.
+RD uint32_t small_limit(const DynArgs& a, uint32_t lane) {
+    if (!a.small_auto) return a.small_max;
+    const uint32_t* h = a.counters + 10;
+    const uint32_t warps = a.large_ctas * uint32_t(LARGE_WARPS);
+    const bool big = h[IS_BIG] > a.giant_ctas;   // too many for a CTA each
+    uint32_t sum = h[IS_MID] + (big ? h[IS_BIG_SUM] : 0u), longest = h[IS_MID_MAX], top = 0;
+    if (big && h[IS_BIG_MAX] > longest) longest = h[IS_BIG_MAX];
+#pragma unroll
+    for (uint32_t c = 1; c <= SIZE_CLASSES; c++) {
+        const uint32_t n = h[c - 1];
+        if (n && c <= lane) top = c;                         // on threads
+        if (n && c > lane) longest = warp_us(c) > longest ? warp_us(c) : longest;
+        if (c > lane) sum += n * warp_us(c);                 // on warps
+    }
+    const uint32_t share = (sum + warps - 1) / warps;
+    const uint32_t us = (top ? thread_us(top) : 0u) + (share > longest ? share : longest);
+    const uint32_t key = lane <= a.small_max && lane <= SIZE_CLASSES ? us << 4 | lane : 0xffffffffu;
+    return __reduce_min_sync(0xffffffffu, key) & 15u;
+}
+
 // ---- kernel 2: ContactSolverSystem::initializeForIsland per manifold ------
 // (ContactSolverSystem.cpp:116-318).  Writes the manifold's solver record and
 // its points' records (layouts in dynamics_launch.h).
 __global__ void __launch_bounds__(128) dyn_manifold_init(const DynArgs a) {
+    // the blocks behind the manifolds' count the islands
+    const uint32_t mblocks = (a.nm + 127u) / 128u;
+    if (blockIdx.x >= mblocks) {
+        count_island_sizes(a, blockIdx.x - mblocks);
+        return;
+    }
     const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= a.nm) return;
     float4* __restrict__ q = a.mrec[m].q;
@@ -616,9 +694,8 @@ RD void store_manifold(const DynArgs& a, uint32_t mi) {
 // movable body, the order of the manifolds touching it gives bit-identical
 // results.
 //
-// 3a: one thread per island runs islands of up to small_max manifolds in
-//     the reference's order (none when the stage has few manifolds) and
-//     queues the larger ones.
+// 3a: one thread per island runs islands of up to small_limit manifolds in
+//     the reference's order and queues the larger ones.
 // 3b: persistent warps take the queued islands.  Lane 0 gives each manifold a
 //     level (1 + the highest level of an earlier manifold sharing a movable
 //     body) and sorts the island's manifolds by level; every pass (warm
@@ -634,7 +711,6 @@ RD void store_manifold(const DynArgs& a, uint32_t mi) {
 // (a.small_max, 8 by default, and a.giant_min, 256 by default: islands above
 // it go to kernel 3c, one CTA per island, the island staged in up to the
 // whole opt-in shared memory of a CTA; both come from DynTuning)
-constexpr uint32_t BIG_ISLAND = 64;   // queued first: the longest islands start first
 constexpr uint32_t ISLAND_DONE = 0xffffffffu;   // entry of giant_list solved by kernel 3b
 
 RD int4 man_ids(const DynArgs& a, uint32_t mi) {
@@ -644,6 +720,12 @@ RD int4 man_ids(const DynArgs& a, uint32_t mi) {
 RD uint32_t man_fixed(const DynArgs& a, uint32_t mi) { return uint32_t(__ldg(a.mrec[mi].q + DQ_MASS).w); }
 
 __global__ void __launch_bounds__(128) dyn_islands_small(const DynArgs a) {
+    __shared__ uint32_t s_limit;
+    if (threadIdx.x < 32) {
+        const uint32_t limit = small_limit(a, threadIdx.x);
+        if (threadIdx.x == 0) s_limit = limit;
+    }
+    __syncthreads();
     const uint32_t is = blockIdx.x * blockDim.x + threadIdx.x;
     if (is >= a.ni) return;
     const uint32_t m0 = a.i_start[is], cnt = a.i_count[is];
@@ -653,7 +735,7 @@ __global__ void __launch_bounds__(128) dyn_islands_small(const DynArgs a) {
     }
     if (a.i_jcount && a.i_jcount[is]) return;  // kernel 3d
     if (cnt == 0) return;
-    if (cnt > a.small_max) {
+    if (cnt > s_limit) {
         // big islands fill the list from the front, the others from the back
         if (cnt > a.giant_min) a.giant_list[atomicAdd(a.counters + 3, 1u)] = is;
         else if (cnt > BIG_ISLAND) a.large_list[atomicAdd(a.counters, 1u)] = is;
@@ -1964,7 +2046,6 @@ __global__ void __launch_bounds__(GIANT_THREADS, 1) dyn_islands_giant(const DynA
                 giant_layout(a, cnt, uint32_t(int64_t(l.w) + int64_t(l.z) - int64_t(s_p0)), g);
             }
             giant_solve(a, m0, cnt, g, warp, lane, s_depth, s_nslots, s_p0);
-            if (threadIdx.x == 0) atomicAdd(a.counters + 10, 1u);
         } else if (size_t(GIANT_LEVELS) * STREAM_RING * sizeof(StreamSlot) + GIANT_LEVELS * sizeof(int2) <= a.giant_smem) {
             // streamed by dyn_islands_stream (giant_list may still hold untaken
             // islands up to its end)
@@ -2312,7 +2393,7 @@ cudaError_t launch_dynamics(const DynArgs& a, cudaStream_t s, uint64_t* launches
     const uint32_t joint_blocks = (a.nji + 2 * joint_lanes - 1) / std::max(2 * joint_lanes, 1u);
     if (a.ni) cudaMemsetAsync(a.counters, 0, DYN_COUNTERS * sizeof(uint32_t), s);
     if (a.nb) { dyn_bodies_pre<<<blocks(a.nb), 128, 0, s>>>(a); (*launches)++; }
-    if (a.nm) { dyn_manifold_init<<<blocks(a.nm), 128, 0, s>>>(a); (*launches)++; }
+    if (a.nm) { dyn_manifold_init<<<blocks(a.nm) + (a.small_auto ? blocks(a.ni) : 0u), 128, 0, s>>>(a); (*launches)++; }
     if (a.nj) { dyn_joints_init<<<blocks(a.nj), 128, 0, s>>>(a); (*launches)++; }
     if (a.stats) cudaMemsetAsync(a.stats, 0, sizeof(SolverStats), s);
     // the graph-coloured solver takes every island when the stage has no

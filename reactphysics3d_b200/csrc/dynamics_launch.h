@@ -155,12 +155,14 @@ struct DynArgs {
                            // [3] giant islands queued, [4] giant islands taken,
                            // [5] streamed islands queued, [6] streamed islands taken,
                            // [7] giant islands offered to kernel 3b,
-                           // islands solved so far: [8] by a thread, [9] by a warp, [10] by a CTA in shared memory
+                           // islands solved so far: [8] by a thread, [9] by a warp,
+                           // [10..] island sizes (IslandSizes)
     uint32_t* large_list;  // ni: queued islands
     uint32_t* giant_list;  // ni: islands for kernel 3c
     uint32_t* stream_list; // ni: islands that do not fit kernel 3c's shared memory
     uint32_t large_ctas;   // grid of kernel 3b (persistent)
     uint32_t small_max;    // islands of up to this many manifolds: one thread each (kernel 3a)
+    int32_t small_auto;    // small_max is the most that small_limit may choose
     uint32_t giant_min;    // islands above this many manifolds: one CTA each (kernel 3c)
     int32_t giant_auto;    // giant_min is the default, and big_on_ctas / giants_on_warps move islands across it
     // joints (nj = 0: none).  j_list holds this step's enabled joints island
@@ -222,7 +224,7 @@ struct DynSolver {
 };
 
 // 32-bit words at DynArgs::counters.
-constexpr uint32_t DYN_COUNTERS = 11;
+constexpr uint32_t DYN_COUNTERS = 23;
 
 // Launches the kernels in order on stream s; *launches counts them.
 cudaError_t launch_dynamics(const DynArgs& a, cudaStream_t s, uint64_t* launches);

@@ -556,7 +556,7 @@ int rp3dg_dynamics_routes(rp3dg_ctx* ctx, uint32_t* out) {
                                     cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "read island routes");
-    out[0] = c[8]; out[1] = c[9]; out[2] = c[10]; out[3] = c[5];
+    out[0] = c[8]; out[1] = c[9]; out[2] = c[0] + c[2] + c[3] - c[9] - c[5]; out[3] = c[5];
     return 0;
 }
 
@@ -2040,12 +2040,8 @@ int dynamics_step_flags(rp3dg_ctx* ctx, const rp3dg_dynamics_params* pr, const r
     const rp3dg::DynTuning tdef{};
     const rp3dg::DynTuning& tn = tune ? *tune : tdef;
     a.large_ctas = uint32_t(ctx->num_sms) * (tn.large_per_sm ? tn.large_per_sm : 1u);
-    // A thread an island saves warps, not time: with few manifolds every island
-    // is faster on a warp of kernel 3b.  Warps / threads, us a stage: 192
-    // worlds of 92 manifolds (20 a warp) 822 / 847, 384 worlds 889 / 877,
-    // 4,096 worlds 2,642 / 1,797.
-    const uint32_t warps = a.large_ctas * uint32_t(rp3dg::LARGE_WARPS);
-    a.small_max = tn.small_auto && a.nm <= 24u * warps ? 0u : tn.small_max;
+    a.small_max = tn.small_max;
+    a.small_auto = tn.small_auto ? 1 : 0;
     a.giant_min = tn.giant_min;
     a.giant_auto = tn.giant_auto ? 1 : 0;
     a.giant_ctas = uint32_t(ctx->num_sms);
