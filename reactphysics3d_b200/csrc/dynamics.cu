@@ -159,8 +159,8 @@ RD float4 F4w(v3 a, float w) { return make_float4(a.x, a.y, a.z, w); }
 // them: 0 2,635, 4 1,846, 8 1,785.
 constexpr uint32_t BIG_ISLAND = 64;   // queued first: the longest islands start first
 constexpr uint32_t SIZE_CLASSES = 8;  // islands of 1 .. 8 manifolds by size
-enum IslandSizes { IS_MID = SIZE_CLASSES, IS_MID_MAX, IS_BIG, IS_BIG_SUM, IS_BIG_MAX, IS_WORDS };   // from counters[10]
-static_assert(10 + IS_WORDS == DYN_COUNTERS, "counters");
+enum IslandSizes { IS_MID = SIZE_CLASSES, IS_MID_MAX, IS_BIG, IS_BIG_SUM, IS_BIG_MAX, IS_WORDS };   // from counters[9]
+static_assert(9 + IS_WORDS == DYN_COUNTERS, "counters");
 
 RD uint32_t thread_us(uint32_t manifolds) { return 35u * manifolds - 14u; }
 RD uint32_t warp_us(uint32_t manifolds) {
@@ -189,8 +189,8 @@ RD void count_island_sizes(const DynArgs& a, uint32_t block) {
     __syncthreads();
     const uint32_t k = threadIdx.x;
     if (k < IS_WORDS && h[k]) {
-        if (k == IS_MID_MAX || k == IS_BIG_MAX) atomicMax(a.counters + 10 + k, h[k]);
-        else atomicAdd(a.counters + 10 + k, h[k]);
+        if (k == IS_MID_MAX || k == IS_BIG_MAX) atomicMax(a.counters + 9 + k, h[k]);
+        else atomicAdd(a.counters + 9 + k, h[k]);
     }
 }
 
@@ -198,7 +198,7 @@ RD void count_island_sizes(const DynArgs& a, uint32_t block) {
 // a warp estimates limit s.
 RD uint32_t small_limit(const DynArgs& a, uint32_t lane) {
     if (!a.small_auto) return a.small_max;
-    const uint32_t* h = a.counters + 10;
+    const uint32_t* h = a.counters + 9;
     const uint32_t warps = a.large_ctas * uint32_t(LARGE_WARPS);
     const bool big = h[IS_BIG] > a.giant_ctas;   // too many for a CTA each
     uint32_t sum = h[IS_MID] + (big ? h[IS_BIG_SUM] : 0u), longest = h[IS_MID_MAX], top = 0;
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(128) dyn_islands_small(const DynArgs a) {
         return;
     }
     const unsigned here = __activemask();
-    if ((threadIdx.x & 31u) == uint32_t(__ffs(here)) - 1u) atomicAdd(a.counters + 8, uint32_t(__popc(here)));
+    if ((threadIdx.x & 31u) == uint32_t(__ffs(here)) - 1u) atomicAdd(a.counters + 7, uint32_t(__popc(here)));
     const uint32_t m1 = m0 + cnt;
     for (uint32_t mi = m0; mi < m1; mi++) {
         const int4 id = man_ids(a, mi);
@@ -1254,6 +1254,46 @@ RD void chunk_stage(const DynArgs& a, uint32_t m0, LaneSlot* slot, const int4& d
     cp_async_commit();
 }
 
+// Whether an island's levels are wide: a warp takes four manifolds at a time
+// with eight lanes each, 32 with one each, and such a round takes 2.2 times as
+// long.  200 islands of 200 manifolds in two levels: 541 us with eight lanes,
+// 339 with one; in 12 levels of 17: 591 and 452; 1,000 of 60 manifolds in ten
+// levels (18 chunks of four): 403 with eight lanes, 514 with one.
+RD bool wide_levels(const WarpStage* st, uint32_t depth, uint32_t lane) {
+    uint32_t fours = 0, rounds = 0;
+    for (uint32_t L = lane; L < depth; L += 32) {
+        const uint32_t width = uint32_t(st->lev[L + 1]) - uint32_t(st->lev[L]);
+        fours += (width + WARP_MANIFOLDS - 1) / WARP_MANIFOLDS;
+        rounds += (width + 31u) / 32u;
+    }
+    return __reduce_add_sync(0xffffffffu, fours) > 2u * __reduce_add_sync(0xffffffffu, rounds);
+}
+// One lane a manifold, level after level, the rows from global memory.
+RD void solve_staged_wide(const DynArgs& a, uint32_t m0, WarpStage* st, uint32_t lane, uint32_t depth) {
+    for (int pass = 0; pass <= a.iterations; pass++)
+        for (uint32_t L = 0; L < depth; L++) {
+            for (uint32_t k = st->lev[L] + lane; k < st->lev[L + 1]; k += 32) {
+                const int4 d = st->desc[k];
+                const uint32_t s1 = uint32_t(d.x) & 0xffffu, s2 = uint32_t(d.x) >> 16;
+                BodyVel bv;
+                bv.v1 = &st->vel[0][s1]; bv.w1 = &st->vel[1][s1]; bv.s1 = &st->vel[2][s1]; bv.t1 = &st->vel[3][s1];
+                bv.v2 = &st->vel[0][s2]; bv.w2 = &st->vel[1][s2]; bv.s2 = &st->vel[2][s2]; bv.t2 = &st->vel[3][s2];
+                const RecSrc r = rec_global(a, m0 + uint32_t(d.z), d.w);
+                if (pass == 0) warm_core<true>(a, r, bv, d.y);
+                else solve_core<true>(a, r, bv, d.y);
+            }
+            __syncwarp();
+        }
+}
+RD void staged_write_back(const DynArgs& a, const WarpStage* st, uint32_t lane) {
+    for (uint32_t s = lane; s < st->nslots; s += 32) {
+        const int32_t b = st->slot_body[s];
+        if (b < 0) continue;
+        a.cv[b] = st->vel[0][s]; a.cw[b] = st->vel[1][s];
+        a.sv[b] = st->vel[2][s]; a.sw[b] = st->vel[3][s];
+    }
+}
+
 // Solves a scheduled island from the warp's stage: the rows of the next
 // chunk arrive by cp.async while a chunk is solved.
 RD void solve_staged(const DynArgs& a, uint32_t m0, uint32_t cnt, WarpStage* st, uint32_t lane, uint32_t depth) {
@@ -1270,6 +1310,11 @@ RD void solve_staged(const DynArgs& a, uint32_t m0, uint32_t cnt, WarpStage* st,
         st->desc[k] = make_int4(int(uint32_t(uint16_t(sl.x)) | (uint32_t(uint16_t(sl.y)) << 16)), id.z, int(kk), id.w);
     }
     __syncwarp();   // the schedule's part of the union is free now
+    if (wide_levels(st, depth, lane)) {
+        solve_staged_wide(a, m0, st, lane, depth);
+        staged_write_back(a, st, lane);
+        return;
+    }
     const LaneId id = lane_id(lane);
     float* vel = reinterpret_cast<float*>(st->vel[2 * id.role]);
     constexpr uint32_t wofs = 4 * STAGE_BODIES;
@@ -1322,12 +1367,7 @@ RD void solve_staged(const DynArgs& a, uint32_t m0, uint32_t cnt, WarpStage* st,
         buf ^= 1;
         job = nxt;
     }
-    for (uint32_t s = lane; s < nslots; s += 32) {
-        const int32_t b = st->slot_body[s];
-        if (b < 0) continue;
-        a.cv[b] = st->vel[0][s]; a.cw[b] = st->vel[1][s];
-        a.sv[b] = st->vel[2][s]; a.sw[b] = st->vel[3][s];
-    }
+    staged_write_back(a, st, lane);
 }
 
 RD bool schedule_staged(const DynArgs& a, uint32_t m0, uint32_t cnt, WarpStage* st, uint32_t lane, uint32_t& depth) {
@@ -1413,45 +1453,35 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32, 2) dyn_islands_large(const D
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     WarpStage* st = reinterpret_cast<WarpStage*>(smem_raw + size_t(wid) * LARGE_WARP_SMEM);
-    uint32_t solved = 0;
     // the longest work first
-    if (giants_on_warps(a)) {
-        const uint32_t n_giant = a.counters[3];
-        for (;;) {
-            uint32_t k = 0;
-            if (lane == 0) k = atomicAdd(a.counters + 7, 1u);
-            k = __shfl_sync(0xffffffffu, k, 0);
-            if (k >= n_giant) break;
-            const uint32_t is = a.giant_list[k];
-            const uint32_t m0 = a.i_start[is], cnt = a.i_count[is];
-            uint32_t depth = 0;
-            if (cnt <= STAGE_MANIFOLDS && schedule_staged(a, m0, cnt, st, lane, depth)) {
-                solve_staged(a, m0, cnt, st, lane, depth);
-                __syncwarp();
-                for (uint32_t j = lane; j < cnt; j += 32) store_manifold(a, m0 + j);
-                if (lane == 0) a.giant_list[k] = ISLAND_DONE;
-                solved++;
-            }
-            __syncwarp();
-        }
-    }
+    const uint32_t n_giant = giants_on_warps(a) ? a.counters[3] : 0u;
     const uint32_t n_big = big_on_ctas(a) ? 0u : a.counters[0], n_mid = a.counters[2];
+    uint32_t solved = 0;
     for (;;) {
         uint32_t k = 0;
         if (lane == 0) k = atomicAdd(a.counters + 1, 1u);
         k = __shfl_sync(0xffffffffu, k, 0);
-        if (k >= n_big + n_mid) break;
-        const uint32_t is = k < n_big ? a.large_list[k] : a.large_list[a.ni - 1 - (k - n_big)];
+        if (k >= n_giant + n_big + n_mid) break;
+        const bool giant = k < n_giant;
+        const uint32_t j = k - n_giant;
+        const uint32_t is = giant ? a.giant_list[k] : (j < n_big ? a.large_list[j] : a.large_list[a.ni - 1 - (j - n_big)]);
         const uint32_t m0 = a.i_start[is], cnt = a.i_count[is];
         uint32_t depth = 0;
-        if (cnt <= STAGE_MANIFOLDS && schedule_staged(a, m0, cnt, st, lane, depth)) solve_staged(a, m0, cnt, st, lane, depth);
-        else solve_global(a, m0, cnt, lane);
+        if (cnt <= STAGE_MANIFOLDS && schedule_staged(a, m0, cnt, st, lane, depth)) {
+            solve_staged(a, m0, cnt, st, lane, depth);
+            if (giant && lane == 0) a.giant_list[k] = ISLAND_DONE;
+        } else if (giant) {
+            __syncwarp();
+            continue;   // kernel 3c takes it
+        } else {
+            solve_global(a, m0, cnt, lane);
+        }
         __syncwarp();
-        for (uint32_t j = lane; j < cnt; j += 32) store_manifold(a, m0 + j);
+        for (uint32_t i = lane; i < cnt; i += 32) store_manifold(a, m0 + i);
         solved++;
         __syncwarp();
     }
-    if (lane == 0 && solved) atomicAdd(a.counters + 9, solved);
+    if (lane == 0 && solved) atomicAdd(a.counters + 8, solved);
 }
 
 

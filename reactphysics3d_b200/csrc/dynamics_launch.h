@@ -151,12 +151,11 @@ struct DynArgs {
     uint32_t* order;       // nm: island manifolds sorted by level (scratch)
     uint32_t* body_level;  // nb: last level of each movable body (scratch)
     int32_t* body_slot;    // nb: shared-memory slot of each movable body (scratch)
-    uint32_t* counters;    // [0] big islands queued (front of large_list), [1] islands taken, [2] others queued (back),
+    uint32_t* counters;    // [0] big islands queued (front of large_list), [1] islands taken by kernel 3b, [2] others queued (back),
                            // [3] giant islands queued, [4] giant islands taken,
                            // [5] streamed islands queued, [6] streamed islands taken,
-                           // [7] giant islands offered to kernel 3b,
-                           // islands solved so far: [8] by a thread, [9] by a warp,
-                           // [10..] island sizes (IslandSizes)
+                           // islands solved so far: [7] by a thread, [8] by a warp,
+                           // [9..] island sizes (IslandSizes)
     uint32_t* large_list;  // ni: queued islands
     uint32_t* giant_list;  // ni: islands for kernel 3c
     uint32_t* stream_list; // ni: islands that do not fit kernel 3c's shared memory
@@ -224,7 +223,7 @@ struct DynSolver {
 };
 
 // 32-bit words at DynArgs::counters.
-constexpr uint32_t DYN_COUNTERS = 23;
+constexpr uint32_t DYN_COUNTERS = 22;
 
 // Launches the kernels in order on stream s; *launches counts them.
 cudaError_t launch_dynamics(const DynArgs& a, cudaStream_t s, uint64_t* launches);

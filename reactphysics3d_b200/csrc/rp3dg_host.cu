@@ -556,7 +556,7 @@ int rp3dg_dynamics_routes(rp3dg_ctx* ctx, uint32_t* out) {
                                     cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "read island routes");
-    out[0] = c[8]; out[1] = c[9]; out[2] = c[0] + c[2] + c[3] - c[9] - c[5]; out[3] = c[5];
+    out[0] = c[7]; out[1] = c[8]; out[2] = c[0] + c[2] + c[3] - c[8] - c[5]; out[3] = c[5];
     return 0;
 }
 
