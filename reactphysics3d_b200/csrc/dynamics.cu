@@ -147,12 +147,13 @@ RD float4 F4w(v3 a, float w) { return make_float4(a.x, a.y, a.z, w); }
 // ---- island sizes: which islands get a thread each -------------------------
 //
 // An island on a thread costs kernel 3a a chain of its manifolds, however many
-// islands there are; an island on a warp costs one of kernel 3b's warps its
-// time, and the warps share the islands.  A thread each pays when the warps
-// would have several small islands each, so the limit is chosen from the
-// stage's island sizes, by what both sides measured (four-point manifolds, 888
-// warps): a thread 21, 56, 91, 126, 266 us for 1, 2, 3, 4, 8 manifolds, a warp
-// 10, 17, 23, 28, 42 us an island.
+// islands there are, and more the more lanes of a warp are at one; an island on
+// a warp costs one of kernel 3b's warps its time, and the warps share the
+// islands.  A thread each pays when the warps would have several small islands
+// each, so the limit is chosen from the stage's island sizes, by what both sides
+// measured (points at random, 888 warps): threads 21, 56, 91, 126, 266 us for
+// islands of 1, 2, 3, 4, 8 manifolds when all lanes have one, a warp 10, 17, 23,
+// 28, 42 us an island.
 // 12,000 islands of one manifold: warps 208 us a stage, threads 97; 2,500
 // islands of eight: warps 206, threads 341; 192 captured worlds (6,976
 // islands, half of them of one manifold): limit 0 817, 1 804, 8 859; 4,096 of
@@ -162,7 +163,10 @@ constexpr uint32_t SIZE_CLASSES = 8;  // islands of 1 .. 8 manifolds by size
 enum IslandSizes { IS_MID = SIZE_CLASSES, IS_MID_MAX, IS_BIG, IS_BIG_SUM, IS_BIG_MAX, IS_WORDS };   // from counters[9]
 static_assert(9 + IS_WORDS == DYN_COUNTERS, "counters");
 
-RD uint32_t thread_us(uint32_t manifolds) { return 35u * manifolds - 14u; }
+// `longest` the most manifolds of an island, `manifolds` those of all, a stage of `ni` islands
+RD uint32_t thread_us(uint32_t longest, uint32_t manifolds, uint32_t ni) {
+    return longest ? uint32_t(13.0f * float(longest) + 22.0f * float(manifolds) / float(ni)) - 5u : 0u;
+}
 RD uint32_t warp_us(uint32_t manifolds) {
     return manifolds <= SIZE_CLASSES ? 7u + 5u * manifolds : 47u + (manifolds - SIZE_CLASSES) * 11u / 4u;
 }
@@ -201,17 +205,17 @@ RD uint32_t small_limit(const DynArgs& a, uint32_t lane) {
     const uint32_t* h = a.counters + 9;
     const uint32_t warps = a.large_ctas * uint32_t(LARGE_WARPS);
     const bool big = h[IS_BIG] > a.giant_ctas;   // too many for a CTA each
-    uint32_t sum = h[IS_MID] + (big ? h[IS_BIG_SUM] : 0u), longest = h[IS_MID_MAX], top = 0;
+    uint32_t sum = h[IS_MID] + (big ? h[IS_BIG_SUM] : 0u), longest = h[IS_MID_MAX], top = 0, mans = 0;
     if (big && h[IS_BIG_MAX] > longest) longest = h[IS_BIG_MAX];
 #pragma unroll
     for (uint32_t c = 1; c <= SIZE_CLASSES; c++) {
         const uint32_t n = h[c - 1];
-        if (n && c <= lane) top = c;                         // on threads
+        if (n && c <= lane) { top = c; mans += n * c; }       // on threads
         if (n && c > lane) longest = warp_us(c) > longest ? warp_us(c) : longest;
         if (c > lane) sum += n * warp_us(c);                 // on warps
     }
     const uint32_t share = (sum + warps - 1) / warps;
-    const uint32_t us = (top ? thread_us(top) : 0u) + (share > longest ? share : longest);
+    const uint32_t us = thread_us(top, mans, a.ni) + (share > longest ? share : longest);
     const uint32_t key = lane <= a.small_max && lane <= SIZE_CLASSES ? us << 4 | lane : 0xffffffffu;
     return __reduce_min_sync(0xffffffffu, key) & 15u;
 }
