@@ -651,17 +651,6 @@ __global__ void __launch_bounds__(RAY_BLOCK, RAY_MIN_BLOCKS) world_raycast_kerne
             if (ret > 0.0f && ret < maxf) maxf = ret;
         }
     }
-    // The last warp leaves the counters at zero for the next launch on the
-    // stream.  (A clear queued before each launch is not enough: two threads
-    // casting rays at one world may queue clear, clear, launch, launch, and
-    // the second launch then finds every ray handed out.)
-    if (lane == 0) {
-        __threadfence();
-        if (atomicAdd(a.queue + 1, 1u) == gridDim.x * (RAY_BLOCK / 32) - 1u) {
-            a.queue[0] = 0u;
-            a.queue[1] = 0u;
-        }
-    }
 }
 
 }  // namespace

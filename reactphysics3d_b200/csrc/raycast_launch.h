@@ -32,7 +32,7 @@ struct RayArgs {
     uint32_t max_hits;
     rp3dg_raycast_hit* hits;       // n * max_hits
     uint32_t* nb_hits;             // n
-    uint32_t* queue;               // rays handed out so far, warps that are done; 0 before and after the launch
+    uint32_t* queue;               // rays handed out so far, 0 before the launch
     uint32_t* error;               // bit 0: a traversal stack overflowed (world or mesh tree)
 };
 

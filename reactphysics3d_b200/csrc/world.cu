@@ -45,6 +45,7 @@
 #include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -977,7 +978,8 @@ struct rp3dg_world {
     rp3dg_ray* d_rays = nullptr;
     rp3dg_raycast_hit* d_rhits = nullptr;
     uint32_t* d_rcount = nullptr;    // n counts
-    uint32_t* d_rwork = nullptr;     // error word, then the ray kernel's two counters (0 between launches)
+    uint32_t* d_rwork = nullptr;     // error word, rays handed out
+    std::mutex ray_mutex;            // a clear of d_rwork and the launch that follows it
     bool ray_finite = false;         // every node of the tables has finite bounds
     cudaEvent_t ev_r0 = nullptr, ev_r1 = nullptr;
     // manifold packing
@@ -3729,14 +3731,11 @@ int raycast_device(Group* g, uint32_t world, const rp3dg_ray* rays, uint32_t n, 
                    rp3dg_raycast_hit* hits, uint32_t* nb_hits, float* kernel_ms) {
     int rc = ray_tables(g, world);
     if (rc) return rc;
-    cudaStream_t st = g->stream;
-    if (!g->d_rwork) {
-        if (dev_grow(&g->d_rwork, &g->cap_rwork, 3))
-            return wfail(g, RP3DG_ENOMEM, "allocation of the raycast error word");
-        cudaMemsetAsync(g->d_rwork, 0, 3 * sizeof(uint32_t), st);
-    }
+    if (dev_grow(&g->d_rwork, &g->cap_rwork, 2))
+        return wfail(g, RP3DG_ENOMEM, "allocation of the raycast error word");
     if (!g->ev_r0 && (cudaEventCreate(&g->ev_r0) != cudaSuccess || cudaEventCreate(&g->ev_r1) != cudaSuccess))
         return wfail(g, RP3DG_ECUDA, "cudaEventCreate(raycast)");
+    cudaStream_t st = g->stream;
     WorldH& w = g->worlds[world];
     rp3dg::RayArgs a{};
     a.nodes = g->d_rnodes;
@@ -3760,10 +3759,16 @@ int raycast_device(Group* g, uint32_t world, const rp3dg_ray* rays, uint32_t n, 
     a.nb_hits = nb_hits;
     a.error = g->d_rwork;
     a.queue = g->d_rwork + 1;
-    cudaMemsetAsync(g->d_rwork, 0, sizeof(uint32_t), st);
-    cudaEventRecord(g->ev_r0, st);
-    cudaError_t e = rp3dg::launch_world_raycast(a, rp3dg::get_num_sms(g->ctx), st);
-    cudaEventRecord(g->ev_r1, st);
+    cudaError_t e;
+    {
+        // two threads casting rays at one world must not queue clear, clear,
+        // launch, launch: the second launch would find every ray handed out
+        std::lock_guard<std::mutex> lock(g->ray_mutex);
+        cudaMemsetAsync(g->d_rwork, 0, 2 * sizeof(uint32_t), st);
+        cudaEventRecord(g->ev_r0, st);
+        e = rp3dg::launch_world_raycast(a, rp3dg::get_num_sms(g->ctx), st);
+        cudaEventRecord(g->ev_r1, st);
+    }
     if (e != cudaSuccess) return wcuda(g, e, "raycast kernel");
     uint32_t err = 0;
     cudaMemcpyAsync(&err, g->d_rwork, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
