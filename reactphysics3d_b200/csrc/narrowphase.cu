@@ -32,7 +32,7 @@ namespace rp3dg {
 // Internal kernel id: the per-thread half of the polyhedron schedule.
 constexpr int ALGO_POLY_PER_THREAD = 7;
 // Internal kernel ids of the warp-per-pair launches, plus their mask.
-constexpr int WARP_KERNEL = 8, WARP_KERNEL_STAGED = 16;
+constexpr int WARP_KERNEL = 8, WARP_KERNEL_STAGED = 16, WARP_KERNEL_SMALL = 24;
 constexpr int NP_MIN_BLOCKS = RP3DG_NP_MIN_BLOCKS;
 constexpr int NP_MIN_BLOCKS_POLY_WARP = RP3DG_NP_MIN_BLOCKS_POLY_WARP;
 constexpr int NP_MIN_BLOCKS_MESH_WARP = 4;
@@ -289,7 +289,7 @@ template <int MASK>
 struct MaskScratch { typedef WarpScratchMesh type; };
 template <>
 struct MaskScratch<WARP_MESH_BOX> { typedef WarpScratch type; };
-template <int COMBO, class Scratch>
+template <int COMBO, bool SMALL, class Scratch>
 RD uint32_t process_pair_warp(const NpArgs& a, uint32_t i, int lane, const BoxTables* box, const uint32_t* mesh_words,
                               Scratch& stage, uint32_t proposal) {
     const int32_t i1 = a.shape1[i], i2 = a.shape2[i];
@@ -318,6 +318,8 @@ RD uint32_t process_pair_warp(const NpArgs& a, uint32_t i, int lane, const BoxTa
         warp_sat_poly_poly(it, mesh_poly(mesh_words, s1.mesh), box_poly(s2, box), a.clip, lane, stage);
     else if constexpr (COMBO == COMBO_BOX_MESH)
         warp_sat_poly_poly(it, box_poly(s1, box), mesh_poly(mesh_words, s2.mesh), a.clip, lane, stage);
+    else if constexpr (SMALL)
+        warp_sat_poly_poly(it, mesh_poly(mesh_words, s1.mesh), SmallMeshPoly(mesh_poly(mesh_words, s2.mesh)), a.clip, lane, stage);
     else
         warp_sat_poly_poly(it, mesh_poly(mesh_words, s1.mesh), mesh_poly(mesh_words, s2.mesh), a.clip, lane, stage);
     // ConvexPolyhedronVsConvexPolyhedronAlgorithm.cpp:53-61
@@ -426,7 +428,7 @@ __global__ void __launch_bounds__(NP_BLOCK, MinBlocks<ALGO>::value) narrowphase_
     }
 }
 
-template <int COMBO, class Scratch>
+template <int COMBO, bool SMALL, class Scratch>
 RD void warp_list(const NpArgs& a, int lane, const BoxTables* box, const uint32_t* mesh_words, Scratch& ws,
                   uint32_t& tested, uint32_t& confirmed) {
     const uint32_t total = __ldcg(a.work + (COMBO - 1));
@@ -439,7 +441,7 @@ RD void warp_list(const NpArgs& a, int lane, const BoxTables* box, const uint32_
         const uint32_t i = list[k];
         uint32_t proposal = a.proposals ? uint32_t(a.proposals[i]) : uint32_t(MLP_NO_PROPOSAL);
         if (proposal >= MLP_OUT) proposal = MLP_NO_PROPOSAL;
-        const uint32_t r = process_pair_warp<COMBO>(a, i, lane, box, mesh_words, ws, proposal);
+        const uint32_t r = process_pair_warp<COMBO, SMALL>(a, i, lane, box, mesh_words, ws, proposal);
         tested += r & 1u;
         confirmed += (r >> 1) & 1u;
         __syncwarp();
@@ -462,7 +464,11 @@ RD void warp_list(const NpArgs& a, int lane, const BoxTables* box, const uint32_
 // launch with nothing to do costs its 2-3 us all the same.  42 hull-box and 42
 // box-box pairs among five other batches 136 -> 128 us, 100,003 box-box pairs
 // 77.0 -> 72.6 us against a launch per combination.
-template <int MASK, bool STAGED>
+// SMALL: every mesh of the context has at most SMALL_MESH_EDGES edges, and mesh
+// pairs skip the masks: 200,000 tetrahedron pairs 663 us, with them 1,023;
+// prisms of 9 edges 677 and 940, of 12 edges 814 and 1,023; of 15 edges about
+// the same either way (1,057 to 1,107).
+template <int MASK, bool STAGED, bool SMALL = false>
 __global__ void __launch_bounds__(NP_BLOCK, MASK == WARP_MESH_BOX ? NP_MIN_BLOCKS_POLY_WARP : NP_MIN_BLOCKS_MESH_WARP)
     narrowphase_warp_kernel(const NpArgs a) {
     extern __shared__ __align__(16) uint32_t s_mesh[];
@@ -485,9 +491,9 @@ __global__ void __launch_bounds__(NP_BLOCK, MASK == WARP_MESH_BOX ? NP_MIN_BLOCK
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t tested = 0, confirmed = 0;
-    if constexpr ((MASK & 4) != 0) warp_list<COMBO_MESH_MESH>(a, lane, &s_box, mesh_words, s_stage[warp], tested, confirmed);
-    if constexpr ((MASK & 2) != 0) warp_list<COMBO_BOX_MESH>(a, lane, &s_box, mesh_words, s_stage[warp], tested, confirmed);
-    if constexpr ((MASK & 1) != 0) warp_list<COMBO_MESH_BOX>(a, lane, &s_box, mesh_words, s_stage[warp], tested, confirmed);
+    if constexpr ((MASK & 4) != 0) warp_list<COMBO_MESH_MESH, SMALL>(a, lane, &s_box, mesh_words, s_stage[warp], tested, confirmed);
+    if constexpr ((MASK & 2) != 0) warp_list<COMBO_BOX_MESH, SMALL>(a, lane, &s_box, mesh_words, s_stage[warp], tested, confirmed);
+    if constexpr ((MASK & 1) != 0) warp_list<COMBO_MESH_BOX, SMALL>(a, lane, &s_box, mesh_words, s_stage[warp], tested, confirmed);
     if (a.mlp_stats && lane == 0 && tested) {
         atomicAdd(&a.mlp_stats[0], (unsigned long long)tested);
         atomicAdd(&a.mlp_stats[1], (unsigned long long)confirmed);
@@ -746,6 +752,7 @@ static const void* kernel_ptr(int algo) {
         case WARP_KERNEL_STAGED + WARP_MESH_BOX: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<WARP_MESH_BOX, true>);
         case WARP_KERNEL_STAGED + WARP_MESH_SECOND: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<WARP_MESH_SECOND, true>);
         case WARP_KERNEL_STAGED + WARP_ALL: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<WARP_ALL, true>);
+        case WARP_KERNEL_SMALL + WARP_MESH_SECOND: return reinterpret_cast<const void*>(&narrowphase_warp_kernel<WARP_MESH_SECOND, true, true>);
         case ALGO_POLY_PER_THREAD: return reinterpret_cast<const void*>(&narrowphase_kernel<ALGO_POLY_PER_THREAD>);
     }
     return nullptr;
@@ -788,7 +795,8 @@ cudaError_t launch_narrowphase(int algo, const NpArgs& args, int num_sms, cudaSt
         const bool all = args.n <= uint32_t(num_sms) * uint32_t(NP_MIN_BLOCKS_MESH_WARP) * (NP_BLOCK / 32);
         for (int mask : {all ? WARP_ALL : WARP_MESH_BOX, all ? 0 : WARP_MESH_SECOND}) {
             if (mask == 0) break;
-            e = launch_one(base + mask, args, num_sms, stream);
+            const bool small = mask == WARP_MESH_SECOND && args.stage_mesh && args.small_meshes;
+            e = launch_one((small ? WARP_KERNEL_SMALL : base) + mask, args, num_sms, stream);
             if (e != cudaSuccess) return e;
             ++*launches;
         }

@@ -2009,6 +2009,37 @@ struct EdgePairs<P1, MeshPoly> {
     }
 };
 
+// A mesh of a context whose meshes all have few edges (SMALL_MESH_EDGES).
+struct SmallMeshPoly : MeshPoly {
+    RD explicit SmallMeshPoly(const MeshPoly& m) : MeshPoly(m) {}
+};
+
+// Two such meshes: the whole test of every pair is done before the masks would
+// be (two tetrahedra have 36 pairs).
+template <class P1>
+struct EdgePairs<P1, SmallMeshPoly> {
+    typedef WarpScratch Scratch;
+    const P1& p1;
+    const SmallMeshPoly& p2;
+    uint32_t base, n2h, total;
+    RD EdgePairs(const P1& a, const SmallMeshPoly& b, uint32_t n1, uint32_t n2, const xform&, Scratch&, int)
+        : p1(a), p2(b), base(0), n2h(n2), total(n1 * n2) {}
+    RD bool more() const { return base < total; }
+    RD void fill(Scratch& ws, uint32_t& ncand, const xform&, int lane) {
+        const uint32_t n = total - base < WARP_CAND_CAP ? total - base : WARP_CAND_CAP;
+        for (uint32_t k = lane; k < n; k += 32) {
+            const uint32_t t = base + k;
+            ws.cand[k] = uint16_t(t / n2h * WARP_EDGE_CAP + t % n2h);
+        }
+        ncand = n;
+        base += n;
+    }
+    RD bool test(uint32_t pair, const xform& p1to2, const Scratch& ws) const {
+        return edges_minkowski(warp_edge1_gauss(p1, pair / WARP_EDGE_CAP, p1to2, ws.nr), p2,
+                               p2.edge(2 * (pair % WARP_EDGE_CAP)));
+    }
+};
+
 // testCollisionConvexPolyhedronVsConvexPolyhedron (SATAlgorithm.cpp:485-889), one warp per pair.
 // Every lane holds the same pair state; contacts and outputs are produced by lane 0.
 template <class P1, class P2>

@@ -13,6 +13,10 @@ constexpr int NP_BLOCK = 128;
 // Mesh arenas up to this size are staged in shared memory by every CTA.
 constexpr uint32_t MESH_STAGE_MAX_BYTES = 108 * 1024;
 
+// Mesh pairs of up to this many edges each are tested pair by pair, without
+// the side masks.
+constexpr uint32_t SMALL_MESH_EDGES = 14;
+
 struct NpArgs {
     uint32_t n;
     uint32_t lanes;   // pairs a warp takes at once (set by the launch, see items_per_warp)
@@ -21,6 +25,7 @@ struct NpArgs {
     uint32_t max_contacts;
     int clip;
     int stage_mesh;
+    int small_meshes;  // no mesh has more than SMALL_MESH_EDGES edges
     uint32_t mesh_nwords;
     const uint32_t* mesh_words;
     const rp3dg_shape* shapes;

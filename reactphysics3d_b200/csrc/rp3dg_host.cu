@@ -226,6 +226,7 @@ struct rp3dg_ctx {
     std::vector<MeshTopo> meshes;
     std::vector<MeshInstance> instances;
     std::vector<uint32_t> arena;  // host copy of the device mesh arena
+    uint32_t max_mesh_edges = 0;  // of its instances
     uint32_t* d_arena = nullptr;
     size_t cap_arena = 0;
     // device error word written by the kernels (bit 0: a pair named a shape outside the table)
@@ -326,6 +327,7 @@ int cuda_fail(rp3dg_ctx* ctx, cudaError_t e, const char* what) {
 void rebuild_arena(rp3dg_ctx* ctx) {
     std::vector<uint32_t>& w = ctx->arena;
     const uint32_t nin = uint32_t(ctx->instances.size());
+    ctx->max_mesh_edges = 0;
     const uint32_t hdr_words = nin * (sizeof(MeshHdr) / 4);
     w.assign(hdr_words, 0u);
     auto align4 = [&]() { w.resize((w.size() + 3) & ~size_t(3), 0u); };
@@ -344,6 +346,7 @@ void rebuild_arena(rp3dg_ctx* ctx) {
         MeshHdr h;
         std::memset(&h, 0, sizeof(h));
         h.nv = m.nv; h.nf = m.nf; h.nhe = uint32_t(m.edges.size());
+        ctx->max_mesh_edges = std::max(ctx->max_mesh_edges, h.nhe / 2);
         h.off_verts = uint32_t(w.size());
         push_rows(m.verts);
         h.off_sverts = uint32_t(w.size());
@@ -1107,6 +1110,7 @@ int np_args(rp3dg_ctx* ctx, int algorithm, const rp3dg_pair_batch* p, const rp3d
     a.mesh_words = ctx->d_arena;
     a.stage_mesh = (algorithm >= RP3DG_ALGO_SPHERE_VS_CONVEX_POLYHEDRON && a.mesh_nwords > 0 &&
                     size_t(a.mesh_nwords) * 4 <= rp3dg::MESH_STAGE_MAX_BYTES) ? 1 : 0;
+    a.small_meshes = ctx->max_mesh_edges <= rp3dg::SMALL_MESH_EDGES ? 1 : 0;
     a.shapes = ctx->d_shapes;
     a.shape1 = p->shape1; a.shape2 = p->shape2;
     a.pos1 = reinterpret_cast<const float4*>(p->pos1); a.rot1 = reinterpret_cast<const float4*>(p->rot1);
