@@ -795,8 +795,7 @@ cudaError_t launch_narrowphase(int algo, const NpArgs& args, int num_sms, cudaSt
         const bool all = args.n <= uint32_t(num_sms) * uint32_t(NP_MIN_BLOCKS_MESH_WARP) * (NP_BLOCK / 32);
         for (int mask : {all ? WARP_ALL : WARP_MESH_BOX, all ? 0 : WARP_MESH_SECOND}) {
             if (mask == 0) break;
-            const bool small = mask == WARP_MESH_SECOND && args.stage_mesh && args.small_meshes;
-            e = launch_one((small ? WARP_KERNEL_SMALL : base) + mask, args, num_sms, stream);
+            e = launch_one((mask == WARP_MESH_SECOND && args.stage_mesh == 2 ? WARP_KERNEL_SMALL : base) + mask, args, num_sms, stream);
             if (e != cudaSuccess) return e;
             ++*launches;
         }

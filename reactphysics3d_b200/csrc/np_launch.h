@@ -24,8 +24,7 @@ struct NpArgs {
     uint32_t* error;  // device word: bit 0 = a pair named a shape outside the table
     uint32_t max_contacts;
     int clip;
-    int stage_mesh;
-    int small_meshes;  // no mesh has more than SMALL_MESH_EDGES edges
+    int stage_mesh;   // 0: no; 1: every CTA stages the arena; 2: and no mesh of it has more than SMALL_MESH_EDGES edges
     uint32_t mesh_nwords;
     const uint32_t* mesh_words;
     const rp3dg_shape* shapes;

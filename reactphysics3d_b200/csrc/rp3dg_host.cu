@@ -1109,8 +1109,8 @@ int np_args(rp3dg_ctx* ctx, int algorithm, const rp3dg_pair_batch* p, const rp3d
     a.mesh_nwords = uint32_t(ctx->arena.size());
     a.mesh_words = ctx->d_arena;
     a.stage_mesh = (algorithm >= RP3DG_ALGO_SPHERE_VS_CONVEX_POLYHEDRON && a.mesh_nwords > 0 &&
-                    size_t(a.mesh_nwords) * 4 <= rp3dg::MESH_STAGE_MAX_BYTES) ? 1 : 0;
-    a.small_meshes = ctx->max_mesh_edges <= rp3dg::SMALL_MESH_EDGES ? 1 : 0;
+                    size_t(a.mesh_nwords) * 4 <= rp3dg::MESH_STAGE_MAX_BYTES)
+                       ? (ctx->max_mesh_edges <= rp3dg::SMALL_MESH_EDGES ? 2 : 1) : 0;
     a.shapes = ctx->d_shapes;
     a.shape1 = p->shape1; a.shape2 = p->shape2;
     a.pos1 = reinterpret_cast<const float4*>(p->pos1); a.rot1 = reinterpret_cast<const float4*>(p->rot1);
