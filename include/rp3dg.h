@@ -499,8 +499,8 @@ int rp3dg_dynamics_step_host(rp3dg_ctx* ctx, const rp3dg_dynamics_params* params
  * no-collision body pairs (joints with collision disabled) are not applied.
  * The order of the pairs is deterministic but is not the reference's (which
  * follows its tree).  The search is a linear BVH (axis RP3DG_BROADPHASE_LBVH:
- * Morton-sorted fat-AABB centres, group in the high key bits, Karras tree,
- * bottom-up refit, warp-cooperative traversal) or a sort and sweep along
+ * Morton-sorted fat-AABB centres, group in the high key bits, radix tree
+ * built and boxed bottom-up, one walk per collider) or a sort and sweep along
  * axis 0, 1 or 2; both return the same set. */
 #define RP3DG_BROADPHASE_LBVH (-1)
 typedef struct rp3dg_broadphase {
@@ -920,7 +920,9 @@ int rp3dg_world_get_tuning(rp3dg_world* world, uint32_t* out);
 int rp3dg_world_get_phase_times(rp3dg_world* world, double* ms, uint32_t n);
 
 /* Number of kernels this context launched so far (instrumentation; a
- * convex-polyhedron batch takes two). */
+ * convex-polyhedron batch takes two, three above a pair for each resident warp
+ * (2,368 pairs on 148 SMs), and two more when its pairs are ordered first, from
+ * 4,096 pairs on). */
 uint64_t rp3dg_kernel_launches(const rp3dg_ctx* ctx);
 /* Islands without joints that the context's last dynamics stage solved by a
  * thread each, by a warp each, by a CTA each in shared memory, and streamed

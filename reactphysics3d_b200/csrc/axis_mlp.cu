@@ -34,8 +34,8 @@ __device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__floa
 // Bound: shared-memory loads and FP32 issue; activations and their gradients
 // never leave the SM (one thread per sample and one thread per weight, with
 // 1088 bytes of scratch per sample between them, took 681 us a call for 8192
-// samples; this takes 62 us, the read-back of the loss included).  The tile of 32 gives 128
-// CTAs at 4096 samples and 256 at 8192; 296 CTAs (two per SM) take any larger
+// samples; this takes 54 us, the read-back of the loss included).  The tile of 32
+// gives 128 CTAs at 4096 samples and 256 at 8192; 296 CTAs (two per SM) take any larger
 // batch, so that the partials stay at 8 MB and the reduction at one pass.
 // Row strides of 68 and 20 floats keep the float4 reads of 8 consecutive
 // rows (the backward products) on distinct banks.

@@ -698,23 +698,24 @@ RD void store_manifold(const DynArgs& a, uint32_t mi) {
 // movable body, the order of the manifolds touching it gives bit-identical
 // results.
 //
-// 3a: one thread per island runs islands of up to small_limit manifolds in
-//     the reference's order and queues the larger ones.
-// 3b: persistent warps take the queued islands.  Lane 0 gives each manifold a
-//     level (1 + the highest level of an earlier manifold sharing a movable
+// 3a: one thread per island queues the islands by size and solves those of up
+//     to small_limit manifolds itself, in the reference's order.
+// 3b: persistent warps take the queued islands.  The warp gives each manifold
+//     a level (1 + the highest level of an earlier manifold sharing a movable
 //     body) and sorts the island's manifolds by level; every pass (warm
-//     start, each velocity iteration) then runs level after level, the
-//     manifolds of a level in parallel across the warp, __syncwarp (which
-//     orders the lanes' memory accesses) between levels.  An island of up to
-//     STAGE_MANIFOLDS manifolds and STAGE_BODIES movable bodies is staged in
-//     the warp's shared memory: its manifold table, the schedule (computed
-//     with a shared hash of body -> slot, last level) and the bodies'
-//     velocities.  Larger islands use the same schedule built in global
-//     scratch, with velocities in global memory.
-
-// (a.small_max, 8 by default, and a.giant_min, 256 by default: islands above
-// it go to kernel 3c, one CTA per island, the island staged in up to the
-// whole opt-in shared memory of a CTA; both come from DynTuning)
+//     start, each velocity iteration) then runs level after level, __syncwarp
+//     (which orders the lanes' memory accesses) between them: four manifolds at
+//     a time on eight lanes each, or 32 on a lane each where the levels are
+//     wide.  An island of up to STAGE_MANIFOLDS manifolds and STAGE_BODIES
+//     bodies (fixed ones too) keeps its schedule and its bodies' velocities in
+//     the warp's shared memory; larger ones use the same schedule built in
+//     global scratch, one lane a manifold, velocities in global memory.
+// 3c: one CTA per island, staged in up to the whole opt-in shared memory of a
+//     CTA: the islands above giant_min manifolds, and those above BIG_ISLAND
+//     when there is a CTA for each (big_on_ctas).  When there are more giant
+//     islands than CTAs, 3b takes those that fit a warp (giants_on_warps).
+// 3d: the islands that do not fit 3c, streamed through global memory.
+// (small_max, 8 by default, and giant_min, 256 by default, come from DynTuning.)
 constexpr uint32_t ISLAND_DONE = 0xffffffffu;   // entry of giant_list solved by kernel 3b
 
 RD int4 man_ids(const DynArgs& a, uint32_t mi) {
@@ -737,7 +738,7 @@ __global__ void __launch_bounds__(128) dyn_islands_small(const DynArgs a) {
         atomicOr(a.error, 4u);
         return;
     }
-    if (a.i_jcount && a.i_jcount[is]) return;  // kernel 3d
+    if (a.i_jcount && a.i_jcount[is]) return;  // kernel 3e
     if (cnt == 0) return;
     if (cnt > s_limit) {
         // big islands fill the list from the front, the others from the back
@@ -1495,7 +1496,7 @@ __global__ void __launch_bounds__(LARGE_WARPS * 32, 2) dyn_islands_large(const D
 namespace rp3dg {
 namespace {
 
-// ---- kernel 3d: islands with joints --------------------------------------
+// ---- kernel 3e: islands with joints --------------------------------------
 //
 // One thread per island, in the reference's order: the contact warm start
 // (ContactSolverSystem::init), the joints' warm start
@@ -1564,22 +1565,21 @@ __global__ void __launch_bounds__(64) dyn_joints_position(const DynArgs a, uint3
     }
 }
 
-// ---- kernel 3c: islands of more than giant_min manifolds -----------------
+// ---- kernel 3c: large islands, a CTA each ---------------------------------
 //
-// One CTA of two warps takes one island at a time with the CTA's whole opt-in
-// shared memory: the movable bodies' velocities, every manifold's and point's
-// impulses, the manifold table and the level schedule (built by lane 0 with a
-// shared hash of body -> slot, last level) stay on chip for the warm start and
-// all velocity iterations.  Warp 0 solves, level after level; warp 1 stages
-// the constant rows of the manifolds (and their points) of level t + 2 into a
-// three-level ring with cp.async, with a compact descriptor per manifold,
-// while warp 0 solves level t, so warp 0's time per level is its arithmetic.
-// The two warps meet at one named barrier per level.  The arithmetic is
-// warm_core / solve_core, the same as the other paths: only where the rows and
-// impulses live changes.  An island that does not fit falls back to the
-// schedule in global scratch (solve_global), run by warp 0.
-// Solver warps, after the staging warp 0: the first solver, which every level
-// needs, then does not share warp 0's scheduler (the fourth does).
+// One CTA of five warps takes one island at a time with the CTA's whole opt-in
+// shared memory: the bodies' velocities, every manifold's and point's impulses,
+// the manifold table and the level schedule (island_schedule, by warp 0) stay
+// on chip for the warm start and all velocity iterations.  Warp 0 then stages
+// the constant rows of the first GIANT_RING manifolds (and their points) of
+// level t + 2 into a three-level ring with cp.async, with a compact descriptor
+// per manifold, while warps 1 to 4 solve level t, four manifolds each on eight
+// lanes a manifold (lanes_warm / lanes_solve); manifolds of a level beyond the
+// ring go one a lane with their rows from global memory (warm_core /
+// solve_core).  The warps meet at one named barrier per level.  An island that
+// does not fit, or whose points are not one range, is queued for kernel 3d.
+// The first solver warp, which every level needs, does not share the staging
+// warp's scheduler (the fourth does).
 constexpr uint32_t GIANT_SOLVERS = 4;
 constexpr uint32_t GIANT_RING = GIANT_SOLVERS * WARP_MANIFOLDS;   // manifolds of a level staged (the first 16)
 constexpr uint32_t GIANT_LEVELS = 3;   // levels in the ring

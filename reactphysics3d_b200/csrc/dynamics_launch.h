@@ -168,7 +168,7 @@ struct DynArgs {
     // by island, each island's ball-and-socket, fixed, hinge then slider
     // joints, each type in component order: record index, body 1 row, body 2 row, bit 0 / bit 1 =
     // body 1 / body 2 dynamic.  Islands with joints (i_jcount > 0) are solved
-    // by kernel 3d; after the position integration kernel 4b runs the
+    // by kernel 3e; after the position integration kernel 4b runs the
     // position correction of their joints and updates their bodies' state.
     uint32_t nj;
     const int4* j_list;
@@ -183,7 +183,7 @@ struct DynArgs {
     float4* xc;                 // constrained positions (centres of mass), all rows, kept between steps
     float4* qc;                 // constrained orientations, all rows
     int32_t position_iterations;
-    uint32_t giant_ctas;   // grid of kernel 3c (persistent, one warp per CTA)
+    uint32_t giant_ctas;   // grid of kernel 3c (persistent): the device's SMs
     uint32_t giant_smem;   // dynamic shared memory of a kernel-3c CTA (0: kernel 3c off)
     // graph-coloured solver (not the drop-in: see launch_dynamics) and the
     // solver statistics of the stage (either solver), when set

@@ -18,7 +18,7 @@ constexpr int RAY_STACK = 96;
 constexpr int RAY_BLOCK = 128;
 // Four resident CTAs per SM: with the lanes of a warp kept busy the spills of
 // 64 registers cost more than the warps they buy (300,007 rays over a
-// 20,000-body terrain: 3.04 ms at 8 CTAs, 2.80 at 6, 2.65 at 4, 2.97 at 3).
+// 20,000-body terrain: 2.64 ms at 8 CTAs, 2.36 at 6, 2.27 at 4, 2.40 at 3).
 #ifndef RAY_MIN_BLOCKS
 #define RAY_MIN_BLOCKS 4
 #endif
@@ -506,7 +506,7 @@ RD bool collider_raycast(const RayArgs& a, int4 col, v3 p1, v3 p2, float maxf, L
 // What a lane's ray waits for.
 enum RayWait { RAY_NODES = 0, RAY_SHAPE = 1, RAY_TERRAIN = 2, RAY_DONE = 3 };
 // Lanes that wait before their phase runs while others still have nodes to
-// visit, and before finished lanes take new rays (4 / 4: 2.58 ms on the
+// visit, and before finished lanes take new rays (4 / 4: 3 % less on the
 // terrain, but 684 us instead of 521 for 100,000 rays over 512 convex shapes).
 constexpr int RAY_GATHER = 8, RAY_REFILL = 4;
 
@@ -518,7 +518,7 @@ constexpr int RAY_GATHER = 8, RAY_REFILL = 4;
 // only the lanes' progress relative to each other changes.  Bound: the node
 // steps (245 a ray on the terrain), two dependent reads and ~75 instructions
 // each.  Each ray on its own path ran 2.7 lanes an instruction: 300,007 rays
-// over a 20,000-body terrain 5.57 ms, here 2.65; 32 rays 844 and 281 us;
+// over a 20,000-body terrain 5.16 ms, here 2.24; 32 rays 844 and 281 us;
 // 100,000 rays over 512 convex shapes 1,102 and 521 us.
 //
 // A node step reads both children of the current node at once and tests them

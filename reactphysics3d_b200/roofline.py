@@ -11,12 +11,16 @@ count 1; negations and copies count 0).  The FP32 work of a batch is then
 sum(events[e] * OPS[e]): the operations the reference's own code performs
 for those pairs, which is also the work the CPU baseline does.
 
-The kernels do less than that where they can: the warp schedule evaluates
-the polyhedron-1 half of each Gauss-map test once per edge instead of once
-per edge pair, and against a box each Gauss-map dot product reduces to one
-product (the other terms are exact zeros).  The fraction of the FP32 peak
-achieved on the reference's operation count therefore measures useful work
-per second in the reference's units.
+The kernels do less than that where they can: box edges are judged from 21
+sign bits of nine products an edge instead of five products for each of twelve
+edge pairs, and two meshes' edge pairs are first sifted by which side of the
+other's edge planes the face normals lie on, so that about one pair in a hundred
+takes the whole Gauss-map test, though all are counted here.  The rate and the
+fraction of the FP32 peak computed from these counts are therefore the
+reference's operations per second, useful work in the reference's units; they
+say nothing about how busy the FP32 pipes are (hull-box, ncu: FMA pipes active
+in 21 % of the cycles, 39,900 thread instructions a pair; with a Gauss-map test
+per edge pair 23 % and 70,700).
 
 Primitive costs (reference headers under include/reactphysics3d/mathematics):
   Quaternion * Vector3 (Quaternion.h:365-379)       41
