@@ -527,6 +527,13 @@ static uint32_t blocks_for(uint32_t n, uint32_t lanes) {
     return (n + per_block - 1) / per_block;
 }
 
+// Static + dynamic shared memory above 48 KB needs an opt-in, which is one value
+// a kernel for all contexts and threads: always the largest that a launch can
+// ask for, so that no context's launch lowers it for another's.
+static cudaError_t allow_staging(const void* k) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(MESH_STAGE_MAX_BYTES));
+}
+
 cudaError_t launch_narrowphase_tri(int algo, const NpArgs& args, int num_sms, cudaStream_t stream) {
     if (args.n == 0) return cudaSuccess;
     const void* k = algo == RP3DG_ALGO_SPHERE_VS_CONVEX_POLYHEDRON
@@ -538,11 +545,9 @@ cudaError_t launch_narrowphase_tri(int algo, const NpArgs& args, int num_sms, cu
                         : nullptr;
     if (!k || !args.tri) return cudaErrorInvalidValue;
     const size_t smem = args.stage_mesh ? size_t(args.mesh_nwords) * 4 : 0;
-    cudaFuncAttributes fa;
-    cudaError_t e = cudaFuncGetAttributes(&fa, k);
-    if (e != cudaSuccess) return e;
-    if (smem > 0 && fa.sharedSizeBytes + smem > 48 * 1024) {
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    cudaError_t e = cudaSuccess;
+    if (smem > 0) {
+        e = allow_staging(k);
         if (e != cudaSuccess) return e;
     }
     NpArgs a = args;
@@ -806,12 +811,11 @@ cudaError_t launch_narrowphase(int algo, const NpArgs& args, int num_sms, cudaSt
     return e;
 }
 
-// Per kernel: its static shared memory, the dynamic size its opt-in was set
-// for, and its resident CTAs per SM for that size (queried once: the
-// queries cost more host time than a launch).
+// Per kernel: the dynamic shared memory of the last launch and its resident CTAs
+// per SM for that size (queried once: the query costs more host time than a
+// launch).
 struct LaunchCache {
-    bool known = false;
-    size_t static_smem = 0, smem = ~size_t(0);
+    size_t smem = ~size_t(0);
     int per_sm = 0;
 };
 
@@ -823,17 +827,9 @@ static cudaError_t launch_one(int algo, const NpArgs& args, int num_sms, cudaStr
     static thread_local LaunchCache cache[32];
     LaunchCache& lc = cache[algo & 31];
     cudaError_t e = cudaSuccess;
-    if (!lc.known) {
-        cudaFuncAttributes fa;
-        e = cudaFuncGetAttributes(&fa, k);
-        if (e != cudaSuccess) return e;
-        lc.static_smem = fa.sharedSizeBytes;
-        lc.known = true;
-    }
     if (lc.smem != smem) {
-        // static + dynamic shared memory above 48 KB needs the opt-in attribute
-        if (smem > 0 && lc.static_smem + smem > 48 * 1024) {
-            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        if (smem > 0) {
+            e = allow_staging(k);
             if (e != cudaSuccess) return e;
         }
         lc.per_sm = 0;
