@@ -4,16 +4,17 @@
 // (reference src/engine/PhysicsWorld.cpp:239-318, src/systems/
 // DynamicsSystem.cpp:44-183, src/systems/ContactSolverSystem.cpp:66-818).
 //
-// Five kernels: bodies (inertia + velocities), manifolds (solver records, one
-// thread per manifold), islands (warm start, iterations, stored impulses: one
-// thread per island, manifolds in the reference's order, so each island sees
-// exactly the reference's sequence of Gauss-Seidel updates), bodies (positions
-// + state), colliders (local-to-world).  Every expression keeps the
+// Five steps: bodies (inertia + velocities), manifolds (solver records, one
+// thread per manifold), islands (warm start, iterations, stored impulses: a
+// thread, a warp or a CTA per island, the manifolds of every body in the
+// reference's order, so each sees exactly the reference's sequence of
+// Gauss-Seidel updates), bodies (positions + state), colliders
+// (local-to-world).  Every expression keeps the
 // reference's operand order; the library is built without FMA contraction,
 // so results are bit-identical to the reference's float build.
 #include <cuda_runtime.h>
-#ifdef RP3DG_PROFILE_GIANT
 #include <algorithm>
+#ifdef RP3DG_PROFILE_GIANT
 #include <cstdio>
 #endif
 
